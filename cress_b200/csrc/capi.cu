@@ -15,6 +15,7 @@
 #include "ctx.h"
 #include "diag.cuh"
 #include "hevi.cuh"
+#include "hevi_row.cuh"
 #include "forcing.cuh"
 #include "openbc.cuh"
 #include "tke.cuh"
@@ -295,40 +296,52 @@ int Ctx::wait_async(int keep) {
 // Elimination factors of the w system for one dts (w_system_factors,
 // wsystem.h: s_stepwi's coefficients and s_gaussel's factors), uploaded
 // once per distinct dts.
-int Ctx::thomas_for(float dts, const ThomasSet** out) {
+int Ctx::thomas_for(float dts, const HeviArgs& a, const ThomasSet** out) {
   uint32_t key;
   std::memcpy(&key, &dts, 4);
   auto it = thomas.find(key);
   if (it != thomas.end()) { *out = &it->second; return CRESS_OK; }
   const int nk = g.nk;
-  std::vector<float> rr(nk + 2), work(4 * (nk + 2));
+  std::vector<float> rr(nk + 2), work(4 * (size_t)(nk + 2));
   std::vector<double> cp(nk + 2), aa(nk + 2);
   w_system_factors(col_h.data(), nk, cfg.dz, cfg.weicoe, cfg.buyopt, dts, rr.data(), aa.data(), cp.data(),
                    work.data());
   std::vector<HeviLevel> rows(nk + 1);
   hevi_level_rows(col_h.data(), nk, rr.data(), aa.data(), cp.data(), rows.data());
-  std::vector<HeviLevel1> rows1(nk + 1);
-  hevi_level_rows1(col_h.data(), nk, rr.data(), aa.data(), cp.data(), rows1.data());
-  ThomasSet t;
-  if (cudaMalloc(&t.rr, sizeof(float) * (nk + 2)) != cudaSuccess ||
-      cudaMalloc(&t.aa, sizeof(double) * (nk + 2)) != cudaSuccess ||
-      cudaMalloc(&t.cp, sizeof(double) * (nk + 2)) != cudaSuccess ||
-      cudaMalloc(&t.lvl3, sizeof(HeviLevel) * (nk + 1)) != cudaSuccess ||
-      cudaMalloc(&t.lvl4, sizeof(HeviLevel1) * (nk + 1)) != cudaSuccess)
-    return set_error(CRESS_E_CUDA, "cudaMalloc (tridiagonal factors) failed");
-  owned.push_back(t.rr); owned.push_back(t.aa); owned.push_back(t.cp); owned.push_back(t.lvl3);
-  owned.push_back(t.lvl4);
+  std::vector<float> rlev;
+  std::vector<double> rdbl;
+  if (hevi_row_supported(g))
+    hevi_row_table(col_h.data(), nk, rr.data(), aa.data(), cp.data(), a, &rlev, &rdbl);
+  // one block, one copy: a new step length is set up inside a step's call
+  std::vector<unsigned char> buf;
+  auto add = [&](const void* p, size_t n) {
+    const size_t at = (buf.size() + 255) / 256 * 256;
+    buf.resize(at + n);
+    if (n) std::memcpy(buf.data() + at, p, n);
+    return at;
+  };
+  const size_t o_rr = add(rr.data(), sizeof(float) * rr.size()), o_aa = add(aa.data(), sizeof(double) * aa.size()),
+               o_cp = add(cp.data(), sizeof(double) * cp.size()),
+               o_l3 = add(rows.data(), sizeof(HeviLevel) * rows.size()),
+               o_rl = add(rlev.data(), sizeof(float) * rlev.size()),
+               o_rd = add(rdbl.data(), sizeof(double) * rdbl.size());
+  unsigned char* d = nullptr;
   int rc;
-  if ((rc = cuda_check(cudaMemcpyAsync(t.rr, rr.data(), sizeof(float) * (nk + 2), cudaMemcpyHostToDevice, stream), "copy rr")) ||
-      (rc = cuda_check(cudaMemcpyAsync(t.aa, aa.data(), sizeof(double) * (nk + 2), cudaMemcpyHostToDevice, stream), "copy aa")) ||
-      (rc = cuda_check(cudaMemcpyAsync(t.cp, cp.data(), sizeof(double) * (nk + 2), cudaMemcpyHostToDevice, stream), "copy cp")) ||
-      (rc = cuda_check(cudaMemcpyAsync(t.lvl3, rows.data(), sizeof(HeviLevel) * (nk + 1), cudaMemcpyHostToDevice,
-                                       stream), "copy level table")) ||
-      (rc = cuda_check(cudaMemcpyAsync(t.lvl4, rows1.data(), sizeof(HeviLevel1) * (nk + 1),
-                                       cudaMemcpyHostToDevice, stream), "copy level table")))
+  if ((rc = cuda_check(cudaMalloc(&d, buf.size()), "cudaMalloc (tridiagonal factors)"))) return rc;
+  owned.push_back(d);
+  // the host buffer is freed on return: make the copy complete
+  if ((rc = cuda_check(cudaMemcpyAsync(d, buf.data(), buf.size(), cudaMemcpyHostToDevice, stream), "copy factors")) ||
+      (rc = cuda_check(cudaStreamSynchronize(stream), "sync after factor upload")))
     return rc;
-  // The host vectors above are freed on return; make the copies complete.
-  if ((rc = cuda_check(cudaStreamSynchronize(stream), "sync after factor upload"))) return rc;
+  ThomasSet t;
+  t.rr = reinterpret_cast<float*>(d + o_rr);
+  t.aa = reinterpret_cast<double*>(d + o_aa);
+  t.cp = reinterpret_cast<double*>(d + o_cp);
+  t.lvl3 = reinterpret_cast<HeviLevel*>(d + o_l3);
+  if (!rlev.empty()) {
+    t.row_lev = reinterpret_cast<float4*>(d + o_rl);
+    t.row_dbl = reinterpret_cast<double2*>(d + o_rd);
+  }
   auto res = thomas.emplace(key, t);
   *out = &res.first->second;
   return CRESS_OK;
@@ -354,9 +367,10 @@ static EncodeTiledFn encode_fn() {
 }
 
 // 3-D tensor map (x = i, y = j, z = k-1) over one field buffer with a box
-// of kHeviBoxX x rows x 1, cached per (buffer, rows).
-int Ctx::tmap(const float* buf, int rows, CUtensorMap* out) {
-  auto key = std::make_pair(reinterpret_cast<const void*>(buf), rows);
+// of kHeviBoxX x rows x 1, or of 64 x 1 x levels (levels > 0, rows unused),
+// cached per (buffer, box).
+int Ctx::tmap(const float* buf, int rows, CUtensorMap* out, int levels) {
+  auto key = std::make_pair(reinterpret_cast<const void*>(buf), levels ? -levels : rows);
   auto it = tmaps.find(key);
   if (it != tmaps.end()) { *out = it->second; return CRESS_OK; }
   EncodeTiledFn fn = encode_fn();
@@ -365,6 +379,7 @@ int Ctx::tmap(const float* buf, int rows, CUtensorMap* out) {
   cuuint64_t dims[3] = {(cuuint64_t)g.px, (cuuint64_t)g.py, (cuuint64_t)g.nk};
   cuuint64_t strides[2] = {(cuuint64_t)g.px * 4, (cuuint64_t)g.plane * 4};
   cuuint32_t box[3] = {(cuuint32_t)kHeviBoxX, (cuuint32_t)rows, 1};
+  if (levels) { box[0] = 64; box[1] = 1; box[2] = (cuuint32_t)levels; }
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(buf), dims, strides, box,
                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -402,19 +417,46 @@ int Ctx::level_table(float dtb2, const float** out) {
   return CRESS_OK;
 }
 
-int Ctx::small_steps(int nsstp, float dts) { return small_steps(nsstp, dts, nullptr); }
+// Tiles 0 and 13 run the row-marching kernel where its chunks cover the
+// column (tile 13 is offered up to kHevi3MaxNk levels): it is the faster one at
+// every size measured, 14 us against 85 us per substep at 64x64x40 and 0.197 ms
+// against 0.289 ms (0.321 ms with tile 0's k_hevi2) at 512x512x64.
+bool Ctx::row_kernel() const {
+  return cfg.impopt == 1 && (cfg.tile == 0 || (cfg.tile == 13 && g.nk <= kHevi3MaxNk)) && hevi_row_supported(g);
+}
 
-int Ctx::small_steps(int nsstp, float dts, std::vector<HeviJob>* jobs) {
+// What the row kernel leaves to the end of the substep loop, on the new
+// level f: boundary levels and y ghosts.
+int Ctx::row_ends(float* const* f) {
+  HeviRowArgs a{};
+  a.g = g;
+  a.u = lev[CRESS_U][CRESS_PAST]; a.v = lev[CRESS_V][CRESS_PAST]; a.p = lev[CRESS_PP][CRESS_PAST];
+  a.un = f[0]; a.vn = f[1]; a.wn = f[2]; a.pn = f[3];
+  a.jw3 = col_h[(size_t)C_JCB8W * (g.nk + 1) + 3]; a.jwt = col_h[(size_t)C_JCB8W * (g.nk + 1) + g.nk - 2];
+  a.sth = cfg.sthopt; a.bbc = cfg.bbc;
+  ++launches;
+  return launch_hevi_row_ends(a, stream);
+}
+
+int Ctx::row_ends_future() {
+  float* const f[4] = {lev[CRESS_U][CRESS_FUTURE], lev[CRESS_V][CRESS_FUTURE], lev[CRESS_W][CRESS_FUTURE],
+                       lev[CRESS_PP][CRESS_FUTURE]};
+  const int rc = row_ends(f);
+  return rc ? set_error(rc, "small-step launch failed: %s", cudaGetErrorString(cudaGetLastError())) : CRESS_OK;
+}
+
+int Ctx::small_steps(int nsstp, float dts) { return small_steps(nsstp, dts, nullptr, nullptr); }
+
+int Ctx::small_steps(int nsstp, float dts, std::vector<HeviJob>* jobs, std::vector<HeviRowJob>* rjobs) {
   if (!base_set) return set_error(CRESS_E_STATE, "cress_small_steps: base state not set");
-  if (jobs && (cfg.impopt != 1 || (cfg.tile != 0 && cfg.tile != 13) || g.openx))
+  if ((jobs || rjobs) && (cfg.impopt != 1 || (cfg.tile != 0 && cfg.tile != 13) || g.openx))
     return set_error(CRESS_E_UNSUPPORTED, "ensemble small steps need impopt=1, tile 0 or 13 and periodic x");
   if (g.openx && cfg.tile != 0 && cfg.tile != 11 && cfg.tile != 12 && cfg.tile != 13)
     return set_error(CRESS_E_UNSUPPORTED, "open x boundaries run the HE-VI tiles 0, 11, 12 and 13");
   if (nsstp < 1) return set_error(CRESS_E_ARG, "cress_small_steps: nsstp=%d", nsstp);
   const bool heve = cfg.impopt == 0;
   const ThomasSet* th = nullptr;
-  int rc = heve ? CRESS_OK : thomas_for(dts, &th);
-  if (rc) return rc;
+  int rc;
   HeviArgs a{};
   a.g = g;
   a.col = col_d;
@@ -423,7 +465,6 @@ int Ctx::small_steps(int nsstp, float dts, std::vector<HeviJob>* jobs) {
     if ((rc = level_table(0.f, &t))) return rc;
   }
   a.lvl = level_tables.begin()->second;
-  if (th) { a.thom_rr = th->rr; a.thom_aa = th->aa; a.thom_cp = th->cp; a.lvl3 = th->lvl3; a.lvl4 = th->lvl4; }
   a.err = err_d;
   a.dts = dts;
   a.dxiv = 1.f / cfg.dx; a.dyiv = 1.f / cfg.dy; a.dziv = 1.f / cfg.dz;
@@ -436,6 +477,31 @@ int Ctx::small_steps(int nsstp, float dts, std::vector<HeviJob>* jobs) {
   a.g05n = -.5f * kG;
   a.divopt = cfg.divopt; a.buyopt = cfg.buyopt; a.sthopt = cfg.sthopt; a.bbc = cfg.bbc;
   a.spin = spin_limit;
+  if (!heve && (rc = thomas_for(dts, a, &th))) return rc;
+  if (th) { a.thom_rr = th->rr; a.thom_aa = th->aa; a.thom_cp = th->cp; a.lvl3 = th->lvl3; }
+  const bool row = row_kernel() && !jobs;
+  if (rjobs && !row) return set_error(CRESS_E_UNSUPPORTED, "the row kernel does not run on this grid");
+  HeviRowArgs ra{};
+  HeviRowMaps rm;
+  if (row) {
+    ra.g = g;
+    ra.err = err_d;
+    ra.spin = spin_limit;
+    const int L = hevi_row_chunk(g.nk);
+    if ((rc = tmap(lev[CRESS_U][CRESS_FORCING], 0, &rm.uf, L)) || (rc = tmap(lev[CRESS_V][CRESS_FORCING], 0, &rm.vf, L)) ||
+        (rc = tmap(lev[CRESS_W][CRESS_FORCING], 0, &rm.wf, L)) || (rc = tmap(lev[CRESS_PP][CRESS_FORCING], 0, &rm.pf, L)))
+      return rc;
+    ra.tab.lev = th->row_lev; ra.tab.dbl = th->row_dbl;
+    auto twice = [](float v) {
+      uint32_t b;
+      std::memcpy(&b, &v, 4);
+      return (uint64_t)b << 32 | b;
+    };
+    ra.dxiv2 = twice(a.dxiv); ra.dyiv2 = twice(a.dyiv); ra.dziv2 = twice(a.dziv);
+    const Grid* gp = &g;
+    ra.rows = hevi_row_rows(&gp, 1);
+    ra.tiles_x = hevi_row_tiles_x(g);
+  }
   const int TY = hevi_tile_rows(heve ? 0 : cfg.tile);
   HeviMaps maps;
   if ((rc = tmap(lev[CRESS_U][CRESS_FORCING], TY, &maps.uf)) ||
@@ -472,7 +538,28 @@ int Ctx::small_steps(int nsstp, float dts, std::vector<HeviJob>* jobs) {
       rc = launch_heve_substep(a, maps, stream);
       ++launches;
     } else {
-      rc = launch_hevi_substep(a, maps, cfg.tile, stream);
+      if (row) {
+        const int L = hevi_row_chunk(g.nk);
+        ra.u = olds[0]; ra.v = olds[1]; ra.p = olds[3];
+        ra.un = news[0]; ra.vn = news[1]; ra.wn = news[2]; ra.pn = news[3];
+        if ((rc = tmap(olds[0], 0, &rm.u, L)) || (rc = tmap(olds[1], 0, &rm.v, L)) ||
+            (rc = tmap(olds[2], 0, &rm.w, L + 1)) || (rc = tmap(olds[3], 0, &rm.p, L)))
+          return rc;
+        ra.wrap = s > 0 && !g.slaby;   // the loop's own levels carry no y ghosts until its end
+        if (rjobs) {
+          HeviRowJob jb;
+          std::memset(&jb, 0, sizeof jb);
+          jb.maps = rm;
+          jb.args = ra;
+          rjobs->push_back(jb);
+          --launches;
+        } else {
+          rc = launch_hevi_row(rm, ra, stream);
+          if (!rc && s == nsstp - 1) rc = row_ends(news);
+        }
+      } else {
+        rc = launch_hevi_substep(a, maps, cfg.tile, stream);
+      }
       ++launches;
       if (!rc && g.openx) {   // the boundary columns of this substep (stepuv/stepwi/steppi rbc*)
         RbcSmallArgs r{};
@@ -921,8 +1008,8 @@ int Ctx::autotune(int nsstp, float dts, int reps, int* best, float* ms) {
 
 // An ensemble of independent domains on one device and one stream: every
 // member runs its own large step, except that the acoustic substeps of all
-// members run as one launch per substep (k_hevi2_batch over every
-// member's tiles), so small domains fill the GPU together.
+// members run as one launch per substep (k_hevi_row_batch, or k_hevi2_batch,
+// over every member's tiles), so small domains fill the GPU together.
 // An ensemble step runs each member's work before and after the acoustic
 // substeps on the member's own stream (members overlap), and the substeps of
 // all members as one launch per substep on the ensemble's stream, joined to
@@ -976,11 +1063,28 @@ struct Ensemble {
   int large_step(long long ctime, float dtb, int nsstp, float dts, HeviJob* jd, HeviJob* jh, bool eager);
   int step(long long ctime, float dtb, int nsstp, float dts);
   int set_tile(int t);
-  int batch(const HeviJob* jd, int nblocks, int nk_max) {
+  // Whether the batched substeps run the row kernel (every member's grid
+  // must allow it; else tile 0's k_hevi2_batch).  Then a substep is one
+  // launch per group of members with equal chunk lengths and counts
+  // (members of equal nk share one).
+  bool rows() const {
+    for (const Ctx* c : members)
+      if (!c->row_kernel()) return false;
+    return true;
+  }
+  struct Group { int first, n, nblocks, nk; };
+  std::vector<Group> groups;   // of the jobs last formed
+  int batch(const HeviJob* jobs, int st, int nblocks, int nk_max) {   // substep st of the job table
     const cress_cfg& c0 = members[0]->cfg;
     const int n = (int)members.size();
-    return tile == 13 ? launch_hevi4_batch(jd, n, nblocks, nk_max, c0.divopt, c0.sthopt != 0, c0.buyopt == 1, stream)
-                      : launch_hevi_batch(jd, n, nblocks, nk_max, c0.divopt, c0.sthopt != 0, c0.buyopt == 1, stream);
+    if (groups.empty())
+      return launch_hevi_batch(jobs + (size_t)st * n, n, nblocks, nk_max, c0.divopt, c0.sthopt != 0, c0.buyopt == 1, stream);
+    const HeviRowJob* rj = reinterpret_cast<const HeviRowJob*>(jobs) + (size_t)st * n;
+    for (const Group& q : groups) {
+      const int rc = launch_hevi_row_batch(rj + q.first, q.n, q.nblocks, q.nk, stream);
+      if (rc) return rc;
+    }
+    return CRESS_OK;
   }
   int jobs_for(int nsstp, float dts, HeviJob* jh, int* nblocks, int* nk_max);
   int autotune(int nsstp, float dts, int reps, int* best, float* ms);
@@ -1012,7 +1116,7 @@ int Ensemble::large_step(long long ctime, float dtb, int nsstp, float dts, HeviJ
     return rc;
   if (eager) cudaEventRecord(staged, stream);
   for (int st = 0; st < nsstp; ++st) {
-    if ((rc = batch(jd + (size_t)st * n, nblocks, nk_max)))
+    if ((rc = batch(jd, st, nblocks, nk_max)))
       return set_error(rc, "ensemble small-step launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     ++launches;
   }
@@ -1020,6 +1124,7 @@ int Ensemble::large_step(long long ctime, float dtb, int nsstp, float dts, HeviJ
   for (int m = 0; m < n; ++m) {
     Ctx* c = members[m];
     cudaStreamWaitEvent(c->stream, done, 0);
+    if (!groups.empty() && (rc = c->row_ends_future())) return rc;
     if ((rc = c->large_step(filter, dtb, nsstp, dts, 2))) return rc;
   }
   for (int m = 0; m < n; ++m) {   // join: the ensemble's stream follows every member
@@ -1037,9 +1142,41 @@ int Ensemble::jobs_for(int nsstp, float dts, HeviJob* jh, int* nblocks, int* nk_
   int rc;
   *nblocks = 0;
   *nk_max = 0;
+  groups.clear();
+  if (rows()) {
+    // the jobs of a substep in group order, in the table's memory
+    static_assert(sizeof(HeviRowJob) <= sizeof(HeviJob), "the job tables hold either kind");
+    HeviRowJob* rj = reinterpret_cast<HeviRowJob*>(jh);
+    std::map<std::pair<int, int>, std::vector<int>> by;   // (chunk length, chunks) -> members
+    for (int m = 0; m < n; ++m) {
+      const int nk = members[m]->g.nk, L = hevi_row_chunk(nk);
+      by[{L, (nk - 3 + L - 1) / L}].push_back(m);
+    }
+    int at = 0;
+    for (auto& kv : by) {
+      std::vector<const Grid*> gs;
+      for (int m : kv.second) gs.push_back(&members[m]->g);
+      const int rows_ = hevi_row_rows(gs.data(), (int)gs.size());
+      Group q{at, (int)gs.size(), 0, gs[0]->nk};
+      for (int m : kv.second) {
+        std::vector<HeviRowJob> per;
+        if ((rc = members[m]->small_steps(nsstp, dts, nullptr, &per))) return rc;
+        for (int st = 0; st < nsstp; ++st) {
+          HeviRowJob& j = rj[(size_t)st * n + at];
+          j = per[st];
+          j.args.rows = rows_;
+          j.first_block = q.nblocks;
+        }
+        q.nblocks += per[0].args.tiles_x * ((members[m]->g.nj - 3 + rows_ - 1) / rows_);
+        ++at;
+      }
+      groups.push_back(q);
+    }
+    return CRESS_OK;
+  }
   for (int m = 0; m < n; ++m) {
     std::vector<HeviJob> per;
-    if ((rc = members[m]->small_steps(nsstp, dts, &per))) return rc;
+    if ((rc = members[m]->small_steps(nsstp, dts, &per, nullptr))) return rc;
     *nk_max = std::max(*nk_max, members[m]->g.nk);
     int tx, ty;
     hevi_job_tiles(members[m]->g, &tx, &ty);
@@ -1098,10 +1235,10 @@ int Ensemble::autotune(int nsstp, float dts, int reps, int* best, float* ms) {
     if ((rc = cuda_check(cudaMemcpyAsync(jd, jh, sizeof(HeviJob) * need, cudaMemcpyHostToDevice, stream),
                          "copy ensemble jobs")))
       break;
-    for (int st = 0; st < nsstp && !rc; ++st) rc = batch(jd + (size_t)st * n, nblocks, nk_max);   // warm-up
+    for (int st = 0; st < nsstp && !rc; ++st) rc = batch(jd, st, nblocks, nk_max);   // warm-up
     cudaEventRecord(e0, stream);
     for (int r = 0; r < reps && !rc; ++r)
-      for (int st = 0; st < nsstp && !rc; ++st) rc = batch(jd + (size_t)st * n, nblocks, nk_max);
+      for (int st = 0; st < nsstp && !rc; ++st) rc = batch(jd, st, nblocks, nk_max);
     cudaEventRecord(e1, stream);
     if (rc == CRESS_E_UNSUPPORTED) { rc = CRESS_OK; continue; }
     if (rc || (rc = cuda_check(cudaEventSynchronize(e1), "ensemble autotune sync"))) break;

@@ -9,6 +9,7 @@
 #include "../../include/cress_b200.h"
 #include "common.cuh"
 #include "hevi.cuh"
+#include "hevi_row.cuh"
 #include "micro.cuh"
 #include "slab.h"
 
@@ -23,7 +24,8 @@ struct ThomasSet {
   double* aa = nullptr;
   double* cp = nullptr;
   HeviLevel* lvl3 = nullptr;   // level table of the on-chip kernel (rows 0..nk)
-  HeviLevel1* lvl4 = nullptr;  // the same once per value (one-column-per-thread kernel)
+  float4* row_lev = nullptr;   // tables of the row-marching kernel (hevi_row.cuh), or null
+  double2* row_dbl = nullptr;
 };
 
 struct Ctx {
@@ -81,17 +83,21 @@ struct Ctx {
   // grown as needed
   void* rec_d = nullptr;
   long long rec_bytes = 0;
-  int thomas_for(float dts, const ThomasSet** out);
+  int thomas_for(float dts, const HeviArgs& a, const ThomasSet** out);   // a: the step's scalars
   std::map<uint32_t, float*> level_tables;   // level table per 2*dtb (bits)
   int level_table(float dtb2, const float** out);
+  // whether the HE-VI substeps run the row-marching kernel
+  bool row_kernel() const;
   int small_steps(int nsstp, float dts);
   // phase 0: the whole step; 1: up to the forcing; 2: from the moist
   // scalars on (an ensemble runs every member's small steps in between)
   int large_step(bool filter, float dtb, int nsstp, float dts, int phase = 0);
-  // jobs != null: instead of launching, append every substep's arguments
-  // and maps (HE-VI, tile 0) for an ensemble launch; the pointer swaps that
+  // jobs or rjobs != null: instead of launching, append every substep's
+  // arguments and maps for an ensemble launch (k_hevi2's or the row kernel's); the pointer swaps that
   // make the result the future level are done either way
-  int small_steps(int nsstp, float dts, std::vector<HeviJob>* jobs);
+  int small_steps(int nsstp, float dts, std::vector<HeviJob>* jobs, std::vector<HeviRowJob>* rjobs);
+  int row_ends(float* const* f);
+  int row_ends_future();
   int ksp0 = 2;            // first Rayleigh-damped level
   bool large_set = false;  // cress_set_base_large was called
   bool moist_set = false;  // cress_set_base_moist was called
@@ -136,7 +142,7 @@ struct Ctx {
   int step(bool filter, float dtb, int nsstp, float dts);
   void free_graphs();
   int satadjst(int level, float thresq);
-  int tmap(const float* buf, int rows, CUtensorMap* out);
+  int tmap(const float* buf, int rows, CUtensorMap* out, int levels = 0);
   int check_device_error();
   void* diag_d = nullptr;
   float* rad_d = nullptr;   // open x: phase speeds (openbc.cuh layout)

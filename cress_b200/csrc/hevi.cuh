@@ -59,18 +59,7 @@ struct alignas(16) HeviLevel {
 };
 static_assert(sizeof(HeviLevel) == 144, "HeviLevel is nine 16-byte vectors");
 
-// The same values once each (five 16-byte vectors per level), for the
-// one-column-per-thread on-chip kernel (tile 13).
-struct alignas(16) HeviLevel1 {
-  float rst8u, rst8v, rst8w, ij8w;
-  float jcb, ijcb, irst8u, irst8v;
-  float jcb8u, jcb8v, rcsq, rst;
-  float rbr, ircsq, irst8w, rr;
-  double aa, cp;
-};
-static_assert(sizeof(HeviLevel1) == 80, "HeviLevel1 is five 16-byte vectors");
-
-// Largest nk the on-chip kernels hold: the eliminated right-hand sides of
+// Largest nk of tiles 12 and 13.  Tile 12: the eliminated right-hand sides of
 // levels 3..nk-2 of two columns in FP64 fill 4 (nk - 4) <= 256 tensor-memory
 // columns per thread.
 constexpr int kHevi3MaxNk = 68;
@@ -85,7 +74,6 @@ struct HeviArgs {
   const double* thom_aa;  // [k] 1/(b_k - a_k c'_{k-1})
   const double* thom_cp;  // [k] c'_k
   const HeviLevel* lvl3;  // level table of tile 12 (rows k = 0..nk), or null
-  const HeviLevel1* lvl4; // level table of tile 13 (rows k = 0..nk), or null
   int* err;               // device error word (nonzero: a bounded wait gave up)
   // HE-VE only: the contravariant w of levels 2 and nk-1 (two planes of
   // px*py each), which the reference keeps from the explicit update while
@@ -105,8 +93,6 @@ struct HeviArgs {
 int hevi_tile_rows(int tile);
 // The on-chip kernel (tile 12); needs a.lvl3 and nk <= kHevi3MaxNk.
 int launch_hevi3(const HeviArgs& a, const HeviMaps& maps, cudaStream_t st);
-// The on-chip kernel with one column per thread (tile 13); needs a.lvl4.
-int launch_hevi4(const HeviArgs& a, const HeviMaps& maps, cudaStream_t st);
 // Launch one substep; `maps` must describe the buffers in `a` with the
 // box rows of HeviRows<hevi_tile_rows(tile)>.
 int launch_hevi_substep(const HeviArgs& a, const HeviMaps& maps, int tile, cudaStream_t st);
@@ -124,11 +110,6 @@ void hevi_job_tiles(const Grid& g, int* tx, int* ty);
 // all); every member uses divopt, sthopt != 0 (sth), buyopt == 1 (buy).
 int launch_hevi_batch(const HeviJob* jobs_d, int njobs, int nblocks, int nk_max, int divopt, bool sth, bool buy,
                       cudaStream_t st);
-// The same with the one-column-per-thread on-chip kernel (tile 13: the same
-// 32 x 8 tiles; every member's args.lvl4 set, nk <= kHevi3MaxNk).
-int launch_hevi4_batch(const HeviJob* jobs_d, int njobs, int nblocks, int nk_max, int divopt, bool sth, bool buy,
-                       cudaStream_t st);
-
 // One HE-VE substep (impopt=0, s_heve); the maps are those of tile 0's
 // box rows (HeviRows<8>) and a.lvl must hold the level table.
 int launch_heve_substep(const HeviArgs& a, const HeviMaps& maps, cudaStream_t st);

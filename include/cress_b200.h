@@ -53,9 +53,10 @@ typedef struct cress_cfg {
                               wbc = ebc = 4, 5 or 7 (open radiation x boundaries: phase speed per
                               point, its column average, or the constant gwave) with sbc = nbc = -1 */
   int bbc, tbc;         /* 2 = rigid (SrcOrig/vbcw.f90:201) */
-  int tile;             /* HE-VI tile shape id (0 = default: 32x8, two rows per thread; 1-11 other shapes;
-                           12, 13: 32x8 with the column kept on chip, FP64 throughout the solve, nk <= 68;
-                           12 two rows per thread, 13 one) */
+  int tile;             /* HE-VI tile shape id (0 = default: the row-marching kernel up to 80 levels, above
+                           that 32x8 with two rows per thread; 1-11 other shapes; 12, 13: FP64 throughout
+                           the solve, nk <= 68; 12 a 32x8 tile of columns kept on chip, 13 the row-marching
+                           kernel, as 0) */
   /* large step (SrcOrig/forcedrv.f90:548-608, SrcOrig/timeflt.f90:335) */
   int advopt;           /* 2: 4th-order horizontal, 2nd-order vertical advection; 3: 4th order in z as well (periodic boundaries) */
   int smtopt;           /* 0 none, 2 horizontal, 3 horizontal + vertical 4th-order smoothing */
@@ -107,7 +108,7 @@ int cress_set_stream(cress_ctx* ctx, void* stream);
 int cress_sync(cress_ctx* ctx);
 
 /* Failure-path test hook, no counterpart in the reference: the number of
- * probes each ring wait of the HE-VI level loop (tile 0) makes before it
+ * probes each copy wait of the HE-VI loop (tile 0) makes before it
  * gives up (default 4194304; 0 gives up at once).  A wait that gives up
  * makes the kernel stop issuing copies, wait for the ones in flight and
  * return, and the next synchronizing call reports CRESS_E_TIMEOUT; the
@@ -322,9 +323,11 @@ int cress_autotune(cress_ctx* ctx, int nsstp, float dts, int reps, int* best_til
  * were seen before replays one CUDA graph of the whole ensemble step
  * (cress_ensemble_set_graphs(e, 0) turns that off).  Members need impopt=1
  * and the same divopt, sthopt (zero or not) and buyopt.  The shared
- * acoustic launch runs tile 0's kernel or tile 13's (the FP64 right-hand
- * sides on chip; every member with 8 <= nk <= 68): tile 13 when every
- * member was created with tile 13, else tile 0, and the members are set
+ * acoustic launch runs the row-marching kernel (members of different
+ * height in separate launches) when every member's grid allows it, else
+ * tile 0's 32x8 kernel.  The ensemble's tile is 13 (every member with
+ * 8 <= nk <= 68) when every member was created with tile 13, else 0, and the
+ * members are set
  * to the ensemble's tile.  cress_ensemble_set_tile switches it (0 or 13);
  * cress_ensemble_autotune times both over `reps` loops of nsstp batched
  * substeps of length dts on the members' present state (only the future
@@ -461,7 +464,7 @@ int cress_set_tuple_sampling(cress_ctx* ctx, cress_mlp* m, int stride, float kee
  * call's on the device, and always clears its error word; calls whose
  * kernels overlap on the GPU race on it and must be serialized.  The
  * horizontal-uniformity scan of base3d runs only on such a change.  The
- * kernel is the context API's for cfg->tile (0-10; 11 is rejected).
+ * kernels are those of the tile shapes 0-10 (0: 32x8, two rows per thread).
  * The first call on a device looks up the
  * array's address with that device current; make it before any stream
  * capture begins.  The call is synchronous on `stream` (NULL = the default

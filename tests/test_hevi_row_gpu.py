@@ -1,0 +1,59 @@
+"""The row-marching HE-VI kernel (tiles 0 and 13) where its partition can go
+wrong: widths around its 60-column tiles, column heights around its chunk
+lengths (2, 3, 4 and 5 levels per warp) and a partial top chunk, strips of one
+row, and several substeps, so that the second and later ones read the rows
+whose periodic images are not written in between.  Against the FP32 oracle with
+the small step's tolerance (test_small_gpu.py)."""
+import numpy as np
+import pytest
+
+from test_ensemble_gpu import NAMES, member
+from test_small_gpu import check, run_pair
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nx,ny,nz", [
+    (5, 5, 5),       # the smallest grid cress_create takes
+    (59, 7, 32),     # one tile with an odd last column; 16 chunks of 2
+    (60, 9, 33),     # a full tile; chunks of 3
+    (61, 6, 48),     # a second tile of one column
+    (120, 13, 49),   # two full tiles; chunks of 4
+    (181, 5, 65),    # a last tile of one column; chunks of 5, the last one full
+    (62, 21, 78),    # a partial top chunk
+])
+def test_partition_edges(cress, oracle_lib, nx, ny, nz):
+    ni, nj, nk, ref, out = run_pair(cress, oracle_lib, nx, ny, nz, 3, sthopt=1, seed=nx + nz, tile=0)
+    check(ni, nj, nk, ref, out, 3)
+
+
+@pytest.mark.parametrize("divopt,sthopt", [(0, 1), (1, 0), (2, 0)])
+def test_options(cress, oracle_lib, divopt, sthopt):
+    ni, nj, nk, ref, out = run_pair(cress, oracle_lib, 70, 34, 27, 4, sthopt=sthopt, divopt=divopt, seed=4, tile=0)
+    check(ni, nj, nk, ref, out, 4)
+
+
+def test_levels_beyond_the_chunks_run_the_ring_kernel(cress, oracle_lib):
+    ni, nj, nk, ref, out = run_pair(cress, oracle_lib, 40, 12, 82, 2, sthopt=1, seed=8, tile=0, dz=150.0)
+    check(ni, nj, nk, ref, out, 2)
+
+
+def test_ensemble_of_different_heights_matches_members(cress, oracle_lib):
+    """Members with different chunk lengths go out in separate launches; each
+    equals the member stepped alone, bit for bit."""
+    sizes = [(40, 33, 22, 1), (64, 20, 36, 2), (29, 45, 22, 3)]
+    out = []
+    for together in (False, True):
+        sols = [member(cress, oracle_lib, *sz) for sz in sizes]
+        ens = cress.Ensemble(sols, graphs=False) if together else None
+        for step in range(2):
+            h = 0.5 if step == 0 else 1.0
+            for s in [ens] if together else sols:
+                s.large_step(step * 5000, 5.0 * h, 10, h)
+        out.append([s.get_field(n, cress.NOW) for s in sols for n in NAMES])
+        if ens:
+            ens.close()
+        for s in sols:
+            s.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
