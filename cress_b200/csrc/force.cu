@@ -81,6 +81,18 @@ __host__ __device__ constexpr int force_slot(int G, int q) {
 // F2 of two consecutive floats of a global field (8-byte aligned index).
 __device__ __forceinline__ F2 gld2(const float* p) { return F2{__ldg(reinterpret_cast<const float2*>(p))}; }
 
+// The buoyancy term of one level (ck: its row of the level table) at the
+// thread's pair, g05 rst (...): dry, or moist with the total condensate.
+__device__ __forceinline__ F2 buoyancy(const ForceArgs& a, const float* ck, long long id) {
+  const float g05 = .5f * 9.8f;
+  if (!a.qv) return g05 * ck[C_RST] * gld2(a.ptp + id) * ck[D_IPTBR];
+  const F2 qvd = gld2(a.qv + id) - ck[C_QVBR];
+  const F2 qall = (((gld2(a.qc + id) + gld2(a.qr + id)) + gld2(a.qi + id)) + gld2(a.qs + id)) +
+                  gld2(a.qg + id);   // totalqwi.f90:163
+  return g05 * ck[C_RST] *
+         ((qvd * ck[D_IEPSQV] - (qvd + qall) * ck[D_I1QV]) + gld2(a.ptp + id) * ck[D_IPTBR]);
+}
+
 // The forcing of group G (0 u, 1 v, 2 w, 3 p', 4 theta') at the thread's
 // pair of columns, level k.  stp[d + 2] is the ring stage of level k + d,
 // rowbase the thread's own row and first column in a box, id the global
@@ -108,7 +120,6 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
   const bool smooth = (a.smtopt % 10 == 2) || (a.smtopt % 10 == 3);
   // advopt=3: 4th-order vertical advection on the levels 3..nk-3 (w: 3..nk-2)
   const bool adv3 = a.advopt == 3 && k >= 3 && k <= (G == 2 ? nk - 2 : nk - 3);
-  const float g05 = .5f * 9.8f;
   const float* ck = tab + k * kNF;   // the level table in shared memory
   auto C = [&](int f, int kk) { return ck[(kk - k) * kNF + f]; };
   // field q of this group at the offset (dx, dy, dz), both points
@@ -292,18 +303,7 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
     if (a.vspopt >= 1 && a.vsp_w && k >= a.ksp0) f = f - C(C_RBCT, k) * C(C_RST8W, k) * WP(0, 0, 0);
     // buoywb.f90:166-172 (dry), 202-299 (moist), 307-313: the term of
     // level k is formed once and reused as the level below of k+1
-    F2 wbk = f2(0.f);
-    if (k <= nk - 2) {
-      if (!a.qv) {
-        wbk = g05 * C(C_RST, k) * gld2(a.ptp + id) * C(D_IPTBR, k);
-      } else {
-        const F2 qvd = gld2(a.qv + id) - C(C_QVBR, k);
-        const F2 qall = (((gld2(a.qc + id) + gld2(a.qr + id)) + gld2(a.qi + id)) + gld2(a.qs + id)) +
-                        gld2(a.qg + id);   // totalqwi.f90:163
-        wbk = g05 * C(C_RST, k) *
-              ((qvd * C(D_IEPSQV, k) - (qvd + qall) * C(D_I1QV, k)) + gld2(a.ptp + id) * C(D_IPTBR, k));
-      }
-    }
+    const F2 wbk = k <= nk - 2 ? buoyancy(a, ck, id) : f2(0.f);
     if (k >= 3 && k <= nk - 2) f = f + (wb_prev + wbk);
     wb_prev = wbk;
     // advuvw.f90:685-852
@@ -418,7 +418,11 @@ k_force(const __grid_constant__ ForceMaps m, const ForceArgs a) {
   // ni-1, the other groups: i = 2 and ni-2)
   const int elast = G == 0 ? ni - 1 : ni - 2;
   const int edge = g.openx ? ((i == 2 || i == elast) ? 1 : 0) | ((i + 1 == 2 || i + 1 == elast) ? 2 : 0) : 0;
-  const int kmax = SG == 0 ? nk - 1 : nk - 2, lmax = SG == 0 ? nk : nk - 1;
+  const int kmax = SG == 0 ? nk - 1 : nk - 2;
+  // this block's levels kA..kB of 2..kmax (blockIdx.z), and the levels it
+  // stages, two more at either end; level lv lives in slot (lv-lv0) % S
+  const int kA = 2 + blockIdx.z * a.kchunk, kB = min(kA + a.kchunk - 1, kmax);
+  const int lv0 = max(kA - 2, 1), lmax = min(SG == 0 ? nk : nk - 1, kB + 2);
 
   extern __shared__ __align__(1024) float fsmem[];
   float* ring = fsmem;
@@ -437,11 +441,10 @@ k_force(const __grid_constant__ ForceMaps m, const ForceArgs a) {
   }
   __syncthreads();
 
-  // Levels 1..lmax are staged; level lv lives in slot (lv-1) % S.
   int issued = 0;   // highest level thread 0 has issued
   auto issue = [&](int lv) {
     issued = lv;
-    const int s = (lv - 1) % S;
+    const int s = (lv - lv0) % S;
     float* st = ring + s * L::stage;
     uint64_t* bar = &bars[s];
     mbar_arrive_expect_tx(bar, L::tx_bytes());
@@ -450,29 +453,31 @@ k_force(const __grid_constant__ ForceMaps m, const ForceArgs a) {
       tma_load_3d(st + L::off(q), &m.m[SG][q], xb, j0 + force_slot_r0(SG, q), lv - 1, bar);
   };
   if (tid == 0)
-    for (int lv = 1; lv <= min(S, lmax); ++lv) issue(lv);
+    for (int lv = lv0; lv <= min(lv0 + S - 1, lmax); ++lv) issue(lv);
 
   bool fail = false;
   auto wait_level = [&](int lv) {
-    if (!fail && lv <= lmax) fail = !mbar_wait(&bars[(lv - 1) % S], ((lv - 1) / S) & 1);
+    if (!fail && lv <= lmax) fail = !mbar_wait(&bars[(lv - lv0) % S], ((lv - lv0) / S) & 1);
   };
-  for (int lv = 1; lv <= 3; ++lv) wait_level(lv);
+  for (int lv = lv0; lv <= kA + 1; ++lv) wait_level(lv);
 
   // stages of levels k-2 .. k+2 (those outside 1..lmax hold other levels
   // and are read only by terms the reference's clamping discards)
-  auto slot_ptr = [&](int lv) { return ring + ((lv - 1 + S) % S) * L::stage; };
-  const float* stp[5] = {slot_ptr(0), slot_ptr(1), slot_ptr(2), slot_ptr(3), slot_ptr(4)};
+  auto slot_ptr = [&](int lv) { return ring + ((lv - lv0 + S) % S) * L::stage; };
+  const float* stp[5] = {slot_ptr(kA - 2), slot_ptr(kA - 1), slot_ptr(kA), slot_ptr(kA + 1), slot_ptr(kA + 2)};
   const int rowbase = ty * BX + 2 * tx + 2;         // even: every pair load is 8-byte aligned
   const long long plane = g.plane;
-  long long id = g.at(i, j, 2);
+  long long id = g.at(i, j, kA);
+  // the w group's buoyancy term of the level below the block's first
   F2 wb_prev = f2(0.f);
+  if (SG == 0 && gz == 2 && kA > 2 && (ownA || ownB)) wb_prev = buoyancy(a, tab + (kA - 1) * kNF, id - plane);
 
-  for (int k = 2; k <= kmax; ++k, id += plane) {
+  for (int k = kA; k <= kB; ++k, id += plane) {
     wait_level(k + 2);
     // Every thread has finished level k-1, so the slot of level k-3 (last
     // read as k'-2 at k' = k-1) may be refilled with level k+S-3.
     __syncthreads();
-    if (tid == 0 && !fail && k >= 4 && k + S - 3 <= lmax) {   // refill only after its copy was seen to land
+    if (tid == 0 && !fail && k - 3 >= lv0 && k + S - 3 <= lmax) {   // refill only after its copy was seen to land
       fence_proxy_async_smem();
       issue(k + S - 3);
     }
@@ -498,9 +503,9 @@ k_force(const __grid_constant__ ForceMaps m, const ForceArgs a) {
       if (a.err) atomicExch(a.err, 1);
       for (int s = 0; s < S; ++s) {
         int kl = -1;
-        for (int lv = 1; lv <= issued; ++lv)
-          if ((lv - 1) % S == s) kl = lv;
-        if (kl >= 0) mbar_wait(&bars[s], ((kl - 1) / S) & 1);
+        for (int lv = lv0; lv <= issued; ++lv)
+          if ((lv - lv0) % S == s) kl = lv;
+        if (kl >= 0) mbar_wait(&bars[s], ((kl - lv0) / S) & 1);
       }
     }
   }
@@ -519,7 +524,12 @@ int launch_sg(const ForceArgs& a, const ForceMaps& maps, cudaStream_t st) {
   const int nx = SG == 0 ? g.ni - 2 : g.ni - 3, ny = SG == 0 ? g.nj - 2 : g.nj - 3;
   dim3 block(kFPairs, kForceTY, L::ngroups);
   dim3 grid((nx + kHeviTX - 1) / kHeviTX, (ny + kForceTY - 1) / kForceTY);
-  k_force<SG, T><<<grid, block, bytes, st>>>(maps, a);
+  const int n = (SG == 0 ? g.nk - 1 : g.nk - 2) - 1;   // levels 2..kmax
+  ForceArgs b = a;
+  b.kchunk = level_chunk(n, (long long)grid.x * grid.y,
+                         resident_blocks(k_force<SG, T>, kFPairs * kForceTY * L::ngroups, bytes));
+  grid.z = (n + b.kchunk - 1) / b.kchunk;
+  k_force<SG, T><<<grid, block, bytes, st>>>(maps, b);
   return cudaGetLastError() == cudaSuccess ? 0 : CRESS_E_CUDA;
 }
 

@@ -1,6 +1,8 @@
 // Large-step kernels (forcing, leapfrog scalar step, Asselin filter,
 // periodic halo planes): internal interface.
 #pragma once
+#include <map>
+#include <utility>
 #include <cuda_runtime.h>
 #include "common.cuh"
 #include "hevi.cuh"
@@ -49,6 +51,7 @@ __host__ __device__ __forceinline__ float level_value(int f, int kk, const FB& B
 
 struct ForceArgs {
   Grid g;
+  int kchunk;                 // levels per block (set by the launcher)
   const float* col;           // 1-D columns, C_NFIELDS_ALL x (nk+1)
   const float* lvl;           // level table (nk+1) x kLevelStride for this dtb
   // present level t
@@ -118,6 +121,7 @@ int launch_force(const ForceArgs& a, const ForceMaps& maps, cudaStream_t st);
 // (Ctx::rks_d ...).
 struct TurbArgs {
   Grid g;
+  int kchunk;                 // levels per block (set by the launcher)
   const float* col;
   const float* lvl;           // a level table (rows 0..nk, kLevelStride floats; its dtb is not used)
   const float *up, *vp, *wp, *ptpp, *ppp;                  // t-dt
@@ -135,6 +139,7 @@ int launch_turb_visc(const TurbArgs& a, cudaStream_t st);
 constexpr int kMoistN = 9;
 struct MoistScalarArgs {
   Grid g;
+  int kchunk;                 // levels per block (set by the launcher)
   const float* col;
   const float* lvl;           // level table (nk+1) x kLevelStride for this dtb
   const float* u; const float* v; const float* w;   // present winds (flux rst*u etc.)
@@ -187,5 +192,41 @@ int launch_halo(const HaloArgs& a, cudaStream_t st);
 // layout (pitch ni+2, contiguous) and the device layout (pitch px).
 int launch_repitch(const float* src, int src_pitch, float* dst, int dst_pitch, int w, long long rows,
                    cudaStream_t st);
+
+// Levels each block of a k-marching kernel takes, for n levels over `tiles` xy
+// tiles of which the GPU holds `resident` blocks at once: a block costs its
+// levels plus about five more (the four levels of vertical halo it stages
+// again and its start), and the blocks run in waves.  On a grid with few
+// tiles the column is cut, so that more SMs march it; where the tiles alone
+// fill the GPU the whole column (one chunk) wins.  Measured with and without
+// (forcing, scalars, eddy viscosity, TKE and the HE-VE substep): 4 HE-VE steps of
+// 192x160x48 9.1 -> 3.4 ms (120 tiles, one block per SM before), 15 dry steps of
+// 64x64x40 4.2 -> 3.3 ms, 3 TKE steps of 209x147x57 4.8 -> 4.0 ms; the 512x512x64
+// steps are cut nowhere and unchanged.
+inline int level_chunk(int n, long long tiles, long long resident) {
+  int best = n;
+  double cost = 1e30;
+  for (int z = 1; z <= 16 && z <= n; ++z) {
+    const int c = (n + z - 1) / z;
+    const double t = (double)((tiles * z + resident - 1) / resident) * (c + 5);
+    if (t < cost - 1e-9) { cost = t; best = c; }
+  }
+  return best;
+}
+
+// Blocks of a kernel the GPU holds at once (threads and bytes of shared
+// memory per block), asked for once per thread.
+template <class K>
+inline long long resident_blocks(K kern, int threads, size_t bytes) {
+  thread_local std::map<std::pair<const void*, size_t>, long long> known;
+  long long& n = known[{reinterpret_cast<const void*>(kern), bytes}];
+  if (!n) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, bytes) != cudaSuccess || per_sm < 1)
+      per_sm = 1;
+    n = 148LL * per_sm;
+  }
+  return n;
+}
 
 }  // namespace cress

@@ -28,6 +28,7 @@
 #include <cstdint>
 #include "common.cuh"
 #include "f2.cuh"
+#include "forcing.cuh"
 #include "hevi.cuh"
 #include "tma.cuh"
 
@@ -89,12 +90,16 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
   }
   __syncthreads();
 
-  // Levels 1..nk-1 are staged; level lv lives in slot (lv-1) % S.
-  const int lmax = nk - 1;
+  // This block's levels kA..kB of 1..nk-1 (blockIdx.z): u, v, w of these and
+  // p' of the levels kA-1..kB-1.  It starts two levels lower without storing
+  // (their pressure, faces and w feed the first ones) and stages one level
+  // more; level lv lives in slot (lv-lv0) % S.
+  const int kA = 1 + blockIdx.z * a.kchunk, kB = min(kA + a.kchunk - 1, nk - 1);
+  const int lv0 = max(kA - 2, 1), lmax = min(nk - 1, kB + 1);
   int issued = 0;   // highest level thread 0 has issued
   auto issue = [&](int lv) {
     issued = lv;
-    const int s = (lv - 1) % S;
+    const int s = (lv - lv0) % S;
     float* st = ring + s * L::stage;
     uint64_t* bar = &bars[s];
     const int z = lv - 1;
@@ -109,7 +114,7 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
     tma_load_3d(st + L::oPF, &m.pf, xb, j0, z, bar);
   };
   if (tid == 0)
-    for (int lv = 1; lv <= min(S, lmax); ++lv) issue(lv);
+    for (int lv = lv0; lv <= min(lv0 + S - 1, lmax); ++lv) issue(lv);
 
   constexpr int NH = 2 * TX + 2 * TY;
   int hx = 0, hy = 0;
@@ -145,21 +150,22 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
   F2 t3v_prev = f2(0.f), wb8s_prev = f2(0.f);   // level k-1, rows A and B
   F2 wcn_prev = f2(0.f), wadv_prev = f2(0.f);   // new wc and new w (after vbcw) of level k-1
   F2 hdiv_prev = f2(0.f), pp_prev = f2(0.f), pf_prev = f2(0.f);
-  float p2A = 0.f, p2B = 0.f, p3A = 0.f, p3B = 0.f, pkA = 0.f, pkB = 0.f;
-  float w3A = 0.f, w3B = 0.f, wkA = 0.f, wkB = 0.f;
+  float p2A = 0.f, p2B = 0.f;
   bool fail = false;
   auto wait_level = [&](int lv) {
-    if (!fail && lv <= lmax) fail = !mbar_wait(&bars[(lv - 1) % S], ((lv - 1) / S) & 1);
+    if (!fail && lv <= lmax) fail = !mbar_wait(&bars[(lv - lv0) % S], ((lv - lv0) / S) & 1);
   };
-  wait_level(1);
-  int idA = (int)g.at(i, jA, 1);
+  wait_level(lv0);
+  int idA = (int)g.at(i, jA, lv0);
 
-  for (int k = 1; k <= nk - 1; ++k, idA += plane) {
+  for (int k = lv0; k <= kB; ++k, idA += plane) {
     const int idB = idA + px;
+    // a column's stores at this level
+    const bool stA = ownA && k >= kA, stB = ownB && k >= kA;
     wait_level(k + 1);
     float* t3h = t3hb + (k & 1) * L::t3h_floats;
-    const float* st0 = ring + ((k - 1) % S) * L::stage;
-    const float* st1 = ring + (k % S) * L::stage;   // level k+1 (not staged for k = nk-1)
+    const float* st0 = ring + ((k - lv0) % S) * L::stage;
+    const float* st1 = ring + ((k + 1 - lv0) % S) * L::stage;   // level k+1 (not staged for k = nk-1)
     const float* U = st0 + L::oU;
     const float* V = st0 + L::oV;
     const float* W0 = st0 + L::oW;
@@ -211,7 +217,7 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
     // Every thread has finished level k-1 and written this level's t3h,
     // so the slot of level k-1 may be refilled with level k+S-1.
     __syncthreads();
-    if (tid == 0 && !fail && k >= 2 && k + S - 1 <= lmax) {   // refill only after its copy was seen to land
+    if (tid == 0 && !fail && k > lv0 && k + S - 1 <= lmax) {   // refill only after its copy was seen to land
       fence_proxy_async_smem();
       issue(k + S - 1);
     }
@@ -247,8 +253,8 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
           if (ylast) store_periodic(a.v_new, g, STAG_V, i, j + 1, kc, v1);
         }
       };
-      if (ownA) store_uv(edgeA, ylastA, jA, idA, un0.v.x, un1.v.x, vs.v.x, vn.v.x);
-      if (ownB) store_uv(edgeB, ylastB, jB, idB, un0.v.y, un1.v.y, vs.v.y, vn.v.y);
+      if (stA) store_uv(edgeA, ylastA, jA, idA, un0.v.x, un1.v.x, vs.v.x, vn.v.x);
+      if (stB) store_uv(edgeB, ylastB, jB, idB, un0.v.y, un1.v.y, vs.v.y, vn.v.y);
       // horizontal part of diverpe's divergence (jcb-weighted new winds)
       const float jcb8u = CK(k, C_JCB8U), jcb8v = CK(k, C_JCB8V);
       hdiv = (jcb8u * un0 - jcb8u * un1) * dxiv + (jcb8v * vs - jcb8v * vn) * dyiv;
@@ -265,17 +271,22 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
       wcn = STH ? wn * CK(k, C_IJCB8W) : wn;                                        // phy2cnt.f90:219
       if (k == 2 || k == nk - 1) {
         // vbcw.f90:317,481: w = 0 here; the contravariant value stays
-        if (ownA) put_side(k, jA, wcn.v.x);
-        if (ownB) put_side(k, jB, wcn.v.y);
+        if (stA) put_side(k, jA, wcn.v.x);
+        if (stB) put_side(k, jB, wcn.v.y);
         wadv = f2(0.f);
-        if (ownA) store_periodic(a.w_new, g, STAG_S, i, jA, k, 0.f);
-        if (ownB) store_periodic(a.w_new, g, STAG_S, i, jB, k, 0.f);
+        if (stA) store_periodic(a.w_new, g, STAG_S, i, jA, k, 0.f);
+        if (stB) store_periodic(a.w_new, g, STAG_S, i, jB, k, 0.f);
       } else {
         wadv = wn;
-        if (ownA) { if (edgeA) store_periodic(a.w_new, g, STAG_S, i, jA, k, wn.v.x); else a.w_new[idA] = wn.v.x; }
-        if (ownB) { if (edgeB) store_periodic(a.w_new, g, STAG_S, i, jB, k, wn.v.y); else a.w_new[idB] = wn.v.y; }
-        if (k == 3) { w3A = wcn.v.x; w3B = wcn.v.y; }
-        if (k == nk - 2) { wkA = wcn.v.x; wkB = wcn.v.y; }
+        if (stA) { if (edgeA) store_periodic(a.w_new, g, STAG_S, i, jA, k, wn.v.x); else a.w_new[idA] = wn.v.x; }
+        if (stB) { if (edgeB) store_periodic(a.w_new, g, STAG_S, i, jB, k, wn.v.y); else a.w_new[idB] = wn.v.y; }
+        // vbcw.f90:285,471 images from the contravariant w of levels 3 and nk-2
+        if (k == 3 || k == nk - 2) {
+          const int kc = k == 3 ? 1 : nk;
+          const float j8w = CK(k, C_JCB8W);
+          if (stA) store_periodic(a.w_new, g, STAG_S, i, jA, kc, -j8w * wcn.v.x - 0.f);
+          if (stB) store_periodic(a.w_new, g, STAG_S, i, jB, kc, -j8w * wcn.v.y - 0.f);
+        }
       }
     }
 
@@ -287,11 +298,18 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
       const F2 psml = g05 * (wadv_prev + wadv) * CK(kp, C_RST) + pdiv;                             // advbspe.f90:127
       const F2 pn = pp_prev + dts * (pf_prev + psml) * CK(kp, C_IJCB);                             // steppe.f90:224
       const int ipA = idA - plane, ipB = idB - plane;
-      if (ownA) { if (edgeA) store_periodic(a.p_new, g, STAG_S, i, jA, kp, pn.v.x); else a.p_new[ipA] = pn.v.x; }
-      if (ownB) { if (edgeB) store_periodic(a.p_new, g, STAG_S, i, jB, kp, pn.v.y); else a.p_new[ipB] = pn.v.y; }
+      if (stA) { if (edgeA) store_periodic(a.p_new, g, STAG_S, i, jA, kp, pn.v.x); else a.p_new[ipA] = pn.v.x; }
+      if (stB) { if (edgeB) store_periodic(a.p_new, g, STAG_S, i, jB, kp, pn.v.y); else a.p_new[ipB] = pn.v.y; }
+      // vbcp.f90:126-160 (levels 2 and 3 belong to the first block)
       if (kp == 2) { p2A = pn.v.x; p2B = pn.v.y; }
-      if (kp == 3) { p3A = pn.v.x; p3B = pn.v.y; }
-      if (kp == nk - 2) { pkA = pn.v.x; pkB = pn.v.y; }
+      if (kp == 3) {
+        if (stA) store_periodic(a.p_new, g, STAG_S, i, jA, 1, (a.bbc == 2) ? 2.f * p2A - pn.v.x : p2A);
+        if (stB) store_periodic(a.p_new, g, STAG_S, i, jB, 1, (a.bbc == 2) ? 2.f * p2B - pn.v.y : p2B);
+      }
+      if (kp == nk - 2) {
+        if (stA) store_periodic(a.p_new, g, STAG_S, i, jA, nk - 1, pn.v.x);
+        if (stB) store_periodic(a.p_new, g, STAG_S, i, jB, nk - 1, pn.v.y);
+      }
     }
     t3v_prev = t3v;
     wb8s_prev = wb8s;
@@ -307,30 +325,25 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
       atomicExch(a.err, 1);
       for (int s = 0; s < S; ++s) {
         int kl = -1;
-        for (int lv = 1; lv <= issued; ++lv)
-          if ((lv - 1) % S == s) kl = lv;
-        if (kl >= 0) mbar_wait(&bars[s], ((kl - 1) / S) & 1);
+        for (int lv = lv0; lv <= issued; ++lv)
+          if ((lv - lv0) % S == s) kl = lv;
+        if (kl >= 0) mbar_wait(&bars[s], ((kl - lv0) / S) & 1);
       }
     }
     return;
   }
-  // vbcw.f90:285,471 images (from the contravariant w of levels 3 and
-  // nk-2), vbcp.f90:126-160, and level nk of u, v, p' carried over
-  auto finish = [&](bool own, bool ylast, int j, float w3, float wk, float p2, float p3, float pk) {
+  if (kB < nk - 1) return;
+  // level nk of u, v, p' carried over
+  auto carry = [&](bool own, bool ylast, int j) {
     if (!own) return;
-    const float j8w3 = CK(3, C_JCB8W), j8wt = CK(nk - 2, C_JCB8W);
-    store_periodic(a.w_new, g, STAG_S, i, j, 1, -j8w3 * w3 - 0.f);
-    store_periodic(a.w_new, g, STAG_S, i, j, nk, -j8wt * wk - 0.f);
-    store_periodic(a.p_new, g, STAG_S, i, j, 1, (a.bbc == 2) ? 2.f * p2 - p3 : p2);
-    store_periodic(a.p_new, g, STAG_S, i, j, nk - 1, pk);
     store_periodic(a.p_new, g, STAG_S, i, j, nk, a.p_old[g.at(i, j, nk)]);
     store_periodic(a.u_new, g, STAG_U, i, j, nk, a.u_old[g.at(i, j, nk)]);
     store_periodic(a.v_new, g, STAG_V, i, j, nk, a.v_old[g.at(i, j, nk)]);
     if (xlast) store_periodic(a.u_new, g, STAG_U, i + 1, j, nk, a.u_old[g.at(i + 1, j, nk)]);
     if (ylast) store_periodic(a.v_new, g, STAG_V, i, j + 1, nk, a.v_old[g.at(i, j + 1, nk)]);
   };
-  finish(ownA, ylastA, jA, w3A, wkA, p2A, p3A, pkA);
-  finish(ownB, ylastB, jB, w3B, wkB, p2B, p3B, pkB);
+  carry(ownA, ylastA, jA);
+  carry(ownB, ylastB, jB);
 }
 
 template <int DIV, bool STH, bool BUY>
@@ -344,7 +357,13 @@ int launch_e(const HeviArgs& a, const HeviMaps& maps, cudaStream_t st) {
     return CRESS_E_CUDA;
   dim3 block(kHeviTX, kVRows);
   dim3 grid((g.ni - 3 + kHeviTX - 1) / kHeviTX, (g.nj - 3 + kVTY - 1) / kVTY);
-  kern<<<grid, block, bytes, st>>>(maps, a);
+  // the first block takes levels 1..4 at least (p' of levels 2 and 3)
+  const int n = g.nk - 1;
+  HeviArgs b = a;
+  b.kchunk = level_chunk(n, (long long)grid.x * grid.y, resident_blocks(kern, kHeviTX * kVRows, bytes));
+  if (b.kchunk < 4) b.kchunk = 4;
+  grid.z = (n + b.kchunk - 1) / b.kchunk;
+  kern<<<grid, block, bytes, st>>>(maps, b);
   return cudaGetLastError() == cudaSuccess ? 0 : CRESS_E_CUDA;
 }
 

@@ -82,6 +82,7 @@ struct HeviArgs {
   const float* wc_old;
   float* wc_new;
   int wc_from_w;
+  int kchunk;             // HE-VE: levels per block (set by the launcher)
   float dts, dxiv, dyiv, dziv, divch, divcv, weicoe, dtdzw, dtw, g05, g05n;
   int divopt, buyopt, sthopt, bbc;
   // probes of each ring wait of the k_hevi2 level loop before it gives up

@@ -38,7 +38,7 @@
 // tiles leaves SMs idle; a substep also spent about 270 warp instructions per 32
 // cells, half of them on ring, address and halo bookkeeping.  Here the levels
 // of a row run at once, the strip length adapts to the grid, and it is about
-// 150 per 32 cells.  It is bound by the latency of its 16 warps per SM: 128 registers each
+// 170 per 32 cells.  It is bound by the latency of its 16 warps per SM: 128 registers each
 // (which is why a row's p' tendency and w right-hand side wait in
 // shared memory, and why per-row addresses are formed again each row), two
 // barriers per row.  Tried and slower: direct global loads instead of TMA (406 us at

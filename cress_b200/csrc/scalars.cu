@@ -102,12 +102,14 @@ k_scalars(const __grid_constant__ MoistMaps m, const MoistScalarArgs a) {
   }
   __syncthreads();
 
-  // Levels 1..nk-1 are staged; level lv lives in slot (lv-1) % S.
-  const int lmax = nk - 1;
+  // this block's levels kA..kB of 2..nk-2 (blockIdx.z), and the levels it
+  // stages, two more at either end; level lv lives in slot (lv-lv0) % S
+  const int kA = 2 + blockIdx.z * a.kchunk, kB = min(kA + a.kchunk - 1, nk - 2);
+  const int lv0 = max(kA - 2, 1), lmax = min(nk - 1, kB + 2);
   int issued = 0;   // highest level thread 0 has issued
   auto issue = [&](int lv) {
     issued = lv;
-    const int s = (lv - 1) % S;
+    const int s = (lv - lv0) % S;
     float* st = ring + s * L::stage;
     uint64_t* bar = &bars[s];
     const int z = lv - 1;
@@ -122,13 +124,13 @@ k_scalars(const __grid_constant__ MoistMaps m, const MoistScalarArgs a) {
     if constexpr (TURB) tma_load_3d(st + L::oR, &m.rkv, xb, j0 - 2, z, bar);
   };
   if (tid == 0)
-    for (int lv = 1; lv <= min(S, lmax); ++lv) issue(lv);
+    for (int lv = lv0; lv <= min(lv0 + S - 1, lmax); ++lv) issue(lv);
 
   bool fail = false;
   auto wait_level = [&](int lv) {
-    if (!fail && lv <= lmax) fail = !mbar_wait(&bars[(lv - 1) % S], ((lv - 1) / S) & 1);
+    if (!fail && lv <= lmax) fail = !mbar_wait(&bars[(lv - lv0) % S], ((lv - lv0) / S) & 1);
   };
-  for (int lv = 1; lv <= 3; ++lv) wait_level(lv);
+  for (int lv = lv0; lv <= kA + 1; ++lv) wait_level(lv);
 
   const float oned24 = 1.f / 24.f, fourd3 = 4.f / 3.f;
   const float dxv24 = oned24 * a.dxiv, dyv24 = oned24 * a.dyiv;
@@ -144,18 +146,18 @@ k_scalars(const __grid_constant__ MoistMaps m, const MoistScalarArgs a) {
   const int oS = q * 2 * L::sbox + (ty + 2) * BX + ox;   // own pair of this species' boxes
   const int oR = (ty + 2) * BX + ox;                     // own pair of the viscosity box
   const long long plane = g.plane;
-  long long id = g.at(i, j, 2);
+  long long id = g.at(i, j, kA);
   // stages of levels k-2 .. k+2 (those outside 1..nk-1 hold other levels
   // and are read only by terms the reference's clamping discards)
-  auto slot_ptr = [&](int lv) { return ring + ((lv - 1 + S) % S) * L::stage; };
-  const float* stp[5] = {slot_ptr(0), slot_ptr(1), slot_ptr(2), slot_ptr(3), slot_ptr(4)};
+  auto slot_ptr = [&](int lv) { return ring + ((lv - lv0 + S) % S) * L::stage; };
+  const float* stp[5] = {slot_ptr(kA - 2), slot_ptr(kA - 1), slot_ptr(kA), slot_ptr(kA + 1), slot_ptr(kA + 2)};
 
-  for (int k = 2; k <= nk - 2; ++k, id += plane) {
+  for (int k = kA; k <= kB; ++k, id += plane) {
     wait_level(k + 2);
     // Every thread has finished level k-1, so the slot of level k-3 (last
     // read as k'-2 at k' = k-1) may be refilled with level k+S-3.
     __syncthreads();
-    if (tid == 0 && !fail && k >= 4 && k + S - 3 <= lmax) {   // refill only after its copy was seen to land
+    if (tid == 0 && !fail && k - 3 >= lv0 && k + S - 3 <= lmax) {   // refill only after its copy was seen to land
       fence_proxy_async_smem();
       issue(k + S - 3);
     }
@@ -251,9 +253,9 @@ k_scalars(const __grid_constant__ MoistMaps m, const MoistScalarArgs a) {
       if (a.err) atomicExch(a.err, 1);
       for (int s = 0; s < S; ++s) {
         int kl = -1;
-        for (int lv = 1; lv <= issued; ++lv)
-          if ((lv - 1) % S == s) kl = lv;
-        if (kl >= 0) mbar_wait(&bars[s], ((kl - 1) / S) & 1);
+        for (int lv = lv0; lv <= issued; ++lv)
+          if ((lv - lv0) % S == s) kl = lv;
+        if (kl >= 0) mbar_wait(&bars[s], ((kl - lv0) / S) & 1);
       }
     }
   }
@@ -271,7 +273,12 @@ int launch_sc(const MoistScalarArgs& a, const MoistMaps& maps, cudaStream_t st) 
   const int nx = g.ni - 3, ny = g.nj - 3;
   dim3 block(kScPairs, kScalarTY, kScGroup);
   dim3 grid((nx + kHeviTX - 1) / kHeviTX * (kMoistN / kScGroup), (ny + kScalarTY - 1) / kScalarTY);
-  k_scalars<S, TURB><<<grid, block, bytes, st>>>(maps, a);
+  const int n = g.nk - 3;   // levels 2..nk-2
+  MoistScalarArgs b = a;
+  b.kchunk = level_chunk(n, (long long)grid.x * grid.y,
+                         resident_blocks(k_scalars<S, TURB>, kScPairs * kScalarTY * kScGroup, bytes));
+  grid.z = (n + b.kchunk - 1) / b.kchunk;
+  k_scalars<S, TURB><<<grid, block, bytes, st>>>(maps, b);
   return cudaGetLastError() == cudaSuccess ? 0 : CRESS_E_CUDA;
 }
 

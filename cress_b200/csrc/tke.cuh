@@ -17,6 +17,7 @@ struct TkeRows {
 
 struct TkeArgs {
   Grid g;
+  int kchunk;                            // levels per block (set by the launcher)
   const float* lvl;                      // level table (nk+1) x kLevelStride for this dtb
   // per point from k_turb_visc: 1/Pr*rkv/jcb, N^2 at w level k, shear
   // production and dissipation

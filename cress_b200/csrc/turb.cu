@@ -35,7 +35,7 @@ namespace {
 constexpr float kRd = 287.f, kCp = 1004.f, kEpsva = .622f, kEpsav = 1.6077f, kTlow = 233.16f;
 constexpr float kLv0 = 2.50078e6f, kLf0 = 3.34e5f, kT0 = 273.16f, kCwmci = 4.218e3f - 2.106e3f;
 
-// Each thread owns one column (i, j) and marches k = 1..nk-1 upward, so the
+// Each thread owns one column (i, j) and marches its block's levels upward, so the
 // thermodynamics of a level (bruntv's theta, and in moist air its
 // saturated and virtual forms, which cost five exp/log each) is formed
 // once and serves N^2 at the w levels below and above it, and the z-x /
@@ -108,15 +108,19 @@ __global__ void __launch_bounds__(kTurbThreads) k_turb_visc(const TurbArgs a) {
     return gdzv * d / (C(C_JCB8W, kk) * (b0 + b1));
   };
 
-  Lev lc = lev(2);   // the upper level of the last N^2 formed
+  // this block's levels (blockIdx.z); a chunk that starts above the ground
+  // forms the N^2 and the faces it would have from the level below again
+  const int kA = 1 + blockIdx.z * a.kchunk, kB = min(kA + a.kchunk - 1, nk - 1);
+  Lev lc = lev(max(kA, 2));   // the upper level of the last N^2 formed
   float nq = 0.f, c31_0 = 0.f, c31_1 = 0.f, c32_0 = 0.f, c32_1 = 0.f;
-  for (int k = 1; k <= nk - 1; ++k) {
+  if (kA > 1) nq = nsqv(lev(kA - 1), lc, kA);
+  for (int k = kA; k <= kB; ++k) {
     const long long id = id0 + (long long)(k - 1) * pl;
     auto U = [&](int x, int y, int z) { return __ldg(a.up + id + x + y * px + z * pl); };
     auto V = [&](int x, int y, int z) { return __ldg(a.vp + id + x + y * px + z * pl); };
     auto W = [&](int x, int y, int z) { return __ldg(a.wp + id + x + y * px + z * pl); };
     const auto D = deform_at(C, U, V, W, k, nk, a.dxiv, a.dyiv, a.dziv);
-    if (k == 1) {
+    if (k == kA) {
       c31_0 = D.s31(0, 0, 0); c31_1 = D.s31(1, 0, 0);
       c32_0 = D.s32(0, 0, 0); c32_1 = D.s32(0, 1, 0);
     }
@@ -182,10 +186,15 @@ int launch_turb_visc(const TurbArgs& a, cudaStream_t st) {
   if (bytes > 48 * 1024) return CRESS_E_UNSUPPORTED;
   dim3 b(32, kTurbThreads / 32, 1);
   dim3 gr((a.g.ni - 1 + 31) / 32, (a.g.nj - 1 + b.y - 1) / b.y, 1);
+  const int n = a.g.nk - 1;   // levels 1..nk-1
+  TurbArgs t = a;
+  t.kchunk = level_chunk(n, (long long)gr.x * gr.y,
+                         resident_blocks(a.tkep ? k_turb_visc<true> : k_turb_visc<false>, kTurbThreads, bytes));
+  gr.z = (n + t.kchunk - 1) / t.kchunk;
   if (a.tkep)
-    k_turb_visc<true><<<gr, b, bytes, st>>>(a);
+    k_turb_visc<true><<<gr, b, bytes, st>>>(t);
   else
-    k_turb_visc<false><<<gr, b, bytes, st>>>(a);
+    k_turb_visc<false><<<gr, b, bytes, st>>>(t);
   return cudaGetLastError() == cudaSuccess ? 0 : CRESS_E_CUDA;
 }
 

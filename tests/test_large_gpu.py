@@ -99,3 +99,12 @@ def test_dry_large_steps_heve(cress, oracle_lib):
     # the explicit small step (impopt=0) inside whole large steps
     dims, ref, got = run_case(cress, oracle_lib, 40, 32, 24, 3, seed=7, impopt=0)
     check(dims, ref, got)
+
+
+@pytest.mark.parametrize("impopt", [0, 1])
+@pytest.mark.parametrize("nz", [5, 6, 9, 14, 33])
+def test_cut_columns(cress, oracle_lib, nz, impopt):
+    # few tiles: the k-marching kernels cut the column, down to one level per
+    # block (HE-VE: four), with a short last piece
+    dims, ref, got = run_case(cress, oracle_lib, 33, 20, nz, 2, seed=nz, tubopt=1, impopt=impopt)
+    check(dims, ref, got)
