@@ -53,6 +53,10 @@ struct GemmArgs {
   bf16* out_bf; int ldb;
   bf16* out_bt; int ldt;
   int* err;
+  // > 1: K is cut into this many parts, one CTA each per tile, and their FP32
+  // sums are added into out_f32 (the only output, zeroed by the caller; no
+  // bias or activation)
+  int split;
 };
 int gemm_bf16(const bf16* A, int lda, const bf16* B, int ldb, const GemmArgs& g, cudaStream_t st);
 

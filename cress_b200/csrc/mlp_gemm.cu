@@ -9,7 +9,12 @@
 // issues the tcgen05.mma K steps (4 per stage) into a 128 x BN FP32
 // accumulator in tensor memory and commits each stage back to its producer
 // barrier; all eight warps then read the accumulator (warp w owns rows
-// 32(w%4)..+31 and half of the columns) and apply the epilogue.  Every mbarrier wait is bounded: on timeout the kernel records
+// 32(w%4)..+31 and half of the columns) and apply the epilogue.
+//
+// Split K (GemmArgs::split): the weight gradients have one or two tiles of
+// output and K = the batch, so with one CTA per tile two SMs walk 128 K steps
+// while 146 idle.  Cut into parts, each CTA adds its FP32 accumulator into
+// the output with 16-byte reductions.  Every mbarrier wait is bounded: on timeout the kernel records
 // CRESS_E_TIMEOUT in the error word, waits (bounded) for its issued copies
 // and MMAs, frees tensor memory and returns.
 #include <cuda.h>
@@ -53,7 +58,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   __shared__ int fail;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
-  const int KB = g.K / kBK;
+  // this CTA's part of K, in steps of kBK
+  const int KT = g.K / kBK, split = g.split > 1 ? g.split : 1;
+  const int kb0 = (int)((long long)KT * blockIdx.z / split), KB = (int)((long long)KT * (blockIdx.z + 1) / split) - kb0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
@@ -81,8 +88,8 @@ __global__ void __launch_bounds__(kThreads, 2)
       }
       unsigned char* a = sm + s * Cfg::STAGE;
       mbar_arrive_expect_tx(&full[s], Cfg::STAGE);
-      tma_load_2d(a, &ta, kb * kBK, m0, &full[s]);
-      tma_load_2d(a + Cfg::A_BYTES, &tb, kb * kBK, n0, &full[s]);
+      tma_load_2d(a, &ta, (kb0 + kb) * kBK, m0, &full[s]);
+      tma_load_2d(a + Cfg::A_BYTES, &tb, (kb0 + kb) * kBK, n0, &full[s]);
       ++issued;
     }
     if (*vfail) {
@@ -138,7 +145,15 @@ __global__ void __launch_bounds__(kThreads, 2)
         a[j] = o;
         r[j] = __float_as_uint(g.act == 1 ? v : o);
       }
-      if (g.out_f32) {
+      if (split > 1) {
+        float* dst = g.out_f32 + (size_t)row * g.ldf + col0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * q),
+                       "f"(__uint_as_float(r[4 * q])), "f"(__uint_as_float(r[4 * q + 1])),
+                       "f"(__uint_as_float(r[4 * q + 2])), "f"(__uint_as_float(r[4 * q + 3]))
+                       : "memory");
+      } else if (g.out_f32) {
         float4* dst = reinterpret_cast<float4*>(g.out_f32 + (size_t)row * g.ldf + col0);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
@@ -214,7 +229,7 @@ int launch_gemm(const bf16* A, int lda, const bf16* B, int ldb, const GemmArgs& 
   if (cudaFuncSetAttribute(k_gemm_bf16<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) !=
       cudaSuccess)
     return set_error(CRESS_E_CUDA, "gemm smem attribute");
-  dim3 grid(g.M / kBM, g.N / BN);
+  dim3 grid(g.M / kBM, g.N / BN, g.split > 1 ? g.split : 1);
   k_gemm_bf16<BN><<<grid, kThreads, Cfg::SMEM, st>>>(ta, tb, g);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? CRESS_OK : set_error(CRESS_E_CUDA, "gemm launch: %s", cudaGetErrorString(e));
@@ -237,6 +252,8 @@ int gemm_bf16(const bf16* A, int lda, const bf16* B, int ldb, const GemmArgs& g,
       (g.out_bf && (g.ldb % 8 || g.ldb < g.N || !aligned16(g.out_bf))) || (g.out_bt && g.ldt < g.M) ||
       (g.act == 2 && (!g.aux || g.ldaux < g.N)))
     return set_error(CRESS_E_ARG, "gemm: bad output / aux leading dimensions");
+  if (g.split > 1 && (!g.out_f32 || g.out_bf || g.out_bt || g.bias || g.act || g.split > g.K / kBK))
+    return set_error(CRESS_E_ARG, "gemm: a split K takes a plain FP32 output and at most K / 64 parts");
   if (g.N % 256 == 0) return launch_gemm<256>(A, lda, B, ldb, g, st);
   if (g.N % 128 == 0) return launch_gemm<128>(A, lda, B, ldb, g, st);
   return launch_gemm<64>(A, lda, B, ldb, g, st);

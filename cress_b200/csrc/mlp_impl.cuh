@@ -44,6 +44,7 @@ struct Mlp {
   float *y = nullptr, *t = nullptr, *dy = nullptr, *dz = nullptr;
   bf16 *dyb = nullptr, *dyt = nullptr, *dzb = nullptr, *dzt = nullptr;
   int* idx_d = nullptr;
+  float* xf = nullptr;              // [B][16] host inputs of forward and loss_grad
   // tuple store: transformed features [n][16] and raw tendencies [n][9]
   float *tx = nullptr, *ty = nullptr;
   long long ntup = 0, tcap = 0;

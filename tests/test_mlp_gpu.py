@@ -64,6 +64,27 @@ def test_backward_matches_oracle(cress):
         assert err <= 5e-3 * scale, f"{name}: max err {err:.3e} of scale {scale:.3e}"
 
 
+@pytest.mark.parametrize("n", [128, 384, 512, 1152, 19072])
+def test_weight_gradient_split(cress, n):
+    """Batches around the split of K in the weight gradients: none (below 512),
+    two parts, uneven parts, the most parts; same bar as above."""
+    rng = np.random.default_rng(n)
+    p = random_params(2)
+    x = rng.standard_normal((n, 16)).astype(np.float32)
+    t = rng.standard_normal((n, 9)).astype(np.float32)
+    m = cress.Mlp(seed=1)
+    m.set_params(p)
+    loss, g = m.loss_grad(x, t)
+    m.close()
+    lr, gr = M.loss_grad(p.astype(np.float64), x.astype(np.float64), t.astype(np.float64))
+    assert abs(loss - lr) <= 1e-3 * abs(lr)
+    o = 0
+    for name, k in M.SIZES:
+        a, b = g[o:o + k], gr[o:o + k]
+        o += k
+        assert float(np.abs(a - b).max()) <= 5e-3 * (float(np.abs(b).max()) + 1e-30), name
+
+
 def test_training_reduces_loss(cress):
     rng = np.random.default_rng(7)
     x = rng.standard_normal((40960, 16)).astype(np.float32)
