@@ -25,6 +25,14 @@
 // of x-neighbouring columns and computes both with packed FP32x2
 // arithmetic (f2.cuh).  The theta' and moisture values of the buoyancy are
 // read from global memory on the thread's own columns, each once.
+//
+// What bounds it: instruction issue.  Every advection term is a sum of (wind
+// sum) x (difference) with the per-level constants factored out of it, the
+// smoothing one weighted sum per direction (stencil.cuh): 926 -> 870 us for
+// both kernels at 512 x 512 x 64 with the eddy mixing.  The launch bounds
+// name the blocks per SM that the rings leave room for (two with the eddy
+// viscosity staged, three without), so that the registers are used up: left
+// to itself the compiler took 56 and spilled (645 against 609 us, momentum).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -78,9 +86,6 @@ __host__ __device__ constexpr int force_slot(int G, int q) {
                 : (q == 0 ? 1 : q == 1 ? 4 : q == 2 ? 5 : q == 3 ? 6 : q == 4 ? 3 : 7);
 }
 
-// F2 of two consecutive floats of a global field (8-byte aligned index).
-__device__ __forceinline__ F2 gld2(const float* p) { return F2{__ldg(reinterpret_cast<const float2*>(p))}; }
-
 // The buoyancy term of one level (ck: its row of the level table) at the
 // thread's pair, g05 rst (...): dry, or moist with the total condensate.
 __device__ __forceinline__ F2 buoyancy(const ForceArgs& a, const float* ck, long long id) {
@@ -116,7 +121,7 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
   const float dxv24 = oned24 * dxiv, dyv24 = oned24 * dyiv;
   const float dxv48 = .5f * dxv24, dyv48 = .5f * dyv24;
   const float dzv24 = oned24 * dziv, dzv48 = .5f * dzv24;
-  const float dxv05n = -.5f * dxiv, dyv05n = -.5f * dyiv, dzv05n = -.5f * dziv;
+  const float dzv05n = -.5f * dziv;
   const bool smooth = (a.smtopt % 10 == 2) || (a.smtopt % 10 == 3);
   // advopt=3: 4th-order vertical advection on the levels 3..nk-3 (w: 3..nk-2)
   const bool adv3 = a.advopt == 3 && k >= 3 && k <= (G == 2 ? nk - 2 : nk - 3);
@@ -129,8 +134,8 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
   };
   // the pair's result: one 8-byte store, or the first point alone
   auto put = [&](float* out, long long at, F2 v) {
-    if (ownB) *reinterpret_cast<float2*>(out + at) = v.v;
-    else out[at] = v.v.x;
+    if (ownB) st2(out + at, v);
+    else out[at] = v.x();
   };
   // present u, v, w (fields 0-2 of the momentum groups in their own order,
   // fields 1-3 of the scalar groups)
@@ -140,13 +145,22 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
   auto Uc = [&](int dx, int dy, int dz) { return X(qU, dx, dy, dz); };
   auto Vc = [&](int dx, int dy, int dz) { return X(qV, dx, dy, dz); };
   auto Wc = [&](int dx, int dy, int dz) { return X(qW, dx, dy, dz); };
-  // flux helpers of rstuvwc.f90:172-210 (wc = w / jcb8w when stretched, phy2cnt.f90:219)
-  auto RXU = [&](int dx, int dy, int dz) { return C(C_RST8U, k + dz) * Uc(dx, dy, dz); };
-  auto RXV = [&](int dx, int dy, int dz) { return C(C_RST8V, k + dz) * Vc(dx, dy, dz); };
-  auto WC = [&](int dx, int dy, int dz) {
-    return a.sthopt ? Wc(dx, dy, dz) * C(C_IJCB8W, k + dz) : Wc(dx, dy, dz);
+  // Advection is written as sums of (wind sum) x (difference), each times one
+  // per-level constant: the rst or jcb weights of rstuvwc.f90:172-210, the
+  // grid spacing and the 4/3 of the 4th-order form (wc = w / jcb8w when
+  // stretched, phy2cnt.f90:219).
+  const float ru = C(C_RST8U, k), rv = C(C_RST8V, k);
+  auto rw = [&](int z) { return a.sthopt ? C(C_RST8W, k + z) * C(C_IJCB8W, k + z) : C(C_RST8W, k + z); };
+  // 2nd-order sums Sx, Sy (coefficients cx, cy) and 4th-order sums Px, Py (dx,
+  // dy); open x: the 2nd-order form in the boundary columns
+  auto hsum = [&](F2 f, F2 Sx, F2 Sy, F2 Px, F2 Py, float cx, float cy, float px, float py) {
+    F2 r = fma2(f2(fourd3 * cx), Sx, f);
+    r = fma2(f2(fourd3 * cy), Sy, r);
+    r = fma2(f2(px), Px, r);
+    r = fma2(f2(py), Py, r);
+    if (edge) r = sel2(edge, fma2(f2(cy), Sy, fma2(f2(cx), Sx, f)), r);
+    return r;
   };
-  auto RXW = [&](int dx, int dy, int dz) { return C(C_RST8W, k + dz) * WC(dx, dy, dz); };
 
   if constexpr (G == 0) {
     // ------------------------------------------------------------ ufrc
@@ -169,11 +183,9 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
       f = ((A(0) - A(-1)) * dxiv + (Cc(1) - Cc(0)) * (.5f * dyiv)) + (T13(1) - T13(0)) * dziv;
     }
     if (smooth) {
-      auto A = [&](int dx, int dy, int dz) {
-        const int kk = k + dz;
-        return C(C_RST8U, kk) * (UP(dx, dy, dz) - C(C_UBR, kk)) * C(D_IJCB8U, kk);
-      };
-      f = smooth_tile(f, a.smtopt, a.smhcoe, a.smvcoe, k, 2, nk - 2, A, edge);
+      auto H = [&](int dx, int dy) { return UP(dx, dy, 0); };
+      auto A = [&](int dz) { return C(C_RST8U, k + dz) * C(D_IJCB8U, k + dz) * (UP(0, 0, dz) - C(C_UBR, k + dz)); };
+      f = smooth_sum(f, a.smtopt, a.smhcoe * (ru * C(D_IJCB8U, k)), a.smvcoe, k, 2, nk - 2, H, A, edge);
     }
     if (a.vspopt >= 1 && a.vsp_u && k >= a.ksp0 - 1) {
       const float r8s = .25f * (C(C_RBCT, k) + C(C_RBCT, k + 1));
@@ -185,30 +197,23 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
       const F2 c1 = a.fc * rst * (Vc(0, 0, 0) + Vc(0, 1, 0));
       f = f + (c0 + c1);
     }
-    // advuvw.f90:231-397
-    auto t1 = [&](int x) { return (RXU(x, 0, 0) + RXU(x + 1, 0, 0)) * (Uc(x + 1, 0, 0) - Uc(x, 0, 0)) * dxv25n; };
-    auto t2 = [&](int y) { return (RXV(-1, y, 0) + RXV(0, y, 0)) * (Uc(0, y, 0) - Uc(0, y - 1, 0)) * dyv25n; };
-    auto t3 = [&](int z) { return (RXW(-1, 0, z) + RXW(0, 0, z)) * (Uc(0, 0, z) - Uc(0, 0, z - 1)) * dzv25n; };
-    F2 hadv = (t1(-1) + t1(0)) + (t2(0) + t2(1));
-    auto t1w = [&](int x) {
-      return (RXU(x - 1, 0, 0) + RXU(x + 1, 0, 0)) * (Uc(x + 1, 0, 0) - Uc(x - 1, 0, 0)) * dxv24;
-    };
-    auto t2w = [&](int y) {
-      return ((RXV(-1, y, 0) + RXV(0, y, 0)) + (RXV(-1, y + 1, 0) + RXV(0, y + 1, 0))) *
-             (Uc(0, y + 1, 0) - Uc(0, y - 1, 0)) * dyv48;
-    };
-    const F2 h2 = hadv;
-    hadv = fourd3 * hadv + ((t1w(-1) + t1w(1)) + (t2w(-1) + t2w(1)));
-    if (edge) hadv = sel2(edge, h2, hadv);
-    F2 vadv = t3(0) + t3(1);
+    // advuvw.f90:231-430
+    const F2 c = Uc(0, 0, 0), ue = Uc(1, 0, 0), uw = Uc(-1, 0, 0), ue2 = Uc(2, 0, 0), uw2 = Uc(-2, 0, 0);
+    auto Vs = [&](int y) { return Vc(-1, y, 0) + Vc(0, y, 0); };
+    const F2 v0 = Vs(0), v1 = Vs(1);
+    f = hsum(f, (uw + c) * (c - uw) + (c + ue) * (ue - c), v0 * (c - Uc(0, -1, 0)) + v1 * (Uc(0, 1, 0) - c),
+             (uw2 + c) * (c - uw2) + (c + ue2) * (ue2 - c),
+             (Vs(-1) + v0) * (c - Uc(0, -2, 0)) + (v1 + Vs(2)) * (Uc(0, 2, 0) - c), dxv25n * ru, dyv25n * rv,
+             dxv24 * ru, dyv48 * rv);
+    auto Ws = [&](int z) { return rw(z) * (Wc(-1, 0, z) + Wc(0, 0, z)); };
+    const F2 w0 = Ws(0), w1 = Ws(1);
+    const F2 z2 = w0 * (c - Uc(0, 0, -1)) + w1 * (Uc(0, 0, 1) - c);
     if (adv3) {   // advuvw.f90:399-430
-      auto t3w = [&](int z) {
-        return ((RXW(-1, 0, z) + RXW(0, 0, z)) + (RXW(-1, 0, z + 1) + RXW(0, 0, z + 1))) *
-               (Uc(0, 0, z + 1) - Uc(0, 0, z - 1)) * dzv48;
-      };
-      vadv = fourd3 * vadv + (t3w(-1) + t3w(1));
+      f = fma2(f2(fourd3 * dzv25n), z2, f);
+      f = fma2(f2(dzv48), (Ws(-1) + w0) * (c - Uc(0, 0, -2)) + (w1 + Ws(2)) * (Uc(0, 0, 2) - c), f);
+    } else {
+      f = fma2(f2(dzv25n), z2, f);
     }
-    f = f + hadv + vadv;
     put(a.ufrc, id, f);
   } else if constexpr (G == 1) {
     // ------------------------------------------------------------ vfrc
@@ -231,11 +236,9 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
       f = ((B(0) - B(-1)) * dyiv + (Cc(1) - Cc(0)) * (.5f * dxiv)) + (T23(1) - T23(0)) * dziv;
     }
     if (smooth) {
-      auto A = [&](int dx, int dy, int dz) {
-        const int kk = k + dz;
-        return C(C_RST8V, kk) * (VP(dx, dy, dz) - C(C_VBR, kk)) * C(D_IJCB8V, kk);
-      };
-      f = smooth_tile(f, a.smtopt, a.smhcoe, a.smvcoe, k, 2, nk - 2, A, edge);
+      auto H = [&](int dx, int dy) { return VP(dx, dy, 0); };
+      auto A = [&](int dz) { return C(C_RST8V, k + dz) * C(D_IJCB8V, k + dz) * (VP(0, 0, dz) - C(C_VBR, k + dz)); };
+      f = smooth_sum(f, a.smtopt, a.smhcoe * (rv * C(D_IJCB8V, k)), a.smvcoe, k, 2, nk - 2, H, A, edge);
     }
     if (a.vspopt >= 1 && a.vsp_v && k >= a.ksp0 - 1) {
       const float r8s = .25f * (C(C_RBCT, k) + C(C_RBCT, k + 1));
@@ -247,30 +250,22 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
       const F2 c1 = -a.fc * rst * (Uc(0, 0, 0) + Uc(1, 0, 0));
       f = f + (c0 + c1);
     }
-    // advuvw.f90:458-624
-    auto t1 = [&](int x) { return (RXU(x, -1, 0) + RXU(x, 0, 0)) * (Vc(x, 0, 0) - Vc(x - 1, 0, 0)) * dxv25n; };
-    auto t2 = [&](int y) { return (RXV(0, y, 0) + RXV(0, y + 1, 0)) * (Vc(0, y + 1, 0) - Vc(0, y, 0)) * dyv25n; };
-    auto t3 = [&](int z) { return (RXW(0, -1, z) + RXW(0, 0, z)) * (Vc(0, 0, z) - Vc(0, 0, z - 1)) * dzv25n; };
-    F2 hadv = (t1(0) + t1(1)) + (t2(-1) + t2(0));
-    auto t1w = [&](int x) {
-      return ((RXU(x, -1, 0) + RXU(x, 0, 0)) + (RXU(x + 1, -1, 0) + RXU(x + 1, 0, 0))) *
-             (Vc(x + 1, 0, 0) - Vc(x - 1, 0, 0)) * dxv48;
-    };
-    auto t2w = [&](int y) {
-      return (RXV(0, y - 1, 0) + RXV(0, y + 1, 0)) * (Vc(0, y + 1, 0) - Vc(0, y - 1, 0)) * dyv24;
-    };
-    const F2 h2 = hadv;
-    hadv = fourd3 * hadv + ((t1w(-1) + t1w(1)) + (t2w(-1) + t2w(1)));
-    if (edge) hadv = sel2(edge, h2, hadv);
-    F2 vadv = t3(0) + t3(1);
+    // advuvw.f90:458-657
+    const F2 c = Vc(0, 0, 0), vn = Vc(0, 1, 0), vs = Vc(0, -1, 0), vn2 = Vc(0, 2, 0), vs2 = Vc(0, -2, 0);
+    auto Us = [&](int x) { return Uc(x, -1, 0) + Uc(x, 0, 0); };
+    const F2 u0 = Us(0), u1 = Us(1);
+    f = hsum(f, u0 * (c - Vc(-1, 0, 0)) + u1 * (Vc(1, 0, 0) - c), (vs + c) * (c - vs) + (c + vn) * (vn - c),
+             (Us(-1) + u0) * (c - Vc(-2, 0, 0)) + (u1 + Us(2)) * (Vc(2, 0, 0) - c),
+             (vs2 + c) * (c - vs2) + (c + vn2) * (vn2 - c), dxv25n * ru, dyv25n * rv, dxv48 * ru, dyv24 * rv);
+    auto Ws = [&](int z) { return rw(z) * (Wc(0, -1, z) + Wc(0, 0, z)); };
+    const F2 w0 = Ws(0), w1 = Ws(1);
+    const F2 z2 = w0 * (c - Vc(0, 0, -1)) + w1 * (Vc(0, 0, 1) - c);
     if (adv3) {   // advuvw.f90:626-657
-      auto t3w = [&](int z) {
-        return ((RXW(0, -1, z) + RXW(0, 0, z)) + (RXW(0, -1, z + 1) + RXW(0, 0, z + 1))) *
-               (Vc(0, 0, z + 1) - Vc(0, 0, z - 1)) * dzv48;
-      };
-      vadv = fourd3 * vadv + (t3w(-1) + t3w(1));
+      f = fma2(f2(fourd3 * dzv25n), z2, f);
+      f = fma2(f2(dzv48), (Ws(-1) + w0) * (c - Vc(0, 0, -2)) + (w1 + Ws(2)) * (Vc(0, 0, 2) - c), f);
+    } else {
+      f = fma2(f2(dzv25n), z2, f);
     }
-    f = f + hadv + vadv;
     put(a.vfrc, id, f);
   } else if constexpr (G == 2) {
     // ------------------------------------------------------------ wfrc
@@ -294,11 +289,9 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
       f = (T33(0) - T33(-1)) * dziv + ((Aw(1) - Aw(0)) * (.5f * dxiv) + (Cw(1) - Cw(0)) * (.5f * dyiv));
     }
     if (smooth) {
-      auto A = [&](int dx, int dy, int dz) {
-        const int kk = k + dz;
-        return C(C_RST8W, kk) * WP(dx, dy, dz) * C(C_IJCB8W, kk);
-      };
-      f = smooth_tile(f, a.smtopt, a.smhcoe, a.smvcoe, k, 2, nk - 1, A, edge);
+      auto H = [&](int dx, int dy) { return WP(dx, dy, 0); };
+      auto A = [&](int dz) { return C(C_RST8W, k + dz) * C(C_IJCB8W, k + dz) * WP(0, 0, dz); };
+      f = smooth_sum(f, a.smtopt, a.smhcoe * (C(C_RST8W, k) * C(C_IJCB8W, k)), a.smvcoe, k, 2, nk - 1, H, A, edge);
     }
     if (a.vspopt >= 1 && a.vsp_w && k >= a.ksp0) f = f - C(C_RBCT, k) * C(C_RST8W, k) * WP(0, 0, 0);
     // buoywb.f90:166-172 (dry), 202-299 (moist), 307-313: the term of
@@ -306,72 +299,67 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
     const F2 wbk = k <= nk - 2 ? buoyancy(a, ck, id) : f2(0.f);
     if (k >= 3 && k <= nk - 2) f = f + (wb_prev + wbk);
     wb_prev = wbk;
-    // advuvw.f90:685-852
-    auto t1 = [&](int x) { return (RXU(x, 0, -1) + RXU(x, 0, 0)) * (Wc(x, 0, 0) - Wc(x - 1, 0, 0)) * dxv25n; };
-    auto t2 = [&](int y) { return (RXV(0, y, -1) + RXV(0, y, 0)) * (Wc(0, y, 0) - Wc(0, y - 1, 0)) * dyv25n; };
-    auto t3 = [&](int z) { return (RXW(0, 0, z) + RXW(0, 0, z + 1)) * (Wc(0, 0, z + 1) - Wc(0, 0, z)) * dzv25n; };
-    F2 hadv = (t1(0) + t1(1)) + (t2(0) + t2(1));
-    auto t1w = [&](int x) {
-      return ((RXU(x, 0, -1) + RXU(x, 0, 0)) + (RXU(x + 1, 0, -1) + RXU(x + 1, 0, 0))) *
-             (Wc(x + 1, 0, 0) - Wc(x - 1, 0, 0)) * dxv48;
-    };
-    auto t2w = [&](int y) {
-      return ((RXV(0, y, -1) + RXV(0, y, 0)) + (RXV(0, y + 1, -1) + RXV(0, y + 1, 0))) *
-             (Wc(0, y + 1, 0) - Wc(0, y - 1, 0)) * dyv48;
-    };
-    const F2 h2 = hadv;
-    hadv = fourd3 * hadv + ((t1w(-1) + t1w(1)) + (t2w(-1) + t2w(1)));
-    if (edge) hadv = sel2(edge, h2, hadv);
-    F2 vadv = t3(-1) + t3(0);
+    // advuvw.f90:685-884
+    const F2 c = Wc(0, 0, 0);
+    const float rum = C(C_RST8U, k - 1), rvm = C(C_RST8V, k - 1);
+    auto Us = [&](int x) { return fma2(f2(rum), Uc(x, 0, -1), ru * Uc(x, 0, 0)); };
+    auto Vs = [&](int y) { return fma2(f2(rvm), Vc(0, y, -1), rv * Vc(0, y, 0)); };
+    const F2 u0 = Us(0), u1 = Us(1), v0 = Vs(0), v1 = Vs(1);
+    f = hsum(f, u0 * (c - Wc(-1, 0, 0)) + u1 * (Wc(1, 0, 0) - c), v0 * (c - Wc(0, -1, 0)) + v1 * (Wc(0, 1, 0) - c),
+             (Us(-1) + u0) * (c - Wc(-2, 0, 0)) + (u1 + Us(2)) * (Wc(2, 0, 0) - c),
+             (Vs(-1) + v0) * (c - Wc(0, -2, 0)) + (v1 + Vs(2)) * (Wc(0, 2, 0) - c), dxv25n, dyv25n, dxv48, dyv48);
+    const F2 wd = Wc(0, 0, -1), wu = Wc(0, 0, 1), fc = rw(0) * c;
+    const F2 z2 = (rw(-1) * wd + fc) * (c - wd) + (fc + rw(1) * wu) * (wu - c);
     if (adv3) {   // advuvw.f90:854-884
-      auto t3w = [&](int z) {
-        return (RXW(0, 0, z - 1) + RXW(0, 0, z + 1)) * (Wc(0, 0, z + 1) - Wc(0, 0, z - 1)) * dzv24;
-      };
-      vadv = fourd3 * vadv + (t3w(-1) + t3w(1));
+      const F2 wd2 = Wc(0, 0, -2), wu2 = Wc(0, 0, 2);
+      f = fma2(f2(fourd3 * dzv25n), z2, f);
+      f = fma2(f2(dzv24), (rw(-2) * wd2 + fc) * (c - wd2) + (fc + rw(2) * wu2) * (wu2 - c), f);
+    } else {
+      f = fma2(f2(dzv25n), z2, f);
     }
-    f = f + hadv + vadv;
     put(a.wfrc, id, f);
   } else {
     // --------------------------------------------- pfrc, theta' step
     // advs-type advection of s with fluxes FU/FV/FW (advs.f90:205-370)
     auto Sc = [&](int dx, int dy, int dz) { return X(0, dx, dy, dz); };
     auto SP = [&](int dx, int dy, int dz) { return X(4, dx, dy, dz); };
-    auto adv = [&](auto FU, auto FV, auto FW) {
-      auto t1 = [&](int x) { return FU(x) * (Sc(x, 0, 0) - Sc(x - 1, 0, 0)) * dxv05n; };
-      auto t2 = [&](int y) { return FV(y) * (Sc(0, y, 0) - Sc(0, y - 1, 0)) * dyv05n; };
-      auto t3 = [&](int z) { return FW(z) * (Sc(0, 0, z) - Sc(0, 0, z - 1)) * dzv05n; };
-      F2 sf = (t1(0) + t1(1)) + (t2(0) + t2(1));
-      auto t1w = [&](int x) { return (FU(x) + FU(x + 1)) * (Sc(x + 1, 0, 0) - Sc(x - 1, 0, 0)) * dxv24; };
-      auto t2w = [&](int y) { return (FV(y) + FV(y + 1)) * (Sc(0, y + 1, 0) - Sc(0, y - 1, 0)) * dyv24; };
-      const F2 s2 = sf;
-      sf = fourd3 * sf + ((t1w(-1) + t1w(1)) + (t2w(-1) + t2w(1)));
-      if (edge) sf = sel2(edge, s2, sf);
-      F2 vadv = t3(0) + t3(1);
+    // cu, cv, cw(z): the winds' weights
+    auto adv = [&](float cu, float cv, auto cw) {
+      const F2 c = Sc(0, 0, 0), u0 = Uc(0, 0, 0), u1 = Uc(1, 0, 0), v0 = Vc(0, 0, 0), v1 = Vc(0, 1, 0);
+      F2 f = hsum(f2(0.f), u0 * (c - Sc(-1, 0, 0)) + u1 * (Sc(1, 0, 0) - c),
+                  v0 * (c - Sc(0, -1, 0)) + v1 * (Sc(0, 1, 0) - c),
+                  (Uc(-1, 0, 0) + u0) * (c - Sc(-2, 0, 0)) + (u1 + Uc(2, 0, 0)) * (Sc(2, 0, 0) - c),
+                  (Vc(0, -1, 0) + v0) * (c - Sc(0, -2, 0)) + (v1 + Vc(0, 2, 0)) * (Sc(0, 2, 0) - c),
+                  -.5f * dxiv * cu, -.5f * dyiv * cv, dxv24 * cu, dyv24 * cv);
+      const F2 w0 = cw(0) * Wc(0, 0, 0), w1 = cw(1) * Wc(0, 0, 1);
+      const F2 z2 = w0 * (c - Sc(0, 0, -1)) + w1 * (Sc(0, 0, 1) - c);
       if (adv3) {   // advs.f90:372-416, advp.f90:627-655
-        auto t3w = [&](int z) { return (FW(z) + FW(z + 1)) * (Sc(0, 0, z + 1) - Sc(0, 0, z - 1)) * dzv24; };
-        vadv = fourd3 * vadv + (t3w(-1) + t3w(1));
+        f = fma2(f2(fourd3 * dzv05n), z2, f);
+        return fma2(f2(dzv24), (cw(-1) * Wc(0, 0, -1) + w0) * (c - Sc(0, 0, -2)) +
+                                   (w1 + cw(2) * Wc(0, 0, 2)) * (Sc(0, 0, 2) - c), f);
       }
-      return sf + vadv;
+      return fma2(f2(dzv05n), z2, f);
     };
     if constexpr (G == 3) {
       // pressure (advp.f90:255-291 J-weighted fluxes)
-      auto FU = [&](int x) { return C(C_JCB8U, k) * Uc(x, 0, 0); };
-      auto FV = [&](int y) { return C(C_JCB8V, k) * Vc(0, y, 0); };
-      auto FW = [&](int z) { return C(C_JCB8W, k + z) * WC(0, 0, z); };
-      F2 f = adv(FU, FV, FW);
-      if (smooth) f = smooth_tile(f, a.smtopt, a.smhcoe, a.smvcoe, k, 2, nk - 2, SP, edge);
+      F2 f = adv(C(C_JCB8U, k), C(C_JCB8V, k), [&](int z) {
+        return a.sthopt ? C(C_JCB8W, k + z) * C(C_IJCB8W, k + z) : C(C_JCB8W, k + z);
+      });
+      if (smooth) {
+        auto H = [&](int dx, int dy) { return SP(dx, dy, 0); };
+        auto A = [&](int dz) { return SP(0, 0, dz); };
+        f = smooth_sum(f, a.smtopt, a.smhcoe, a.smvcoe, k, 2, nk - 2, H, A, edge);
+      }
       if (a.vspopt >= 1 && a.vsp_p && k >= a.ksp0 - 1)
         f = f - .5f * (C(C_RBCT, k) + C(C_RBCT, k + 1)) * C(C_JCB, k) * SP(0, 0, 0);
       put(a.pfrc, id, f);
     } else {
       // theta'
-      auto FU = [&](int x) { return RXU(x, 0, 0); };
-      auto FV = [&](int y) { return RXV(0, y, 0); };
-      auto FW = [&](int z) { return RXW(0, 0, z); };
-      F2 f = adv(FU, FV, FW);
+      F2 f = adv(ru, rv, rw);
       if (smooth) {
-        auto A = [&](int dx, int dy, int dz) { return C(C_RBR, k + dz) * SP(dx, dy, dz); };
-        f = smooth_tile(f, a.smtopt, a.smhcoe, a.smvcoe, k, 2, nk - 2, A, edge);
+        auto H = [&](int dx, int dy) { return SP(dx, dy, 0); };
+        auto A = [&](int dz) { return C(C_RBR, k + dz) * SP(0, 0, dz); };
+        f = smooth_sum(f, a.smtopt, a.smhcoe * C(C_RBR, k), a.smvcoe, k, 2, nk - 2, H, A, edge);
       }
       if constexpr (T) {   // forcept.f90:313-320, 383-393: mixing of the full theta at t-dt
         auto RK = [&](int dx, int dy, int dz) { return X(5, dx, dy, dz); };
@@ -396,7 +384,7 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
 }
 
 template <int SG, bool T>
-__global__ void __launch_bounds__(kFPairs * kForceTY * (SG == 0 ? 3 : 2))
+__global__ void __launch_bounds__(kFPairs * kForceTY * (SG == 0 ? 3 : 2), T ? 2 : 3)
 k_force(const __grid_constant__ ForceMaps m, const ForceArgs a) {
   using L = FLayout<SG, T>;
   constexpr int S = L::S, BX = kHeviBoxX, TY = kForceTY;

@@ -203,8 +203,8 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
       else if constexpr (DIV == 1) th = pp + a.divcv * jcbk * div;
       else th = pp;
       tc = jcbk * th;
-      t3h[oyA * BX + ox] = tc.v.x;
-      t3h[oyB * BX + ox] = tc.v.y;
+      t3h[oyA * BX + ox] = tc.x();
+      t3h[oyB * BX + ox] = tc.y();
       if (has_halo) {
         const float dh = div3d_at(hx, hy), ph = P[hy * BX + hx];
         float thh;
@@ -227,13 +227,13 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
     if (uvlev) {
       const float irst8u = CK(k, C_IRST8U), irst8v = CK(k, C_IRST8V);
       const F2 un0 = col2(U, oyA) + dts * (col2(UF, fyA) + (col2(t3h - 1, oyA) - tc) * dxiv) * irst8u;
-      F2 un1 = f2(__shfl_down_sync(full, un0.v.x, 1), __shfl_down_sync(full, un0.v.y, 1));
+      F2 un1 = f2(__shfl_down_sync(full, un0.x(), 1), __shfl_down_sync(full, un0.y(), 1));
       if (tx == TX - 1)
         un1 = col2(U + 1, oyA) + dts * (col2(UF + 1, fyA) + (tc - col2(t3h + 1, oyA)) * dxiv) * irst8u;
-      const F2 vs = col2(V, oyA) + dts * (col2(VF, fyA) + (f2(t3h[(oyA - 1) * BX + ox], tc.v.x) - tc) * dyiv) * irst8v;
+      const F2 vs = col2(V, oyA) + dts * (col2(VF, fyA) + (f2(t3h[(oyA - 1) * BX + ox], tc.x()) - tc) * dyiv) * irst8v;
       const float vf2 = V[(oyB + 1) * BX + ox] +
-                        dts * (VF[(fyB + 1) * BX + ox] + (tc.v.y - t3h[(oyB + 1) * BX + ox]) * dyiv) * irst8v;
-      const F2 vn = f2(vs.v.y, vf2);
+                        dts * (VF[(fyB + 1) * BX + ox] + (tc.y() - t3h[(oyB + 1) * BX + ox]) * dyiv) * irst8v;
+      const F2 vn = f2(vs.y(), vf2);
       const bool kend = (k == 2) || (k == nk - 2);
       auto store_uv = [&](bool edge, bool ylast, int j, int id, float u0, float u1, float v0, float v1) {
         if (edge) {
@@ -253,8 +253,8 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
           if (ylast) store_periodic(a.v_new, g, STAG_V, i, j + 1, kc, v1);
         }
       };
-      if (stA) store_uv(edgeA, ylastA, jA, idA, un0.v.x, un1.v.x, vs.v.x, vn.v.x);
-      if (stB) store_uv(edgeB, ylastB, jB, idB, un0.v.y, un1.v.y, vs.v.y, vn.v.y);
+      if (stA) store_uv(edgeA, ylastA, jA, idA, un0.x(), un1.x(), vs.x(), vn.x());
+      if (stB) store_uv(edgeB, ylastB, jB, idB, un0.y(), un1.y(), vs.y(), vn.y());
       // horizontal part of diverpe's divergence (jcb-weighted new winds)
       const float jcb8u = CK(k, C_JCB8U), jcb8v = CK(k, C_JCB8V);
       hdiv = (jcb8u * un0 - jcb8u * un1) * dxiv + (jcb8v * vs - jcb8v * vn) * dyiv;
@@ -271,21 +271,21 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
       wcn = STH ? wn * CK(k, C_IJCB8W) : wn;                                        // phy2cnt.f90:219
       if (k == 2 || k == nk - 1) {
         // vbcw.f90:317,481: w = 0 here; the contravariant value stays
-        if (stA) put_side(k, jA, wcn.v.x);
-        if (stB) put_side(k, jB, wcn.v.y);
+        if (stA) put_side(k, jA, wcn.x());
+        if (stB) put_side(k, jB, wcn.y());
         wadv = f2(0.f);
         if (stA) store_periodic(a.w_new, g, STAG_S, i, jA, k, 0.f);
         if (stB) store_periodic(a.w_new, g, STAG_S, i, jB, k, 0.f);
       } else {
         wadv = wn;
-        if (stA) { if (edgeA) store_periodic(a.w_new, g, STAG_S, i, jA, k, wn.v.x); else a.w_new[idA] = wn.v.x; }
-        if (stB) { if (edgeB) store_periodic(a.w_new, g, STAG_S, i, jB, k, wn.v.y); else a.w_new[idB] = wn.v.y; }
+        if (stA) { if (edgeA) store_periodic(a.w_new, g, STAG_S, i, jA, k, wn.x()); else a.w_new[idA] = wn.x(); }
+        if (stB) { if (edgeB) store_periodic(a.w_new, g, STAG_S, i, jB, k, wn.y()); else a.w_new[idB] = wn.y(); }
         // vbcw.f90:285,471 images from the contravariant w of levels 3 and nk-2
         if (k == 3 || k == nk - 2) {
           const int kc = k == 3 ? 1 : nk;
           const float j8w = CK(k, C_JCB8W);
-          if (stA) store_periodic(a.w_new, g, STAG_S, i, jA, kc, -j8w * wcn.v.x - 0.f);
-          if (stB) store_periodic(a.w_new, g, STAG_S, i, jB, kc, -j8w * wcn.v.y - 0.f);
+          if (stA) store_periodic(a.w_new, g, STAG_S, i, jA, kc, -j8w * wcn.x() - 0.f);
+          if (stB) store_periodic(a.w_new, g, STAG_S, i, jB, kc, -j8w * wcn.y() - 0.f);
         }
       }
     }
@@ -298,17 +298,17 @@ k_heve(const __grid_constant__ HeviMaps m, const HeviArgs a) {
       const F2 psml = g05 * (wadv_prev + wadv) * CK(kp, C_RST) + pdiv;                             // advbspe.f90:127
       const F2 pn = pp_prev + dts * (pf_prev + psml) * CK(kp, C_IJCB);                             // steppe.f90:224
       const int ipA = idA - plane, ipB = idB - plane;
-      if (stA) { if (edgeA) store_periodic(a.p_new, g, STAG_S, i, jA, kp, pn.v.x); else a.p_new[ipA] = pn.v.x; }
-      if (stB) { if (edgeB) store_periodic(a.p_new, g, STAG_S, i, jB, kp, pn.v.y); else a.p_new[ipB] = pn.v.y; }
+      if (stA) { if (edgeA) store_periodic(a.p_new, g, STAG_S, i, jA, kp, pn.x()); else a.p_new[ipA] = pn.x(); }
+      if (stB) { if (edgeB) store_periodic(a.p_new, g, STAG_S, i, jB, kp, pn.y()); else a.p_new[ipB] = pn.y(); }
       // vbcp.f90:126-160 (levels 2 and 3 belong to the first block)
-      if (kp == 2) { p2A = pn.v.x; p2B = pn.v.y; }
+      if (kp == 2) { p2A = pn.x(); p2B = pn.y(); }
       if (kp == 3) {
-        if (stA) store_periodic(a.p_new, g, STAG_S, i, jA, 1, (a.bbc == 2) ? 2.f * p2A - pn.v.x : p2A);
-        if (stB) store_periodic(a.p_new, g, STAG_S, i, jB, 1, (a.bbc == 2) ? 2.f * p2B - pn.v.y : p2B);
+        if (stA) store_periodic(a.p_new, g, STAG_S, i, jA, 1, (a.bbc == 2) ? 2.f * p2A - pn.x() : p2A);
+        if (stB) store_periodic(a.p_new, g, STAG_S, i, jB, 1, (a.bbc == 2) ? 2.f * p2B - pn.y() : p2B);
       }
       if (kp == nk - 2) {
-        if (stA) store_periodic(a.p_new, g, STAG_S, i, jA, nk - 1, pn.v.x);
-        if (stB) store_periodic(a.p_new, g, STAG_S, i, jB, nk - 1, pn.v.y);
+        if (stA) store_periodic(a.p_new, g, STAG_S, i, jA, nk - 1, pn.x());
+        if (stB) store_periodic(a.p_new, g, STAG_S, i, jB, nk - 1, pn.y());
       }
     }
     t3v_prev = t3v;

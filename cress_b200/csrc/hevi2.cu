@@ -225,8 +225,8 @@ __device__ __forceinline__ void hevi2_tile(const HeviMaps& m, const HeviArgs& a,
     else if constexpr (DIV == 1) th = pp + a.divcv * jcbk * div;
     else th = pp;
     const F2 tc = jcbk * th;
-    t3h[oyA * BX + ox] = tc.v.x;
-    t3h[oyB * BX + ox] = tc.v.y;
+    t3h[oyA * BX + ox] = tc.x();
+    t3h[oyB * BX + ox] = tc.y();
     const F2 t3v = (DIV >= 1) ? pp + a.divcv * jcbk * div : pp;                    // pgrad.f90:300
     if (has_halo) t3h[hy * BX + hx] = t3h_of(div3d_at(hx, hy), P[hy * BX + hx]);
     __syncthreads();
@@ -239,15 +239,15 @@ __device__ __forceinline__ void hevi2_tile(const HeviMaps& m, const HeviArgs& a,
     // stepuv.f90:294,304 with pgrad.f90:379,389: west u faces, the east
     // face from the next lane (lane 31 forms its own)
     const F2 un0 = col2(U, oyA) + dts * (col2(UF, fyA) + (col2(t3h - 1, oyA) - tc) * dxiv) * irst8u;
-    F2 un1 = f2(__shfl_down_sync(full, un0.v.x, 1), __shfl_down_sync(full, un0.v.y, 1));
+    F2 un1 = f2(__shfl_down_sync(full, un0.x(), 1), __shfl_down_sync(full, un0.y(), 1));
     if (tx == TX - 1)
       un1 = col2(U + 1, oyA) + dts * (col2(UF + 1, fyA) + (tc - col2(t3h + 1, oyA)) * dxiv) * irst8u;
     // v faces south of rows A and B (the one between the rows serves both),
     // and north of row B
-    const F2 vs = col2(V, oyA) + dts * (col2(VF, fyA) + (f2(t3h[(oyA - 1) * BX + ox], tc.v.x) - tc) * dyiv) * irst8v;
+    const F2 vs = col2(V, oyA) + dts * (col2(VF, fyA) + (f2(t3h[(oyA - 1) * BX + ox], tc.x()) - tc) * dyiv) * irst8v;
     const float vf2 = V[(oyB + 1) * BX + ox] +
-                      dts * (VF[(fyB + 1) * BX + ox] + (tc.v.y - t3h[(oyB + 1) * BX + ox]) * dyiv) * irst8v;
-    const F2 vn = f2(vs.v.y, vf2);
+                      dts * (VF[(fyB + 1) * BX + ox] + (tc.y() - t3h[(oyB + 1) * BX + ox]) * dyiv) * irst8v;
+    const F2 vn = f2(vs.y(), vf2);
 
     const float jcb8u = CK(k, C_JCB8U), jcb8v = CK(k, C_JCB8V);
     const float rcsq = CK(k, C_RCSQ), rst = CK(k, C_RST), rbr = CK(k, C_RBR), ircsq = CK(k, C_IRCSQ);
@@ -272,16 +272,16 @@ __device__ __forceinline__ void hevi2_tile(const HeviMaps& m, const HeviArgs& a,
         if (ylast) store_periodic(a.v_new, g, STAG_V, i, j + 1, kc, v1);
       }
     };
-    if (ownA) store_uv(edgeA, ylastA, jA, idA, un0.v.x, un1.v.x, vs.v.x, vn.v.x);
-    if (ownB) store_uv(edgeB, ylastB, jB, idB, un0.v.y, un1.v.y, vs.v.y, vn.v.y);
+    if (ownA) store_uv(edgeA, ylastA, jA, idA, un0.x(), un1.x(), vs.x(), vn.x());
+    if (ownB) store_uv(edgeB, ylastB, jB, idB, un0.y(), un1.y(), vs.y(), vn.y());
 
     F2 phd = (jcb8u * un0 - jcb8u * un1) * dxiv + (jcb8v * vs - jcb8v * vn) * dyiv;    // diver2d.f90:288
     phd = rcsq * phd;                                                                   // diverpih.f90:208
     const F2 wk = col2(W0, oyA), wk1 = col2(W1, oyA);
     const F2 pvd = rcsq * (wk - wk1) * dziv;                                            // diverpiv.f90:124
     const F2 fp = col2(PF, fyA) + phd + weic1m * (a.g05 * (wk + wk1) * rst + pvd);      // advbspi.f90:158
-    if (ownA) a.p_new[idA] = fp.v.x;   // parked until the way down
-    if (ownB) a.p_new[idB] = fp.v.y;
+    if (ownA) a.p_new[idA] = fp.x();   // parked until the way down
+    if (ownB) a.p_new[idB] = fp.y();
     const F2 fpdvj = fp * ijcbk;                                                        // pgradiv.f90:149
     const F2 wb8s = (pp * rst + fp * rbr * a.dtw) * ircsq * a.g05n;                     // buoywsi.f90:171
     if (k >= 3) {
@@ -291,8 +291,8 @@ __device__ __forceinline__ void hevi2_tile(const HeviMaps& m, const HeviArgs& a,
       const F2 wrhs = wk + dts * fw * irst8w;                                           // stepwi.f90:325
       // gaussel.f90:189-240 in double with the 1-D factors, one recurrence per row
       const double rr = (double)TH_RR(k), aa = TH_AA(k);
-      const double fA = (k == 3) ? (double)wrhs.v.x * aa : ((double)wrhs.v.x - rr * fA_prev) * aa;
-      const double fB = (k == 3) ? (double)wrhs.v.y * aa : ((double)wrhs.v.y - rr * fB_prev) * aa;
+      const double fA = (k == 3) ? (double)wrhs.x() * aa : ((double)wrhs.x() - rr * fA_prev) * aa;
+      const double fB = (k == 3) ? (double)wrhs.y() * aa : ((double)wrhs.y() - rr * fB_prev) * aa;
       if (ownA) a.w_new[idA] = (float)fA;   // parked until the way down
       if (ownB) a.w_new[idB] = (float)fB;
       fA_prev = fA;

@@ -178,8 +178,8 @@ __device__ __forceinline__ void hevi3_tile(const HeviMaps& m, const HeviArgs& a,
     r.aa = __ldg(reinterpret_cast<const double*>(p + 8));
     r.n1 = __ldg(p + 9 + 1);
   };
-  auto lo2 = [](float4 v) { return F2{make_float2(v.x, v.y)}; };   // first pair of a vector
-  auto hi2 = [](float4 v) { return F2{make_float2(v.z, v.w)}; };   // second pair
+  auto lo2 = [](float4 v) { return f2(v.x, v.y); };   // first pair of a vector
+  auto hi2 = [](float4 v) { return f2(v.z, v.w); };   // second pair
   Row cur, nxt;
   load_row(2, cur);
   float4 v1k = __ldg(rows + 9 * 2 + 1);   // row k's vector 1
@@ -208,18 +208,18 @@ __device__ __forceinline__ void hevi3_tile(const HeviMaps& m, const HeviArgs& a,
     const float* P = st0 + L::oP;
     auto div3d_at = [&](int x, int y) {
       float wck = W0[y * BX + x], wck1 = W1s[y * BX + x];
-      if constexpr (STH) { wck = wck * ij8wk.v.x; wck1 = wck1 * ij8wk1.v.x; }
-      return (rst8wk.v.x * wck - rst8wk1.v.x * wck1) * dziv.v.x +
-             ((rst8u.v.x * U[y * BX + x] - rst8u.v.x * U[y * BX + x + 1]) * dxiv.v.x +
-              (rst8v.v.x * V[y * BX + x] - rst8v.v.x * V[(y + 1) * BX + x]) * dyiv.v.x);
+      if constexpr (STH) { wck = wck * ij8wk.x(); wck1 = wck1 * ij8wk1.x(); }
+      return (rst8wk.x() * wck - rst8wk1.x() * wck1) * dziv.x() +
+             ((rst8u.x() * U[y * BX + x] - rst8u.x() * U[y * BX + x + 1]) * dxiv.x() +
+              (rst8v.x() * V[y * BX + x] - rst8v.x() * V[(y + 1) * BX + x]) * dyiv.x());
     };
     // pgrad.f90:300,341,363
     auto t3h_of = [&](float div, float pp) {
       float th;
-      if constexpr (DIV == 2) th = pp + divch * div * ijcbk.v.x;
-      else if constexpr (DIV == 1) th = pp + divcv * jcbk.v.x * div;
+      if constexpr (DIV == 2) th = pp + divch * div * ijcbk.x();
+      else if constexpr (DIV == 1) th = pp + divcv * jcbk.x() * div;
       else th = pp;
-      return jcbk.v.x * th;
+      return jcbk.x() * th;
     };
     // rows A and B of the thread in the two lanes of F2: one packed
     // instruction for both rows (offsets relative to the own cell)
@@ -236,8 +236,8 @@ __device__ __forceinline__ void hevi3_tile(const HeviMaps& m, const HeviArgs& a,
     else if constexpr (DIV == 1) th = pp + divcv2 * jcbk * div;
     else th = pp;
     const F2 tc = jcbk * th;
-    th0[0] = tc.v.x;
-    th0[BX] = tc.v.y;
+    th0[0] = tc.x();
+    th0[BX] = tc.y();
     const F2 t3v = (DIV >= 1) ? pp + divcv2 * jcbk * div : pp;               // pgrad.f90:300
     if (has_halo) t3h[hy * BX + hx] = t3h_of(div3d_at(hx, hy), P[hy * BX + hx]);
     // the rest of this level's own inputs, read before the barrier
@@ -254,25 +254,25 @@ __device__ __forceinline__ void hevi3_tile(const HeviMaps& m, const HeviArgs& a,
     // stepuv.f90:294,304 with pgrad.f90:379,389: west u faces, the east
     // face from the next lane (lane 31 forms its own)
     const F2 un0 = uo + dts * (uf + (at2(th0, -1) - tc) * dxiv) * irst8u;
-    F2 un1 = f2(__shfl_down_sync(full, un0.v.x, 1), __shfl_down_sync(full, un0.v.y, 1));
+    F2 un1 = f2(__shfl_down_sync(full, un0.x(), 1), __shfl_down_sync(full, un0.y(), 1));
     if (tx == TX - 1)
       un1 = at2(tb, L::oU + 1) + dts * (at2(tb, L::oUF - BX + 1) + (tc - at2(th0, 1)) * dxiv) * irst8u;
     // v faces south of rows A and B (the one between the rows serves both),
     // and north of row B
-    const F2 vs = vo + dts * (vf + (f2(th0[-BX], tc.v.x) - tc) * dyiv) * irst8v;
-    const float vn2 = vo2 + a.dts * (vf2f + (tc.v.y - th0[2 * BX]) * a.dyiv) * irst8v.v.x;
-    const F2 vn = f2(vs.v.y, vn2);
+    const F2 vs = vo + dts * (vf + (f2(th0[-BX], tc.x()) - tc) * dyiv) * irst8v;
+    const float vn2 = vo2 + a.dts * (vf2f + (tc.y() - th0[2 * BX]) * a.dyiv) * irst8v.x();
+    const F2 vn = f2(vs.y(), vn2);
 
     const F2 jcb8u = lo2(cur.v4), jcb8v = hi2(cur.v4), rcsq = lo2(cur.v5), rst = hi2(cur.v5);
     const F2 rbr = lo2(cur.v6), ircsq = hi2(cur.v6), irst8w = lo2(cur.v7);
     const bool kend = (k == 2) || (k == nk - 2);
     if constexpr (!EDGE) {
-      uA[0] = un0.v.x; uA[px] = un0.v.y;
-      vA[0] = vs.v.x; vA[px] = vs.v.y;
+      uA[0] = un0.x(); uA[px] = un0.y();
+      vA[0] = vs.x(); vA[px] = vs.y();
       if (kend) {   // vbcu.f90:120,134 (and vbcv): levels 1 and nk-1 copy levels 2 and nk-2
         const int dk = (k == 2 ? -1 : 1) * plane;
-        uA[dk] = un0.v.x; uA[dk + px] = un0.v.y;
-        vA[dk] = vs.v.x; vA[dk + px] = vs.v.y;
+        uA[dk] = un0.x(); uA[dk + px] = un0.y();
+        vA[dk] = vs.x(); vA[dk + px] = vs.y();
       }
     } else {
       auto store_uv = [&](bool edge, bool ylast, int j, float u0, float u1, float v0, float v1) {
@@ -293,8 +293,8 @@ __device__ __forceinline__ void hevi3_tile(const HeviMaps& m, const HeviArgs& a,
           if (ylast) store_periodic(a.v_new, g, STAG_V, i, j + 1, kc, v1);
         }
       };
-      if (ownA) store_uv(edgeA, ylastA, jA, un0.v.x, un1.v.x, vs.v.x, vn.v.x);
-      if (ownB) store_uv(edgeB, ylastB, jB, un0.v.y, un1.v.y, vs.v.y, vn.v.y);
+      if (ownA) store_uv(edgeA, ylastA, jA, un0.x(), un1.x(), vs.x(), vn.x());
+      if (ownB) store_uv(edgeB, ylastB, jB, un0.y(), un1.y(), vs.y(), vn.y());
     }
 
     F2 phd = (jcb8u * un0 - jcb8u * un1) * dxiv + (jcb8v * vs - jcb8v * vn) * dyiv;    // diver2d.f90:288
@@ -302,7 +302,7 @@ __device__ __forceinline__ void hevi3_tile(const HeviMaps& m, const HeviArgs& a,
     const F2 pvd = rcsq * (wk - wk1) * dziv;                                            // diverpiv.f90:124
     const F2 fp = pf + phd + weic1m * (g05 * (wk + wk1) * rst + pvd);                   // advbspi.f90:158
     const F2 q = pp + dts * fp * ijcbk;           // steppi.f90:217, explicit part of the new p'
-    qs[(k - 2) * NT + tid] = q.v;
+    qs[(k - 2) * NT + tid] = make_float2(q.x(), q.y());
     const F2 fpdvj = fp * ijcbk;                                                        // pgradiv.f90:149
     const F2 wb8s = (pp * rst + fp * rbr * dtw) * ircsq * g05n;                         // buoywsi.f90:171
     if (k >= 3) {
@@ -312,8 +312,8 @@ __device__ __forceinline__ void hevi3_tile(const HeviMaps& m, const HeviArgs& a,
       const F2 wrhs = wk + dts * fw * irst8w;                                           // stepwi.f90:325
       // gaussel.f90:189-240 in double with the 1-D factors, one recurrence per row
       const double rr = (double)cur.v7.z, aa = cur.aa;
-      const double fA = (k == 3) ? (double)wrhs.v.x * aa : ((double)wrhs.v.x - rr * fA_prev) * aa;
-      const double fB = (k == 3) ? (double)wrhs.v.y * aa : ((double)wrhs.v.y - rr * fB_prev) * aa;
+      const double fA = (k == 3) ? (double)wrhs.x() * aa : ((double)wrhs.x() - rr * fA_prev) * aa;
+      const double fB = (k == 3) ? (double)wrhs.y() * aa : ((double)wrhs.y() - rr * fB_prev) * aa;
       tmem_st4(tmem + 4u * (uint32_t)(k - 3), lo32(fA), hi32(fA), lo32(fB), hi32(fB));
       fA_prev = fA;
       fB_prev = fB;
@@ -366,32 +366,33 @@ __device__ __forceinline__ void hevi3_tile(const HeviMaps& m, const HeviArgs& a,
       wdA = mk64(r[4 * e], r[4 * e + 1]) - cpk * wdA;    // gaussel.f90:254
       wdB = mk64(r[4 * e + 2], r[4 * e + 3]) - cpk * wdB;
       const F2 wk = f2((float)wdA, (float)wdB);
-      const F2 q = F2{qs[(k - 2) * NT + tid]};
+      const float2 qv = qs[(k - 2) * NT + tid];
+      const F2 q = f2(qv.x, qv.y);
       // steppi.f90:217 with diverpiv.f90:124 and advbspi.f90:175 (the implicit part)
       const F2 pvd = lo2(d5) * (wk - wup) * dziv;
       const F2 fpw = weicoe * (g05 * (wk + wup) * hi2(d5) + pvd);
       const F2 pn = q + dts * fpw * hi2(d2);
       const int off = (k - ktop) * plane;
       if constexpr (!EDGE) {
-        wT[off] = wk.v.x; wT[off + px] = wk.v.y;
-        pT[off] = pn.v.x; pT[off + px] = pn.v.y;
+        wT[off] = wk.x(); wT[off + px] = wk.y();
+        pT[off] = pn.x(); pT[off + px] = pn.y();
       } else {
         if (ownA) {
           if (edgeA) {
-            store_periodic(a.w_new, g, STAG_S, i, jA, k, wk.v.x);
-            store_periodic(a.p_new, g, STAG_S, i, jA, k, pn.v.x);
+            store_periodic(a.w_new, g, STAG_S, i, jA, k, wk.x());
+            store_periodic(a.p_new, g, STAG_S, i, jA, k, pn.x());
           } else {
-            wT[off] = wk.v.x;
-            pT[off] = pn.v.x;
+            wT[off] = wk.x();
+            pT[off] = pn.x();
           }
         }
         if (ownB) {
           if (edgeB) {
-            store_periodic(a.w_new, g, STAG_S, i, jB, k, wk.v.y);
-            store_periodic(a.p_new, g, STAG_S, i, jB, k, pn.v.y);
+            store_periodic(a.w_new, g, STAG_S, i, jB, k, wk.y());
+            store_periodic(a.p_new, g, STAG_S, i, jB, k, pn.y());
           } else {
-            wT[off + px] = wk.v.y;
-            pT[off + px] = pn.v.y;
+            wT[off + px] = wk.y();
+            pT[off + px] = pn.y();
           }
         }
       }
@@ -405,7 +406,8 @@ __device__ __forceinline__ void hevi3_tile(const HeviMaps& m, const HeviArgs& a,
   // stretched) and vbcp.f90:126-160, and level nk of u, v, p' carried over
   {
     const float4 d2 = __ldg(rows + 9 * 2 + 2), d5 = __ldg(rows + 9 * 2 + 5);
-    const F2 q = F2{qs[tid]};
+    const float2 qv = qs[tid];
+    const F2 q = f2(qv.x, qv.y);
     const F2 w0 = f2(0.f);
     const F2 pvd = lo2(d5) * (w0 - wup) * dziv;
     const F2 fpw = weicoe * (g05 * (w0 + wup) * hi2(d5) + pvd);
@@ -430,8 +432,8 @@ __device__ __forceinline__ void hevi3_tile(const HeviMaps& m, const HeviArgs& a,
       if (xlast) store_periodic(a.u_new, g, STAG_U, i + 1, j, nk, a.u_old[g.at(i + 1, j, nk)]);
       if (ylast) store_periodic(a.v_new, g, STAG_V, i, j + 1, nk, a.v_old[g.at(i, j + 1, nk)]);
     };
-    finish(ownA, edgeA, ylastA, jA, p2.v.x, p3.v.x, wup.v.x, wkend.v.x, pkend.v.x);
-    finish(ownB, edgeB, ylastB, jB, p2.v.y, p3.v.y, wup.v.y, wkend.v.y, pkend.v.y);
+    finish(ownA, edgeA, ylastA, jA, p2.x(), p3.x(), wup.x(), wkend.x(), pkend.x());
+    finish(ownB, edgeB, ylastB, jB, p2.y(), p3.y(), wup.y(), wkend.y(), pkend.y());
   }
 }
 

@@ -48,6 +48,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include "common.cuh"
+#include "f2.cuh"
 #include "hevi_row.cuh"
 #include "status.h"
 #include "tma.cuh"
@@ -58,43 +59,10 @@ namespace {
 constexpr int kHrCols = 60;       // columns a tile owns (64 held)
 constexpr int kHrMaxWarps = 16;
 
-// The values of a column pair in one 64-bit register pair, so that packed
-// arithmetic, 64-bit loads and stores take it without moves.
-struct P2 {
-  uint64_t b;
-};
-__device__ __forceinline__ P2 p2(float x, float y) {
-  P2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.b) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ float px(P2 a) { return __uint_as_float((uint32_t)a.b); }
-__device__ __forceinline__ float py(P2 a) { return __uint_as_float((uint32_t)(a.b >> 32)); }
-__device__ __forceinline__ P2 operator+(P2 a, P2 b) {
-  P2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.b) : "l"(a.b), "l"(b.b));
-  return r;
-}
-__device__ __forceinline__ P2 operator-(P2 a, P2 b) {
-  P2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.b) : "l"(a.b), "l"(b.b));
-  return r;
-}
-__device__ __forceinline__ P2 operator*(P2 a, P2 b) {
-  P2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.b) : "l"(a.b), "l"(b.b));
-  return r;
-}
-__device__ __forceinline__ P2 fma2(P2 a, P2 b, P2 c) {
-  P2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.b) : "l"(a.b), "l"(b.b), "l"(c.b));
-  return r;
-}
-
 // (second column, first of the next lane): the pair one column to the east
-__device__ __forceinline__ P2 east(P2 a) { return p2(py(a), __shfl_down_sync(0xffffffffu, px(a), 1)); }
+__device__ __forceinline__ F2 east(F2 a) { return f2(a.y(), __shfl_down_sync(0xffffffffu, a.x(), 1)); }
 // (second of the previous lane, first column): the pair one column to the west
-__device__ __forceinline__ P2 west(P2 a) { return p2(__shfl_up_sync(0xffffffffu, py(a), 1), px(a)); }
+__device__ __forceinline__ F2 west(F2 a) { return f2(__shfl_up_sync(0xffffffffu, a.y(), 1), a.x()); }
 
 // The row of the old level that holds row r's values: itself, or with the
 // wrap (the y ghosts not written) its periodic image (SrcOrig/bcycle.f90).
@@ -119,9 +87,9 @@ __device__ __forceinline__ int edge_code(const Grid& g, bool ustag, int i, bool 
   if (n0 && i == 2) return ustag ? e | 2 | 4 * (4 * (g.ni - 2)) : e | 4 * (4 * (g.ni - 3));   // u: column 3 to ni
   return e;
 }
-__device__ __forceinline__ void put_edge(char* p, P2 x, int e) {
-  if (e & 1) *reinterpret_cast<float*>(p) = px(x);
-  if (e >> 2) *reinterpret_cast<float*>(p + (e >> 2)) = (e & 2) ? py(x) : px(x);
+__device__ __forceinline__ void put_edge(char* p, F2 x, int e) {
+  if (e & 1) *reinterpret_cast<float*>(p) = x.x();
+  if (e >> 2) *reinterpret_cast<float*>(p + (e >> 2)) = (e & 2) ? x.y() : x.x();
 }
 
 // Shared memory (bytes), at offsets known to the compiler; only the stages,
@@ -210,21 +178,21 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
   char* pv = reinterpret_cast<char*>(a.vn) + at0;
   char* pw = reinterpret_cast<char*>(a.wn) + at0 - px4;
   char* pp = reinterpret_cast<char*>(a.pn) + at0 - px4;
-  auto lo2 = [](ulonglong2 q) { return P2{q.x}; };
-  auto hi2 = [](ulonglong2 q) { return P2{q.y}; };
+  auto lo2 = [](ulonglong2 q) { return F2{q.x}; };
+  auto hi2 = [](ulonglong2 q) { return F2{q.y}; };
 
   const int es = EDGE ? edge_code(a.g, false, i, o0, o1) : 0, eu = EDGE ? edge_code(a.g, true, i, u0, u1) : 0;
   const bool edge = es | eu;
-  const P2 zero{0}, dxiv{a.dxiv2}, dyiv{a.dyiv2}, dziv{a.dziv2};
-  P2 tc[L], vc[L], vsp[L];                     // row r-1: damped pressure, new v; row r: v
-  P2 pk[L];                                    // row r-1: p'
-  P2 held[Y::park ? 1 : 2 * L];                // row r-1: explicit p' tendency but the v part, w right-hand side
-  P2 wf0 = zero, t30 = zero, t3l = zero;       // row r-1: what the chunk's first and last level hand on
+  const F2 zero{0}, dxiv{a.dxiv2}, dyiv{a.dyiv2}, dziv{a.dziv2};
+  F2 tc[L], vc[L], vsp[L];                     // row r-1: damped pressure, new v; row r: v
+  F2 pk[L];                                    // row r-1: p'
+  F2 held[Y::park ? 1 : 2 * L];                // row r-1: explicit p' tendency but the v part, w right-hand side
+  F2 wf0 = zero, t30 = zero, t3l = zero;       // row r-1: what the chunk's first and last level hand on
 #pragma unroll
   for (int l = 0; l < L; ++l) {
     const int k = min(k0 + l, nk), ic = min(i, g.px - 2);
     const size_t at = (size_t)(k - 1) * g.plane + (size_t)wrap_row(a, true, j0 - 1) * g.px + ic;
-    vc[l] = P2{__ldg(reinterpret_cast<const unsigned long long*>(a.v + at))};
+    vc[l] = F2{__ldg(reinterpret_cast<const unsigned long long*>(a.v + at))};
     tc[l] = vsp[l] = pk[l] = zero;
     if constexpr (!Y::park) held[2 * l] = held[2 * l + 1] = zero;
     else {
@@ -249,20 +217,20 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     const unsigned char* dt = smem + Y::oD + c * (32 * L);
     auto T = [&](int l, int n) { return *reinterpret_cast<const ulonglong2*>(ct + 16 * (kHrVec * l + n)); };
     auto D = [&](int l, int n) { return *reinterpret_cast<const double2*>(dt + 16 * (2 * l + n)); };
-    auto S = [&](int o, int l) { return P2{*reinterpret_cast<const uint64_t*>(sp + o + Y::row * l)}; };
+    auto S = [&](int o, int l) { return F2{*reinterpret_cast<const uint64_t*>(sp + o + Y::row * l)}; };
     auto get = [&](int n) {
       if constexpr (Y::park) return S(Y::stage, n);
       else return held[n];
     };
-    auto set = [&](int n, P2 x) {
+    auto set = [&](int n, F2 x) {
       if constexpr (Y::park) *reinterpret_cast<uint64_t*>(const_cast<unsigned char*>(sp) + Y::stage + Y::row * n) = x.b;
       else held[n] = x;
     };
     // level l's pair into a new field, and what an edge lane adds
-    auto emit = [&](char* p, int l, P2 x, bool on) {
+    auto emit = [&](char* p, int l, F2 x, bool on) {
       if (on) *reinterpret_cast<uint64_t*>(p + (uint64_t)pl4 * l) = x.b;
     };
-    auto extra = [&](char* p, int l, P2 x, int e) {
+    auto extra = [&](char* p, int l, F2 x, int e) {
       if (e) put_edge(p + (uint64_t)pl4 * l, x, e);
     };
     if (!fail) {   // a warp whose wait gave up stages nothing more and goes on with the barriers
@@ -275,57 +243,57 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     // arithmetic; only the results that belong to the strip are stored.
     const bool su = r >= j0 && r <= j1, sv = r >= j0 && (r <= j1 || r == nj - 1);   // row nj-1: the last v face
     const bool fu = su && u1, fv = sv && o1;
-    P2 q[L];
+    F2 q[L];
     double fa[L], fb[L];
     {
-      P2 Gpp = zero, t3p = zero, w = S(Y::sW, 0), W0 = hi2(T(0, 3)) * w;
+      F2 Gpp = zero, t3p = zero, w = S(Y::sW, 0), W0 = hi2(T(0, 3)) * w;
 #pragma unroll
       for (int l = 0; l < L; ++l) {
         const ulonglong2 q0 = T(l, 0), q1 = T(l, 1), q2 = T(l, 2), q3 = T(l, 3);
-        const P2 u = S(Y::sU, l), vN = S(Y::sV, l), p = S(Y::sP, l), w1 = S(Y::sW, l + 1), wf = S(Y::sWF, l);
+        const F2 u = S(Y::sU, l), vN = S(Y::sV, l), p = S(Y::sP, l), w1 = S(Y::sW, l + 1), wf = S(Y::sWF, l);
         // diver3d.f90:318 with phy2cnt.f90:219
-        const P2 W1 = lo2(q1) * w1;
-        P2 div = fma2(lo2(q0), u - east(u), W0 - W1);
+        const F2 W1 = lo2(q1) * w1;
+        F2 div = fma2(lo2(q0), u - east(u), W0 - W1);
         div = fma2(hi2(q0), vc[l] - vN, div);
         // pgrad.f90:341,363 and :300
-        const P2 t = fma2(lo2(q2), div, hi2(q1) * p), t3 = fma2(hi2(q2), div, p);
+        const F2 t = fma2(lo2(q2), div, hi2(q1) * p), t3 = fma2(hi2(q2), div, p);
         // stepuv.f90:304 with pgrad.f90:389: the south v face
-        const P2 vs = fma2(lo2(q3), fma2(tc[l] - t, dyiv, S(Y::sVF, l)), vc[l]);
+        const F2 vs = fma2(lo2(q3), fma2(tc[l] - t, dyiv, S(Y::sVF, l)), vc[l]);
         vc[l] = vN;
         tc[l] = t;
         {   // row r-1
           const ulonglong2 q4 = T(l, 4), q5 = T(l, 5), q6 = T(l, 6);
-          const P2 fp = fma2(lo2(q4), vsp[l] - vs, get(2 * l));            // advbspi.f90:158 with diver2d.f90:288
+          const F2 fp = fma2(lo2(q4), vsp[l] - vs, get(2 * l));            // advbspi.f90:158 with diver2d.f90:288
           q[l] = fma2(hi2(q4), fp, pk[l]);                              // steppi.f90:217, explicit part
-          const P2 gd = lo2(q5) * fp;                                   // pgradiv.f90:149,163
-          const P2 wb = fma2(lo2(q6), fp, hi2(q5) * pk[l]);             // buoywsi.f90:171
-          const P2 Gp = gd + wb, Gm = gd - wb;
+          const F2 gd = lo2(q5) * fp;                                   // pgradiv.f90:149,163
+          const F2 wb = fma2(lo2(q6), fp, hi2(q5) * pk[l]);             // buoywsi.f90:171
+          const F2 Gp = gd + wb, Gm = gd - wb;
           const double2 ab = D(l, 0);
-          const P2 wp = get(2 * l + 1);
+          const F2 wp = get(2 * l + 1);
           if (l == 0) {   // the level below belongs to the chunk below: its part enters with the chunk's entry value
-            const double cw = (double)px(hi2(q6)), dz = (double)px(dziv);
-            fa[0] = __dmul_rn(ab.x, __fma_rn(cw, __fma_rn(-dz, (double)px(t30), (double)px(wf0)) - (double)px(Gm), (double)px(wp)));
-            fb[0] = __dmul_rn(ab.x, __fma_rn(cw, __fma_rn(-dz, (double)py(t30), (double)py(wf0)) - (double)py(Gm), (double)py(wp)));
+            const double cw = (double)(hi2(q6)).x(), dz = (double)dziv.x();
+            fa[0] = __dmul_rn(ab.x, __fma_rn(cw, __fma_rn(-dz, (double)t30.x(), (double)wf0.x()) - (double)Gm.x(), (double)wp.x()));
+            fb[0] = __dmul_rn(ab.x, __fma_rn(cw, __fma_rn(-dz, (double)t30.y(), (double)wf0.y()) - (double)Gm.y(), (double)wp.y()));
           } else {        // stepwi.f90:325, gaussel.f90:189-240
-            const P2 rw = fma2(hi2(q6), Gpp - Gm, wp);
-            fa[l] = __fma_rn(ab.y, fa[l - 1], __dmul_rn(ab.x, (double)px(rw)));
-            fb[l] = __fma_rn(ab.y, fb[l - 1], __dmul_rn(ab.x, (double)py(rw)));
+            const F2 rw = fma2(hi2(q6), Gpp - Gm, wp);
+            fa[l] = __fma_rn(ab.y, fa[l - 1], __dmul_rn(ab.x, (double)rw.x()));
+            fb[l] = __fma_rn(ab.y, fb[l - 1], __dmul_rn(ab.x, (double)rw.y()));
           }
           Gpp = Gp;
           if (l == L - 1) {   // what this chunk hands to the one above
-            const double dz = (double)px(dziv);
+            const double dz = (double)dziv.x();
             const double2 e = *reinterpret_cast<const double2*>(smem + Y::oN + 16 * c);   // bn, an
             double xa = fa[l], xb = fb[l];
             if (nlev < L) xa = xb = 0.0;
             *reinterpret_cast<double2*>(smem + Y::oE + 16 * (c * 32 + lane)) =
-                make_double2(__fma_rn(e.x, xa, __dmul_rn(e.y, __fma_rn((double)px(t3l), dz, (double)px(Gpp)))),
-                             __fma_rn(e.x, xb, __dmul_rn(e.y, __fma_rn((double)py(t3l), dz, (double)py(Gpp)))));
+                make_double2(__fma_rn(e.x, xa, __dmul_rn(e.y, __fma_rn((double)t3l.x(), dz, (double)Gpp.x()))),
+                             __fma_rn(e.x, xb, __dmul_rn(e.y, __fma_rn((double)t3l.y(), dz, (double)Gpp.y()))));
           }
           vsp[l] = vs;
         }
         // stepuv.f90:294 with pgrad.f90:379: the west u face
         const ulonglong2 q7 = T(l, 7), q8 = T(l, 8);
-        const P2 un = fma2(lo2(q7), fma2(west(t) - t, dxiv, S(Y::sUF, l)), u);
+        const F2 un = fma2(lo2(q7), fma2(west(t) - t, dxiv, S(Y::sUF, l)), u);
         if (l < nlev) {
           emit(pv, l, vs, fv);
           emit(pu, l, un, fu);
@@ -337,7 +305,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
           }
         }
         // advbspi.f90:158 without the v part of diver2d.f90:288
-        const P2 B = fma2(lo2(q8), w + w1, fma2(hi2(q7), un - east(un), S(Y::sPF, l)));
+        const F2 B = fma2(lo2(q8), w + w1, fma2(hi2(q7), un - east(un), S(Y::sPF, l)));
         set(2 * l, fma2(hi2(q8), w - w1, B));
         pk[l] = p;
         if (l == 0) { set(1, w); wf0 = wf; t30 = t3; }
@@ -393,15 +361,15 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     }
     // back substitution (gaussel.f90:254) and the p' update (steppi.f90:217,
     // diverpiv.f90:124, advbspi.f90:175)
-    P2 wup = p2((float)ya, (float)yb);
+    F2 wup = f2((float)ya, (float)yb);
 #pragma unroll
     for (int l = L - 1; l >= 0; --l) {
       const ulonglong2 q9 = T(l, 9);
       const double cp = D(l, 1).x;
       ya = __fma_rn(-cp, ya, fa[l]);
       yb = __fma_rn(-cp, yb, fb[l]);
-      const P2 wn = p2((float)ya, (float)yb);
-      const P2 pn = fma2(hi2(q9), wn - wup, fma2(lo2(q9), wn + wup, q[l]));
+      const F2 wn = f2((float)ya, (float)yb);
+      const F2 pn = fma2(hi2(q9), wn - wup, fma2(lo2(q9), wn + wup, q[l]));
       if (l < nlev) {
         emit(pw, l, wn, o1);
         emit(pp, l, pn, o1);

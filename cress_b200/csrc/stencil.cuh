@@ -10,35 +10,39 @@
 namespace cress {
 
 // 4th-order smoothing increments (smoo4s.f90:199-296 and its u/v/w/p
-// variants) added to frc at a point of level k: A(dx, dy, dz) returns the
-// smoothed quantity at an offset, and may be evaluated at every dz in
-// -2..2 (a shared-memory ring that holds those levels, whatever they
-// contain at the ends of the column).  The reference clamps the vertical
-// second difference at kmin and kmax (tmp3(kmin-1) = tmp3(kmin),
-// tmp3(kmax+1) = tmp3(kmax)); here that is a selection, so every offset is
-// a compile-time constant.
-// T is float, or F2 (f2.cuh) for two points at once.  edge: the points
-// (bit 0 first, bit 1 second) in an open-x boundary column, where only the
-// 2nd-order part applies (smoo4uvw.f90:286-330 and the other smoo4*: the
-// 4th-order loops run over i = 2+iwest .. with iwest = 1).
-template <class T, class FA>
-__device__ __forceinline__ T smooth_tile(T frc, int smtopt, float smhcoe, float smvcoe, int k, int kmin, int kmax,
-                                         const FA& A, int edge = 0) {
-  auto t1 = [&](int x) { return (A(x + 1, 0, 0) + A(x - 1, 0, 0)) - 2.f * A(x, 0, 0); };
-  auto t2 = [&](int y) { return (A(0, y + 1, 0) + A(0, y - 1, 0)) - 2.f * A(0, y, 0); };
-  auto t3 = [&](int z) { return (A(0, 0, z + 1) + A(0, 0, z - 1)) - 2.f * A(0, 0, z); };
-  const T t10 = t1(0), t20 = t2(0), t30 = t3(0);
-  frc = frc + smhcoe * (t10 + t20) + smvcoe * t30;
-  const T frc2 = frc;
-  if (smtopt % 10 == 2) {
-    frc = frc + smhcoe * ((t10 - (t1(1) + t1(-1))) + (t20 - (t2(1) + t2(-1))));
-  } else {
-    const T t3p = k >= kmax ? t30 : t3(1);    // tmp3(kmax+1) = tmp3(kmax)
-    const T t3m = k <= kmin ? t30 : t3(-1);   // tmp3(kmin-1) = tmp3(kmin)
-    frc = frc + (smvcoe * (t30 - (t3p + t3m)) +
-                 smhcoe * ((t10 - (t1(1) + t1(-1))) + (t20 - (t2(1) + t2(-1)))));
+// variants) added to frc at a pair of points of level k.  The smoothed quantity is
+// a field times (and less) per-level constants, so that along x and y only
+// the constant factor remains: H(dx, dy) is the field itself on level k,
+// smhc the coefficient times that factor; A(dz) is the smoothed quantity on
+// the own column, and may be evaluated at every dz in -2..2 (a shared-memory
+// ring that holds those levels, whatever they contain at the ends of the
+// column).  The reference's nested second differences are one weighted sum
+// per direction, -(H(2) + H(-2)) + 4 (H(1) + H(-1)) - 6 H(0); it differs from
+// them by FP32 rounding, about 1e-6 of the field times the coefficient
+// (1e-3).  The reference clamps the vertical second difference at kmin and
+// kmax (tmp3(kmin-1) = tmp3(kmin), tmp3(kmax+1) = tmp3(kmax)); here that is a
+// selection, so every offset is a compile-time constant.
+// edge: the points (bit 0 first, bit 1 second) in an open-x boundary column,
+// where only the 2nd-order part applies (smoo4uvw.f90:286-330 and the other
+// smoo4*: the 4th-order loops run over i = 2+iwest .. with iwest = 1).
+template <class FH, class FA>
+__device__ __forceinline__ F2 smooth_sum(F2 frc, int smtopt, float smhc, float smvcoe, int k, int kmin, int kmax,
+                                         const FH& H, const FA& A, int edge = 0) {
+  const F2 c = H(0, 0);
+  const F2 n1 = (H(1, 0) + H(-1, 0)) + (H(0, 1) + H(0, -1));
+  const F2 n2 = (H(2, 0) + H(-2, 0)) + (H(0, 2) + H(0, -2));
+  const F2 h4 = fma2(f2(-12.f), c, fma2(f2(4.f), n1, F2{0} - n2));
+  const F2 a0 = A(0), am = A(-1), ap = A(1);
+  const F2 t30 = (ap + am) - 2.f * a0;
+  F2 v = t30;
+  if (smtopt % 10 != 2) {
+    const F2 t3p = k >= kmax ? t30 : (A(2) + a0) - 2.f * ap;    // tmp3(kmax+1) = tmp3(kmax)
+    const F2 t3m = k <= kmin ? t30 : (a0 + A(-2)) - 2.f * am;   // tmp3(kmin-1) = tmp3(kmin)
+    v = (t30 + t30) - (t3p + t3m);
   }
-  return edge ? sel2(edge, frc2, frc) : frc;
+  const F2 r = fma2(f2(smvcoe), v, fma2(f2(smhc), h4, frc));
+  if (!edge) return r;
+  return sel2(edge, fma2(f2(smvcoe), t30, fma2(f2(smhc), fma2(f2(-4.f), c, n1), frc)), r);
 }
 
 // Turbulent mixing of a scalar S (the full field at t-dt) at a point of
