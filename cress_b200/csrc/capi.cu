@@ -445,6 +445,44 @@ int Ctx::row_ends_future() {
   return rc ? set_error(rc, "small-step launch failed: %s", cudaGetErrorString(cudaGetLastError())) : CRESS_OK;
 }
 
+// The microphysics' level table of one step length (micro.cuh), kept per
+// distinct one like the large step's; a new base state rewrites the tables
+// in place (captured steps read them).
+int Ctx::refresh_micro_tables() {
+  std::vector<MicroLevel> t(g.nk + 1);
+  for (auto& kv : micro_tables) {
+    float dtb;
+    std::memcpy(&dtb, &kv.first, 4);
+    micro_levels(col_h.data(), g.nk, dtb, t.data());
+    int rc;
+    if ((rc = cuda_check(cudaMemcpyAsync(kv.second, t.data(), sizeof(MicroLevel) * t.size(), cudaMemcpyHostToDevice,
+                                         stream), "copy microphysics table")) ||
+        (rc = cuda_check(cudaStreamSynchronize(stream), "sync microphysics table")))
+      return rc;
+  }
+  return CRESS_OK;
+}
+
+int Ctx::micro_table(float dtb, const MicroLevel** out) {
+  uint32_t key;
+  std::memcpy(&key, &dtb, 4);
+  auto it = micro_tables.find(key);
+  if (it != micro_tables.end()) { *out = it->second; return CRESS_OK; }
+  std::vector<MicroLevel> t(g.nk + 1);
+  micro_levels(col_h.data(), g.nk, dtb, t.data());
+  MicroLevel* d = nullptr;
+  int rc;
+  if ((rc = cuda_check(cudaMalloc(&d, sizeof(MicroLevel) * t.size()), "cudaMalloc microphysics table"))) return rc;
+  owned.push_back(d);
+  if ((rc = cuda_check(cudaMemcpyAsync(d, t.data(), sizeof(MicroLevel) * t.size(), cudaMemcpyHostToDevice, stream),
+                       "copy microphysics table")) ||
+      (rc = cuda_check(cudaStreamSynchronize(stream), "sync microphysics table")))
+    return rc;
+  micro_tables.emplace(key, d);
+  *out = d;
+  return CRESS_OK;
+}
+
 int Ctx::small_steps(int nsstp, float dts) { return small_steps(nsstp, dts, nullptr, nullptr); }
 
 int Ctx::small_steps(int nsstp, float dts, std::vector<HeviJob>* jobs, std::vector<HeviRowJob>* rjobs) {
@@ -854,7 +892,9 @@ int Ctx::cloudphy(float dtb, float thresq, bool defer_adjstni) {
   m.dz = cfg.dz;
   m.thresq = thresq;
   m.defer_adjstni = defer_adjstni ? 1 : 0;
+  m.mc = micro_const(m.dtb);
   int rc;
+  if ((rc = micro_table(m.dtb, &m.lv))) return rc;
   if (sampler) {
     // tuples of the plain scheme on this step's state (before it changes)
     const long long room = sampler->tcap - sampler->ntup;
@@ -1545,7 +1585,7 @@ int cress_set_base3d(cress_ctx* ctx, const float* const* b3) {
   if (rc) return rc;
   c->thomas.clear();
   c->base_set = true;
-  return CRESS_OK;
+  return c->refresh_micro_tables();
 }
 
 int cress_put_field(cress_ctx* ctx, int field, int level, const float* host) {
@@ -1697,7 +1737,7 @@ int cress_set_base_moist(cress_ctx* ctx, const float* pbr, const float* qvbr) {
   if (rc) return rc;
   if ((rc = cuda_check(cudaStreamSynchronize(c->stream), "sync moist columns"))) return rc;
   c->moist_set = true;
-  return CRESS_OK;
+  return c->refresh_micro_tables();
 }
 
 int cress_cloudphy(cress_ctx* ctx, float dtb, float thresq) {

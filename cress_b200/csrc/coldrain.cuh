@@ -57,6 +57,10 @@ struct MCell {
   R ptpf, qvf, qcf, qrf, qif, qsf, qgf, ncif, ncsf, ncgf;
   // fall speeds of the past level (termblk)
   R ucq, urq, uiq, usq, ugq, ucn, urn, uin, usn, ugn;
+  // ln(q / (cc rho n)) of rain, snow, graupel at t-dt (termblk): three times the
+  // logarithm of the mean diameter, from which every power of it follows
+  R lqr, lqs, lqg;
+  const MicroLevel* lv;   // the cell's level
 };
 
 // sqrt(sqrt(x)); for x = +-0 it returns x, which is what the two square
@@ -65,12 +69,11 @@ struct MCell {
 __device__ __forceinline__ R root4(R x) { return x == R(0) ? x : sqrtf(sqrtf(x)); }
 
 // s_diagnw, SrcOrig/diagnw.f90:120-160: diagnosed cloud and rain numbers.
-__device__ inline void diagnw_cell(R rbr, R qr, R& ncc, R& ncr) {
+__device__ inline void diagnw_cell(const MicroLevel& lv, R qr, R& ncc, R& ncr) {
   const R mrmiv2 = R(1.e-2) / R(MP::mrmax), mr0iv2 = R(1.e2) / R(MP::mr0);
   const R cdiaqr = R(MP::nr0) * R(MP::nr0) * R(MP::nr0) / (R(MP::cc) * R(MP::rhow));
-  const R rbv = R(1) / rbr;
-  ncc = R(MP::nclcst) * rbv;
-  ncr = root4(cdiaqr * rbr * qr) * rbv;
+  ncc = lv.ncc;
+  ncr = root4(cdiaqr * lv.rbr * qr) * lv.rbv;
   ncr = fminf(fmaxf(ncr, mrmiv2 * qr), mr0iv2 * qr);
 }
 
@@ -102,17 +105,22 @@ __device__ inline void termblk_cell(R thresq, MCell& c) {
   const R cdiaqg = R(1) / (R(MP::cc) * R(MP::rhog));
   if (c.qcp > thresq) { c.ucq = R(MP::ucqcst); c.ucn = R(MP::ucncst); } else { c.ucq = R(0); c.ucn = R(0); }
   if (c.qip > thresq) { c.uiq = R(MP::uiqcst); c.uin = R(MP::uincst); } else { c.uiq = R(0); c.uin = R(0); }
-  const R lnr0r = logf(R(MP::r0) * c.rbv);
+  static_assert(MP::gur == .5 && MP::gus == .5 && MP::gug == .5, "MicroLevel::sr0v is the square root");
+  const R sr = c.lv->sr0v;
+  c.lqr = c.lqs = c.lqg = R(0);
   if (c.qrp > thresq) {
-    c.urq = curq * expf(R(MP::gur) * lnr0r) * expf(bur3 * logf(cdiaqr * c.qrp / c.ncrp));
+    c.lqr = logf(cdiaqr * c.qrp / c.ncrp);
+    c.urq = curq * sr * expf(bur3 * c.lqr);
     c.urn = curn * c.urq;
   } else { c.urq = R(0); c.urn = R(0); }
   if (c.qsp > thresq) {
-    c.usq = cusq * expf(R(MP::gus) * lnr0r) * expf(bus3 * logf(cdiaqs * c.qsp / c.ncsp));
+    c.lqs = logf(cdiaqs * c.qsp / c.ncsp);
+    c.usq = cusq * sr * expf(bus3 * c.lqs);
     c.usn = cusn * c.usq;
   } else { c.usq = R(0); c.usn = R(0); }
   if (c.qgp > thresq) {
-    c.ugq = cugq * expf(R(MP::gug) * lnr0r) * expf(bug3 * logf(cdiaqg * c.qgp / c.ncgp));
+    c.lqg = logf(cdiaqg * c.qgp / c.ncgp);
+    c.ugq = cugq * sr * expf(bug3 * c.lqg);
     c.ugn = cugn * c.ugq;
   } else { c.ugq = R(0); c.ugn = R(0); }
 }
@@ -120,7 +128,8 @@ __device__ inline void termblk_cell(R thresq, MCell& c) {
 // s_srcblk cphopt=3, haiopt=0 (SrcOrig/srcblk.f90:488-630) on one cell:
 // setblk, the process routines, more0q and newblk in the reference order.
 // dtb is the microphysics step passed to coldblk (2*dtb of the leapfrog).
-__device__ inline void srcblk_cell(R dtb, R thresq, MCell& c) {
+__device__ inline void srcblk_cell(R dtb, R thresq, const MicroConst& mc, MCell& c) {
+  const MicroLevel& lv_ = *c.lv;
     const R oned3 = R(MP::oned3), cc = R(MP::cc), t0 = R(MP::t0), tlow = R(MP::tlow);
   const R qv = c.qvp, qc = c.qcp, qr = c.qrp, qi = c.qip, qs = c.qsp, qg = c.qgp;
   const R ncc = c.nccp, ncr = c.ncrp, nci = c.ncip, ncs = c.ncsp, ncg = c.ncgp;
@@ -130,18 +139,12 @@ __device__ inline void srcblk_cell(R dtb, R thresq, MCell& c) {
   const R cwmci = R(MP::cw) - R(MP::ci);
   const R epses0 = R(MP::epsva) * R(MP::es0);
   const R t23iv = R(1) / R(MP::t23);
-  R cdv = R(1) / t0;
-  const R cnu = expf(R(.57013) * logf(R(MP::nu0))) * cdv;
-  cdv = expf(R(.55249) * logf(R(MP::dv0))) * cdv;
-  const R pdiaqr = R(.5) * (R(5) + R(MP::bur)) - R(1);
-  const R pdiaqs = R(.5) * (R(5) + R(MP::bus)) - R(1);
-  const R pdiaqg = R(.5) * (R(5) + R(MP::bug)) - R(1);
+  const R cnu = mc.cnu, cdv = mc.cdv;
+  const R pdiaqr3 = oned3 * (R(.5) * (R(5) + R(MP::bur)) - R(1));   // exponents of exp(3 ln diameter)
+  const R pdiaqs3 = oned3 * (R(.5) * (R(5) + R(MP::bus)) - R(1));
+  const R pdiaqg3 = oned3 * (R(.5) * (R(5) + R(MP::bug)) - R(1));
   const R ccrw6 = R(6) / (cc * R(MP::rhow)), ccri6 = R(6) / (cc * R(MP::rhoi));
-  const R cdiaqr = R(1) / (cc * R(MP::rhow)), cdiaqs = R(1) / (cc * R(MP::rhos));
-  const R cdiaqg = R(1) / (cc * R(MP::rhog));
-  const R cvntr = R(.31) * sqrtf(R(MP::aur)) * expf(oned3 * logf(R(MP::sc))) * R(MP::gf5bur);
-  const R cvnts = R(.31) * sqrtf(R(MP::aus)) * expf(oned3 * logf(R(MP::sc))) * R(MP::gf5bus);
-  const R cvntg = R(.31) * sqrtf(R(MP::aug)) * expf(oned3 * logf(R(MP::sc))) * R(MP::gf5bug);
+  const R cvntr = mc.cvntr, cvnts = mc.cvnts, cvntg = mc.cvntg;
   const R t = (c.ptbr + c.ptpp) * c.pi;
   const R tcel = t - t0;
   const R esi = R(MP::es0) * expf(R(21.875) * tcel / (t - R(7.66)));
@@ -177,21 +180,21 @@ __device__ inline void srcblk_cell(R dtb, R thresq, MCell& c) {
   const R kp = (R(MP::kp0) / (R(120) + t)) * expf(R(1.5) * logf(t23iv * t));
   const R mu = rbr * nu;
   const R dv = p20dvp * expf(R(1.81) * logf(cdv * t));
-  const R cvnt = sqrtf(sqrtf(R(MP::r0) * rbv) / nu);
+  const R cvnt = sqrtf(lv_.sr0v / nu);
   R diaqc, diaqr, vntr, mi, diaqi, diaqs, vnts, diaqg, vntg;
   if (qc > thresq) diaqc = expf(oned3 * logf(ccrw6 * qc / ncc)); else diaqc = R(0);
   if (qr > thresq) {
-    diaqr = expf(oned3 * logf(cdiaqr * qr / ncr));
-    vntr = rbr * ncr * (R(.78) * diaqr + cvnt * cvntr * expf(pdiaqr * logf(diaqr)));
+    diaqr = expf(oned3 * c.lqr);
+    vntr = rbr * ncr * (R(.78) * diaqr + cvnt * cvntr * expf(pdiaqr3 * c.lqr));
   } else { diaqr = R(0); vntr = R(0); }
   if (qi > thresq) { mi = qi / nci; diaqi = expf(oned3 * logf(ccri6 * mi)); } else { mi = R(0); diaqi = R(0); }
   if (qs > thresq) {
-    diaqs = expf(oned3 * logf(cdiaqs * qs / ncs));
-    vnts = rbr * ncs * (R(.78) * diaqs + cvnt * cvnts * expf(pdiaqs * logf(diaqs)));
+    diaqs = expf(oned3 * c.lqs);
+    vnts = rbr * ncs * (R(.78) * diaqs + cvnt * cvnts * expf(pdiaqs3 * c.lqs));
   } else { diaqs = R(0); vnts = R(0); }
   if (qg > thresq) {
-    diaqg = expf(oned3 * logf(cdiaqg * qg / ncg));
-    vntg = rbr * ncg * (R(.78) * diaqg + cvnt * cvntg * expf(pdiaqg * logf(diaqg)));
+    diaqg = expf(oned3 * c.lqg);
+    vntg = rbr * ncg * (R(.78) * diaqg + cvnt * cvntg * expf(pdiaqg3 * c.lqg));
   } else { diaqg = R(0); vntg = R(0); }
 
   // ---- s_nuc1stv (nuc1stv.f90:179-216)
@@ -240,7 +243,7 @@ __device__ inline void srcblk_cell(R dtb, R thresq, MCell& c) {
   R clcr, clcs, clcg, clri, clrs, clrg, clir, clis, clig, clsr, clsg, clrin, clrsn, clsrn, clsgn, ecs;
   {
     const R rwdv9 = R(MP::oned9) * R(MP::rhow);
-    const R bur2 = R(2) + R(MP::bur), bus2 = R(2) + R(MP::bus), bug2 = R(2) + R(MP::bug);
+    const R bur23 = oned3 * (R(2) + R(MP::bur)), bus23 = oned3 * (R(2) + R(MP::bus)), bug23 = oned3 * (R(2) + R(MP::bug));
     const R esgiv = R(1) / R(MP::esg);
     const R cclcr = R(.25) * R(MP::aur) * R(MP::gf3bur) * cc * dtb;
     const R cclcs = R(.25) * R(MP::aus) * R(MP::gf3bus) * cc * dtb;
@@ -254,13 +257,13 @@ __device__ inline void srcblk_cell(R dtb, R thresq, MCell& c) {
     const R cclsg = R(MP::esg) * cc * cc * R(MP::rhos) * dtb;
     const R cclrsn = R(.5) * R(MP::ers) * cc * dtb;
     const R cclsgn = R(.5) * R(MP::esg) * cc * dtb;
-    const R r0rsq = sqrtf(R(MP::r0) * rbr);
+    const R r0rsq = lv_.sr0r;
     R diaqr2, diaqr3, qr2b, diaqs2, diaqs3, qs2b, diaqg2, qg2b;
-    if (qr > thresq) { diaqr2 = diaqr * diaqr; diaqr3 = diaqr * diaqr2; qr2b = r0rsq * expf(bur2 * logf(diaqr)); }
+    if (qr > thresq) { diaqr2 = diaqr * diaqr; diaqr3 = diaqr * diaqr2; qr2b = r0rsq * expf(bur23 * c.lqr); }
     else { diaqr2 = R(0); diaqr3 = R(0); qr2b = R(0); }
-    if (qs > thresq) { diaqs2 = diaqs * diaqs; diaqs3 = diaqs * diaqs2; qs2b = r0rsq * expf(bus2 * logf(diaqs)); }
+    if (qs > thresq) { diaqs2 = diaqs * diaqs; diaqs3 = diaqs * diaqs2; qs2b = r0rsq * expf(bus23 * c.lqs); }
     else { diaqs2 = R(0); diaqs3 = R(0); qs2b = R(0); }
-    if (qg > thresq) { diaqg2 = diaqg * diaqg; qg2b = r0rsq * expf(bug2 * logf(diaqg)); }
+    if (qg > thresq) { diaqg2 = diaqg * diaqg; qg2b = r0rsq * expf(bug23 * c.lqg); }
     else { diaqg2 = R(0); qg2b = R(0); }
     const R urq = c.urq, usq = c.usq, ugq = c.ugq, urn = c.urn, usn = c.usn, ugn = c.ugn;
     if (t > tlow) {
@@ -393,12 +396,10 @@ __device__ inline void srcblk_cell(R dtb, R thresq, MCell& c) {
   // ---- s_aggregat cphopt=3 (aggregat.f90:150-191, 434-469)
   R agin, agsn;
   {
-    const R expo1 = oned3 * (R(2) + R(MP::bus)), expo2 = oned3 * (R(4) - R(MP::bus));
-    const R cagin = R(MP::r0) * expf(R(3) * logf(R(.5) * R(MP::aui) * R(MP::eii) * R(MP::xl) / R(MP::rhoi) * dtb));
-    const R cagsn = R(3.47222e-4) * R(MP::aus) * R(MP::ess) * R(MP::hfbus) * dtb *
-                    expf(oned3 * (R(1) - R(MP::bus)) * logf(cc)) * expf(-oned3 * (R(2) + R(MP::bus)) * logf(R(MP::rhos)));
-    if (qi > thresq) agin = rbr * nci * qi * expf(oned3 * logf(cagin * rbv)); else agin = R(0);
-    if (qs > thresq) agsn = cagsn * rbr * expf(expo1 * logf(qs)) * expf(expo2 * logf(ncs)); else agsn = R(0);
+    // qs^((2+bus)/3) ncs^((4-bus)/3) = ncs^2 (qs/ncs)^((2+bus)/3)
+    const R expo1 = oned3 * (R(2) + R(MP::bus));
+    if (qi > thresq) agin = lv_.agin * nci * qi; else agin = R(0);
+    if (qs > thresq) agsn = mc.agsn * rbr * (ncs * ncs) * expf(expo1 * c.lqs); else agsn = R(0);
   }
 
   // ---- s_melting (melting.f90:150, 278-360)
@@ -453,23 +454,21 @@ __device__ inline void srcblk_cell(R dtb, R thresq, MCell& c) {
   // ---- s_convers cphopt>=3 (convers.f90:180-225, 604-719)
   R cncr, cnis, cnsg, cnsgn;
   {
-    const R busm1 = R(MP::bus) - R(1);
+    const R busm13 = oned3 * (R(MP::bus) - R(1));
     const R ms05 = R(.5) * R(MP::ms0);
     const R qccm = R(MP::oned6) * R(MP::rhow) * cc * R(MP::diaqcm) * R(MP::diaqcm) * R(MP::diaqcm);
-    const R diaqs0 = expf(oned3 * logf(R(6) * R(MP::ms0) / (cc * R(MP::rhos))));
-    const R cagin = R(MP::r0) * expf(R(3) * logf(R(.5) * oned3 * R(MP::aui) * R(MP::eii) * R(MP::xl) / R(MP::rhoi) * dtb));
-    const R ccncr = R(.104) * R(kGrav) * R(MP::ecc) * expf(-oned3 * logf(R(MP::rhow))) * dtb;
+    const R diaqs0 = mc.diaqs0;
     R ccnsgn = R(1) / (R(MP::rhog) - R(MP::rhos));
     const R ccnsg = R(MP::rhog) * ccnsgn;
     ccnsgn = R(1.5) * R(MP::aus) * R(MP::gfbus) * sqrtf(R(MP::r0)) * ccnsgn * dtb;
     if (qc > thresq) {
       const R qcm = qccm * ncc;
-      if (t > tlow && qc >= qcm) cncr = ccncr * rbr * expf(-oned3 * logf(ncc)) * expf(R(MP::sevnd3) * logf(qc)) / mu;
+      if (t > tlow && qc >= qcm) cncr = lv_.cncr * expf(R(MP::sevnd3) * logf(qc)) / mu;
       else cncr = R(0);
     } else cncr = R(0);
     if (t < t0) {
       if (qi > thresq) {
-        cnis = rbr * expf(oned3 * logf(cagin * rbv)) * qi * qi / logf(diaqs0 / diaqi);
+        cnis = lv_.cnis * qi * qi / logf(diaqs0 / diaqi);
         if (vdvi >= R(0)) {
           if (mi < ms05) cnis = cnis + mi / (R(MP::ms0) - mi) * vdvi;
           else cnis = cnis + (vdvi + (R(1) - ms05 / mi) * qi);
@@ -479,7 +478,7 @@ __device__ inline void srcblk_cell(R dtb, R thresq, MCell& c) {
       if (qs > thresq) {
         if (vdvs > R(0) && vdvs < clcs) {
           cnsg = fminf(ccnsg * clcs, qs);
-          cnsgn = fminf(ccnsgn * ecs * qc * ncs * sqrtf(rbr) * expf(busm1 * logf(diaqs)), ncs);
+          cnsgn = fminf(ccnsgn * ecs * qc * ncs * lv_.srbr * expf(busm13 * c.lqs), ncs);
         } else { cnsg = R(0); cnsgn = R(0); }
       } else { cnsg = R(0); cnsgn = R(0); }
     } else { cnis = R(0); cnsg = R(0); cnsgn = R(0); }

@@ -86,6 +86,9 @@ struct Ctx {
   int thomas_for(float dts, const HeviArgs& a, const ThomasSet** out);   // a: the step's scalars
   std::map<uint32_t, float*> level_tables;   // level table per 2*dtb (bits)
   int level_table(float dtb2, const float** out);
+  std::map<uint32_t, MicroLevel*> micro_tables;   // microphysics level table per step (bits)
+  int micro_table(float dtb, const MicroLevel** out);
+  int refresh_micro_tables();
   // whether the HE-VI substeps run the row-marching kernel
   bool row_kernel() const;
   int small_steps(int nsstp, float dts);

@@ -16,6 +16,7 @@
 // fall speeds k_micro_src stored, and the surface precipitation rate and
 // accumulation; k_adjstni then applies the final adjstni (coldblk.f90:469).
 #include <cuda_runtime.h>
+#include <cmath>
 #include "common.cuh"
 #include "hevi.cuh"
 #include "micro.cuh"
@@ -29,18 +30,19 @@ namespace {
 
 
 __device__ inline void load_cell(const MicroArgs& a, long long id, int k, MCell& c) {
-  const int nc = a.g.nk + 1;
   const float rddvcp = 287.f / 1004.f, p0iv = 1.f / 1.e5f;
-  c.ptbr = __ldg(a.col + C_PTBR * nc + k);
-  c.rbr = __ldg(a.col + C_RBR * nc + k);
-  c.rbv = 1.f / c.rbr;                                                  // getvdens.f90:106
-  c.p = __ldg(a.col + C_PBR * nc + k) + __ldg(a.ppp + id);              // getexner.f90:129
+  c.lv = a.lv + k;
+  const float4 v = __ldg(reinterpret_cast<const float4*>(c.lv));
+  c.ptbr = v.x;
+  c.rbr = v.y;
+  c.rbv = v.z;                                                          // getvdens.f90:106
+  c.p = v.w + __ldg(a.ppp + id);                                        // getexner.f90:129
   c.pi = expf(rddvcp * logf(p0iv * c.p));                               // getexner.f90:131
   c.ptpp = __ldg(a.ptpp + id); c.qvp = __ldg(a.qvp + id); c.qcp = __ldg(a.qcp + id);
   c.qrp = __ldg(a.qrp + id); c.qip = __ldg(a.qip + id); c.qsp = __ldg(a.qsp + id);
   c.qgp = __ldg(a.qgp + id); c.ncip = __ldg(a.nip + id); c.ncsp = __ldg(a.nsp + id);
   c.ncgp = __ldg(a.ngp + id);
-  diagnw_cell(c.rbr, c.qrp, c.nccp, c.ncrp);                           // cloudphy.f90:366
+  diagnw_cell(*c.lv, c.qrp, c.nccp, c.ncrp);                           // cloudphy.f90:366
 }
 
 // The fall speeds of the past level (termblk) in the order the
@@ -70,7 +72,7 @@ __global__ void __launch_bounds__(256, 3) k_micro_src(const MicroArgs a) {
     adjstni_cell(c.rbr, c.rbv, c.qif, c.qsf, c.qgf, c.ncif, c.ncsf, c.ncgf);   // coldblk.f90:327
     termblk_cell(a.thresq, c);                                                // coldblk.f90:344
     store_speeds(a, id, c);
-    srcblk_cell(a.dtb, a.thresq, c);                                          // coldblk.f90:356
+    srcblk_cell(a.dtb, a.thresq, a.mc, c);                                          // coldblk.f90:356
     adjstni_cell(c.rbr, c.rbv, c.qif, c.qsf, c.qgf, c.ncif, c.ncsf, c.ncgf);   // coldblk.f90:425
     a.ptpf[id] = c.ptpf; a.qvf[id] = c.qvf; a.qcf[id] = c.qcf; a.qrf[id] = c.qrf;
     a.qif[id] = c.qif; a.qsf[id] = c.qsf; a.qgf[id] = c.qgf; a.nif[id] = c.ncif;
@@ -78,11 +80,8 @@ __global__ void __launch_bounds__(256, 3) k_micro_src(const MicroArgs a) {
     // fallblk.f90:362-377 (flqcqi_opt=1: cloud water and ice fall too)
     const float eps = 1.e-20f;
     const float dzjcb = a.dz * __ldg(a.col + C_JCB * (g.nk + 1) + k);
-    lim = fminf(lim, dzjcb / (c.ucq + eps));
-    lim = fminf(lim, dzjcb / (c.urq + eps));
-    lim = fminf(lim, dzjcb / (c.uiq + eps));
-    lim = fminf(lim, dzjcb / (c.usq + eps));
-    lim = fminf(lim, dzjcb / (c.ugq + eps));
+    // the smallest of the five quotients is that of the largest speed
+    lim = dzjcb / (fmaxf(fmaxf(fmaxf(c.ucq, c.urq), fmaxf(c.uiq, c.usq)), c.ugq) + eps);
   }
   for (int o = 16; o > 0; o >>= 1) lim = fminf(lim, __shfl_xor_sync(0xffffffffu, lim, o));
   if ((threadIdx.x & 31) == 0 && lim < 3.0e38f) atomicMin(a.dtp_bits, __float_as_int(lim));
@@ -423,6 +422,47 @@ int launch_cloudphy_fused(const MicroArgs& a, const float* w, Mlp* m, const Lear
   launch_fall(a, st);
   *launches += a.defer_adjstni ? 4 : 5;
   return cudaGetLastError() == cudaSuccess ? 0 : CRESS_E_CUDA;
+}
+
+MicroConst micro_const(float dtb) {
+  MicroConst c;
+  const double o3 = MP::oned3, cc = MP::cc;
+  c.cnu = (float)(std::pow(MP::nu0, .57013) / MP::t0);
+  c.cdv = (float)(std::pow(MP::dv0, .55249) / MP::t0);
+  const double sc3 = .31 * std::pow(MP::sc, o3);
+  c.cvntr = (float)(sc3 * std::sqrt(MP::aur) * MP::gf5bur);
+  c.cvnts = (float)(sc3 * std::sqrt(MP::aus) * MP::gf5bus);
+  c.cvntg = (float)(sc3 * std::sqrt(MP::aug) * MP::gf5bug);
+  // aggregat.f90:150-191 times (cc rhos)^((2+bus)/3): the cell has ln(qs/(cc rhos ncs))
+  c.agsn = (float)(3.47222e-4 * MP::aus * MP::ess * MP::hfbus * (double)dtb * std::pow(cc, o3 * (1. - MP::bus)) *
+                   std::pow(MP::rhos, -o3 * (2. + MP::bus)) * std::pow(cc * MP::rhos, o3 * (2. + MP::bus)));
+  c.diaqs0 = (float)std::pow(6. * MP::ms0 / (cc * MP::rhos), o3);
+  return c;
+}
+
+void micro_levels(const float* col, int nk, float dtb, MicroLevel* out) {
+  const double o3 = MP::oned3;
+  const double ag = .5 * MP::aui * MP::eii * MP::xl / MP::rhoi * (double)dtb, cn = o3 * ag;
+  const double ccncr = .104 * (double)kGrav * MP::ecc * std::pow(MP::rhow, -o3) * (double)dtb;   // convers.f90
+  for (int k = 0; k <= nk; ++k) {
+    auto B = [&](int f) { return col[(size_t)f * (nk + 1) + k]; };
+    MicroLevel r{};
+    r.ptbr = B(C_PTBR);
+    r.rbr = B(C_RBR);
+    r.pbr = B(C_PBR);
+    if (r.rbr > 0.f) {
+      const double rb = (double)r.rbr;
+      r.rbv = 1.f / r.rbr;
+      r.sr0v = (float)std::sqrt(MP::r0 / rb);
+      r.sr0r = (float)std::sqrt(MP::r0 * rb);
+      r.srbr = (float)std::sqrt(rb);
+      r.ncc = (float)MP::nclcst * r.rbv;
+      r.agin = (float)(rb * std::pow(MP::r0 * ag * ag * ag / rb, o3));
+      r.cnis = (float)(rb * std::pow(MP::r0 * cn * cn * cn / rb, o3));
+      r.cncr = (float)(ccncr * rb * std::pow(MP::nclcst / rb, -o3));
+    }
+    out[k] = r;
+  }
 }
 
 }  // namespace cress

@@ -71,7 +71,7 @@ __device__ inline void plain_source(const MicroArgs& a, MCell c, float (&d)[kMlp
   const float pt0 = c.ptpf;
   adjstni_cell(c.rbr, c.rbv, c.qif, c.qsf, c.qgf, c.ncif, c.ncsf, c.ncgf);
   termblk_cell(a.thresq, c);
-  srcblk_cell(a.dtb, a.thresq, c);
+  srcblk_cell(a.dtb, a.thresq, a.mc, c);
   adjstni_cell(c.rbr, c.rbv, c.qif, c.qsf, c.qgf, c.ncif, c.ncsf, c.ncgf);
   const float e[kMlpOut] = {c.qvf, c.qcf, c.qrf, c.qif, c.qsf, c.qgf, c.ncif, c.ncsf, c.ncgf};
 #pragma unroll
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(128) k_micro_src_list(const MicroArgs a, long 
     load_future(a, id, c);
     adjstni_cell(c.rbr, c.rbv, c.qif, c.qsf, c.qgf, c.ncif, c.ncsf, c.ncgf);
     termblk_cell(a.thresq, c);
-    srcblk_cell(a.dtb, a.thresq, c);
+    srcblk_cell(a.dtb, a.thresq, a.mc, c);
     adjstni_cell(c.rbr, c.rbv, c.qif, c.qsf, c.qgf, c.ncif, c.ncsf, c.ncgf);
     a.ptpf[id] = c.ptpf; a.qvf[id] = c.qvf; a.qcf[id] = c.qcf; a.qrf[id] = c.qrf;
     a.qif[id] = c.qif; a.qsf[id] = c.qsf; a.qgf[id] = c.qgf; a.nif[id] = c.ncif;
