@@ -1470,9 +1470,9 @@ int cress_create(const cress_cfg* cfg, int device, cress_ctx** out) {
     c->owned.push_back(c->prec_d);
     c->owned.push_back(c->dtp_d);
     cudaMemsetAsync(c->prec_d, 0, pb, c->stream);
-    // fall speeds of the 8 sedimenting quantities (written by the process
+    // fall speeds of rain, snow and graupel (written by the process
     // rates, read by the column sedimentation)
-    const size_t ub = sizeof(float) * 8 * (size_t)c->g.plane * c->g.nk;
+    const size_t ub = sizeof(float) * 3 * (size_t)c->g.plane * c->g.nk;
     if ((rc = cuda_check(cudaMalloc(&c->uspd_d, ub), "cudaMalloc fall speeds"))) {
       delete c;
       return rc;

@@ -105,7 +105,7 @@ struct Ctx {
   bool large_set = false;  // cress_set_base_large was called
   bool moist_set = false;  // cress_set_base_moist was called
   float* prec_d = nullptr; // surface precipitation planes (10 x px*py)
-  float* uspd_d = nullptr; // fall speeds (8 fields)
+  float* uspd_d = nullptr; // fall speeds (3 fields)
   float* rkv_d = nullptr;  // eddy viscosity rbr*K at scalar points (tubopt 1 and 2)
   // TKE closure (tubopt=2), written by the eddy-viscosity kernel from the
   // past level: the scalar diffusivity 1/Pr*rkv/jcb, N^2 at w level k, and

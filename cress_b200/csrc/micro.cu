@@ -13,10 +13,12 @@
 // species are independent): recovers npstp and dtp from that minimum
 // (fallblk.f90:441-449) and runs the upwind sedimentation sub-steps of its
 // species column (upwqp.f90:160-225, upwnp.f90:140-176) with the past-level
-// fall speeds k_micro_src stored, and the surface precipitation rate and
-// accumulation; k_adjstni then applies the final adjstni (coldblk.f90:469).
+// fall speeds k_micro_src stored (rain, snow, graupel; the others follow from
+// the past level), and the surface precipitation rate and accumulation;
+// k_adjstni then applies the final adjstni (coldblk.f90:469).
 #include <cuda_runtime.h>
 #include <cmath>
+#include <type_traits>
 #include "common.cuh"
 #include "hevi.cuh"
 #include "micro.cuh"
@@ -45,14 +47,21 @@ __device__ inline void load_cell(const MicroArgs& a, long long id, int k, MCell&
   diagnw_cell(*c.lv, c.qrp, c.nccp, c.ncrp);                           // cloudphy.f90:366
 }
 
-// The fall speeds of the past level (termblk) in the order the
-// sedimentation kernel runs the species: cloud water, cloud ice, ice
-// number, rain, snow, graupel, snow number, graupel number.
+// The fall speeds of the past level (termblk) that depend on more than a
+// threshold: rain, snow, graupel.
 __device__ __forceinline__ void store_speeds(const MicroArgs& a, long long id, const MCell& c) {
   const long long n3 = (long long)a.g.plane * a.g.nk;
   float* u = a.uspd + id;
-  u[0] = c.ucq; u[n3] = c.uiq; u[2 * n3] = c.uin; u[3 * n3] = c.urq;
-  u[4 * n3] = c.usq; u[5 * n3] = c.ugq; u[6 * n3] = c.usn; u[7 * n3] = c.ugn;
+  u[0] = c.urq; u[n3] = c.usq; u[2 * n3] = c.ugq;
+}
+
+// The cell's limit on the sedimentation step, fallblk.f90:362-377
+// (flqcqi_opt=1: cloud water and ice fall too): the smallest of the five
+// quotients is that of the largest speed.
+__device__ __forceinline__ float fall_limit(const MicroArgs& a, int k, const MCell& c) {
+  const float eps = 1.e-20f;
+  const float dzjcb = a.dz * __ldg(a.col + C_JCB * (a.g.nk + 1) + k);
+  return dzjcb / (fmaxf(fmaxf(fmaxf(c.ucq, c.urq), fmaxf(c.uiq, c.usq)), c.ugq) + eps);
 }
 
 __global__ void __launch_bounds__(256, 3) k_micro_src(const MicroArgs a) {
@@ -77,22 +86,98 @@ __global__ void __launch_bounds__(256, 3) k_micro_src(const MicroArgs a) {
     a.ptpf[id] = c.ptpf; a.qvf[id] = c.qvf; a.qcf[id] = c.qcf; a.qrf[id] = c.qrf;
     a.qif[id] = c.qif; a.qsf[id] = c.qsf; a.qgf[id] = c.qgf; a.nif[id] = c.ncif;
     a.nsf[id] = c.ncsf; a.ngf[id] = c.ncgf;
-    // fallblk.f90:362-377 (flqcqi_opt=1: cloud water and ice fall too)
-    const float eps = 1.e-20f;
-    const float dzjcb = a.dz * __ldg(a.col + C_JCB * (g.nk + 1) + k);
-    // the smallest of the five quotients is that of the largest speed
-    lim = dzjcb / (fmaxf(fmaxf(fmaxf(c.ucq, c.urq), fmaxf(c.uiq, c.usq)), c.ugq) + eps);
+    lim = fall_limit(a, k, c);
   }
   for (int o = 16; o > 0; o >>= 1) lim = fminf(lim, __shfl_xor_sync(0xffffffffu, lim, o));
   if ((threadIdx.x & 31) == 0 && lim < 3.0e38f) atomicMin(a.dtp_bits, __float_as_int(lim));
 }
 
-// One thread per column and species (blockIdx.z).  npstp upwind sub-steps
-// of s_upwqp / s_upwnp (upwqp.f90:160-225, upwnp.f90:140-176) stream up the
-// column: the flux rbr*u*q of level k+1 is formed from the not yet updated
-// q(k+1) while q(k) is written, so a sub-step is one read and one write of
-// the column; the surface rate (flx(1)+flx(2))/2/rhow accumulates over
-// the sub-steps.
+// The fall speed of species f at a point, formed from what k_micro_src
+// stores (rain, snow and graupel speeds) and the past level: the cloud and
+// ice speeds are constants where there is cloud or ice, the snow and graupel
+// numbers fall at a constant times their mass's speed (termblk_cell).
+struct FallSpeed {
+  const float* p;
+  float thresq, c;
+  bool past;      // p is a past mixing ratio: c where it exceeds thresq
+  __device__ __forceinline__ float operator()(float v) const { return past ? (v > thresq ? c : 0.f) : c * v; }
+};
+
+// M upwind sub-steps of one column in one sweep up: sub-step s updates level
+// k-s when level k+1 arrives, from the values sub-step s-1 has just left
+// there.  The column is read once and written once; arithmetic and order
+// are those of M sweeps.  flx1, flx2: rbr u q at levels 1 and 2 before each
+// sub-step.
+template <int M>
+__device__ __forceinline__ void fall_sweep(float* fld, const FallSpeed& us, const MicroLevel* lv, float dzvdt,
+                                           long long pl, int nk, float (&flx1)[M], float (&flx2)[M]) {
+  float q[M], fl[M], qn[M], ru[M], org[M + 1];   // org[s]: the value in memory at level k-s
+  for (int s = 0; s < M; ++s) { q[s] = fl[s] = qn[s] = ru[s] = 0.f; }
+  for (int s = 0; s <= M; ++s) org[s] = 0.f;
+  // level k arrives with value v and speed u; EDGE: some sub-step is not
+  // inside its column yet or any more
+  auto step = [&](int k, float v, float u, auto edge) {
+    constexpr bool EDGE = decltype(edge)::value;
+#pragma unroll
+    for (int s = M - 1; s > 0; --s) ru[s] = ru[s - 1];
+#pragma unroll
+    for (int s = M; s > 0; --s) org[s] = org[s - 1];
+    org[0] = v;
+    ru[0] = EDGE && k > nk - 1 ? 0.f : lv[k].rbr * u;
+    float in = v;
+#pragma unroll
+    for (int s = 0; s < M; ++s) {
+      const int ks = k - s;   // the level whose value arrives at sub-step s
+      if (EDGE && ks < 1) break;
+      float out = qn[s];      // ks = nk: q(nk-1) = q(nk-2)
+      if (!EDGE || ks <= nk - 1) {
+        const float f = ru[s] * in;
+        if (EDGE && ks == 1) flx1[s] = f;
+        if (EDGE && ks == 2) flx2[s] = f;
+        if (!EDGE || ks >= 2) out = fmaxf(fmaf(f - fl[s], lv[ks - 1].rstv * dzvdt, q[s]), 0.f);
+        q[s] = in;
+        fl[s] = f;
+        qn[s] = out;
+      }
+      if (EDGE && (ks < 2 || ks > nk)) { in = out; continue; }
+      in = out;
+      // level ks-1 = k-M after the last sub-step; a value that has not
+      // changed (no condensate falls through it) is not written again
+      if (s == M - 1 && __float_as_uint(out) != __float_as_uint(org[M])) fld[(long long)(ks - 2) * pl] = out;
+    }
+  };
+  // levels in batches, loaded ahead of the batch's stores
+  constexpr int kAhead = 8;
+  using Edge = std::true_type;
+  using Inner = std::false_type;
+  for (int k = 1; k <= nk - 1 + M; k += kAhead) {
+    float v[kAhead], u[kAhead];
+#pragma unroll
+    for (int d = 0; d < kAhead; ++d) {
+      const bool in = k + d <= nk - 1;
+      v[d] = in ? fld[(long long)(k + d - 1) * pl] : 0.f;
+      u[d] = in ? __ldg(us.p + (long long)(k + d - 1) * pl) : 0.f;
+    }
+    if (k > M + 1 && k + kAhead - 1 <= nk - 1) {   // level 2 reaches the last sub-step at k = M+1
+#pragma unroll
+      for (int d = 0; d < kAhead; ++d) step(k + d, v[d], us(u[d]), Inner{});
+    } else {
+#pragma unroll
+      for (int d = 0; d < kAhead; ++d)
+        if (k + d <= nk - 1 + M) step(k + d, v[d], us(u[d]), Edge{});
+    }
+  }
+}
+
+// One thread per column and species (blockIdx.z): npstp upwind sub-steps of
+// s_upwqp / s_upwnp (upwqp.f90:160-225, upwnp.f90:140-176), up to four per
+// sweep of the column; the surface rate (flx(1)+flx(2))/2/rhow accumulates
+// over the sub-steps.
+//
+// What bounds it: memory, one read of the field and of its speed and one
+// write where the field changes, and the latency of a column's march, which
+// the batches of loads hide.  One sub-step per sweep, level by level, with eight
+// speed fields stored and read: 634 us at 512 x 512 x 64; this: 449.
 __global__ void __launch_bounds__(128) k_micro_fall(const MicroArgs a) {
   const Grid g = a.g;
   const int nk = g.nk;
@@ -114,9 +199,6 @@ __global__ void __launch_bounds__(128) k_micro_fall(const MicroArgs a) {
   const float dziv = 1.f / a.dz;
   const float dzvdt = dziv * dtp;
   const float rwiv05 = .5f / 1.e3f, dtp05 = .5f * dtp;
-  const int nc = nk + 1;
-  const float* crbr = a.col + C_RBR * nc;
-  const float* crst = a.col + C_RST * nc;
   const long long id1 = g.at(i, j, 1);
   const long long pl = g.plane;
   const long long n3 = pl * nk;
@@ -124,39 +206,34 @@ __global__ void __launch_bounds__(128) k_micro_fall(const MicroArgs a) {
   const long long pid = (long long)j * g.px + i;
   // species f: qc, qi, ni, qr, qs, qg, ns, ng; its precipitation slot
   // (prc, pri, -, prr, prs, prg, -, -)
-  float* const field = f == 0 ? a.qcf : f == 1 ? a.qif : f == 2 ? a.nif : f == 3 ? a.qrf
-                     : f == 4 ? a.qsf : f == 5 ? a.qgf : f == 6 ? a.nsf : a.ngf;
+  float* const fld = (f == 0 ? a.qcf : f == 1 ? a.qif : f == 2 ? a.nif : f == 3 ? a.qrf
+                    : f == 4 ? a.qsf : f == 5 ? a.qgf : f == 6 ? a.nsf : a.ngf) + id1;
   const int s = f == 0 ? 0 : f == 1 ? 2 : f == 3 ? 1 : f == 4 ? 3 : f == 5 ? 4 : -1;
-  {
-    float* fld = field + id1;
-    const float* u = a.uspd + f * n3 + id1;
-    float rate = 0.f, acc = 0.f;
-    if (s >= 0) { rate = a.prec[(2 * s) * pp2 + pid]; acc = a.prec[(2 * s + 1) * pp2 + pid]; }
-#pragma unroll 1
-    for (int it = 0; it < npstp; ++it) {
-      float q0 = fld[0];
-      float f0 = __ldg(crbr + 1) * __ldg(u) * q0;
-      const float flx1 = f0;
-      float flx2 = 0.f, qn = 0.f;
-#pragma unroll 4
-      for (int k = 1; k <= nk - 2; ++k) {
-        const long long o = (long long)k * pl;             // level k+1
-        const float q1 = fld[o];
-        const float f1 = __ldg(crbr + k + 1) * __ldg(u + o) * q1;
-        if (k == 1) flx2 = f1;
-        qn = fmaxf(q0 + (f1 - f0) / __ldg(crst + k) * dzvdt, 0.f);
-        fld[o - pl] = qn;
-        q0 = q1;
-        f0 = f1;
-      }
-      fld[(long long)(nk - 2) * pl] = qn;                   // q(nk-1) = q(nk-2)
-      if (s >= 0) {
-        rate = (flx1 + flx2) * rwiv05;
-        acc = acc + rate * dtp05;
-      }
+  FallSpeed us;
+  us.thresq = a.thresq;
+  us.past = f <= 2;
+  us.p = (f == 0 ? a.qcp : f <= 2 ? a.qip : a.uspd + (f == 3 ? 0 : f == 4 || f == 6 ? 1 : 2) * n3) + id1;
+  us.c = f == 0 ? (float)MP::ucqcst : f == 1 ? (float)MP::uiqcst : f == 2 ? (float)MP::uincst
+       : f == 6 ? 6.f * (float)MP::gf1bus / (float)MP::gf4bus
+       : f == 7 ? 6.f * (float)MP::gf1bug / (float)MP::gf4bug : 1.f;
+  float rate = 0.f, acc = 0.f;
+  if (s >= 0) acc = a.prec[(2 * s + 1) * pp2 + pid];
+  auto sweep = [&](auto m) {
+    constexpr int M = decltype(m)::value;
+    float flx1[M], flx2[M];
+    fall_sweep<M>(fld, us, a.lv, dzvdt, pl, nk, flx1, flx2);
+    for (int n = 0; n < M; ++n) {
+      rate = (flx1[n] + flx2[n]) * rwiv05;
+      acc = acc + rate * dtp05;
     }
-    if (s >= 0) { a.prec[(2 * s) * pp2 + pid] = rate; a.prec[(2 * s + 1) * pp2 + pid] = acc; }
-  }
+  };
+  int left = npstp;
+#pragma unroll 1
+  for (; left >= 4; left -= 4) sweep(std::integral_constant<int, 4>{});
+  if (left == 3) sweep(std::integral_constant<int, 3>{});
+  if (left == 2) sweep(std::integral_constant<int, 2>{});
+  if (left == 1) sweep(std::integral_constant<int, 1>{});
+  if (s >= 0) { a.prec[(2 * s) * pp2 + pid] = rate; a.prec[(2 * s + 1) * pp2 + pid] = acc; }
 }
 
 // coldblk.f90:467-470: adjstni once more after the sedimentation
@@ -453,6 +530,7 @@ void micro_levels(const float* col, int nk, float dtb, MicroLevel* out) {
     if (r.rbr > 0.f) {
       const double rb = (double)r.rbr;
       r.rbv = 1.f / r.rbr;
+      r.rstv = 1.f / B(C_RST);
       r.sr0v = (float)std::sqrt(MP::r0 / rb);
       r.sr0r = (float)std::sqrt(MP::r0 * rb);
       r.srbr = (float)std::sqrt(rb);

@@ -20,7 +20,7 @@ struct alignas(16) MicroLevel {
   float ncc;                    // diagnosed cloud number (diagnw.f90)
   float agin, cnis;             // rbr (cagin/rbr)^(1/3) of aggregat.f90 and convers.f90
   float cncr;                   // autoconversion's level factor (convers.f90)
-  float pad;
+  float rstv;                   // 1/rst
 };
 // The same for constants of the scheme and the step.
 struct MicroConst {
@@ -40,7 +40,7 @@ struct MicroArgs {
   // future level t+dt (updated)
   float *ptpf, *qvf, *qcf, *qrf, *qif, *qsf, *qgf, *nif, *nsf, *ngf;
   float* prec;       // 10 planes (px*py): prc, prr, pri, prs, prg x (rate, accumulated)
-  float* uspd;       // 8 fall-speed fields (past level), written by the process-rate kernels
+  float* uspd;       // fall speeds of rain, snow and graupel (past level), written by the process-rate kernels
   int* dtp_bits;     // domain minimum of the sedimentation step (float bits, positive)
   float dtb;         // microphysics step = 2*dtb of the leapfrog (cloudphy.f90:282)
   float dz, thresq;

@@ -1,5 +1,5 @@
-"""The moist scalars' kernel and the microphysics' per-level table at their
-edges, against the CPU oracle with the criteria of the moist large steps
+"""The moist scalars' kernel, the sedimentation's sweeps and the microphysics'
+per-level table at their edges, against the CPU oracle with the criteria of the moist large steps
 (every case here is two steps of the same state at another size): blocks with
 one column pair or one row beyond a tile, and columns of a few levels, where
 the vertical stencils are clamped at both ends and a block's chunk is cut
@@ -8,6 +8,7 @@ short, for each form of the kernel (with and without turbulence, 2nd- and
 import numpy as np
 import pytest
 
+from test_micro_gpu import MICRO, compare, setup_solver
 from test_moist_gpu import NAMES, check, run_case
 
 pytestmark = pytest.mark.gpu
@@ -23,6 +24,34 @@ def test_moist_scalars_edges(cress, oracle_lib, monkeypatch, nx, ny, nz, tubopt,
     dims, ref, got = run_case(cress, oracle_lib, nx, ny, nz, 2, seed=nx + nz, tubopt=tubopt, advopt=advopt,
                               dtbig=2.0)
     check(dims, ref, got)
+
+
+@pytest.mark.parametrize("nz,dz,dtb,npstp", [
+    (6, 300.0, 2.0, 1), (6, 300.0, 10.0, 2), (6, 300.0, 20.0, 3), (12, 900.0, 90.0, 4), (6, 300.0, 40.0, 5),
+    (17, 700.0, 120.0, 6), (20, 600.0, 120.0, 7), (6, 300.0, 90.0, 10)])
+def test_sedimentation_sweeps(cress, oracle_lib, nz, dz, dtb, npstp):
+    # one to four sub-steps per sweep and more than one sweep, in columns shorter
+    # and longer than a batch of loads; criteria of test_micro_gpu
+    from cress_b200 import cases
+    dims, base, past, fut, _ = cases.micro_case(34, 33, nz, dz, seed=nz)
+    ni, nj, nk = dims
+    ref = {k: v.copy() for k, v in fut.items()}
+    prec_ref = np.zeros((5, 2, nj + 2, ni + 2), np.float32)
+    assert oracle_lib.cloudphy(dims, base, past, ref, prec_ref, dtb, dz) == npstp
+    s = setup_solver(cress, dims, base, dz)
+    for k in MICRO:
+        s.put_field(k, cress.PAST, past[k])
+        s.put_field(k, cress.FUTURE, fut[k])
+    s.put_field("pp", cress.PAST, past["pp"])
+    s.cloudphy(dtb)
+    got = {k: s.get_field(k, cress.FUTURE) for k in MICRO}
+    prec = s.get_precip()
+    s.close()
+    sl = (slice(0, nk - 1), slice(2, nj - 1), slice(2, ni - 1))
+    for k in MICRO:
+        compare(k, got[k][sl], ref[k][sl])
+    psl = (slice(None), slice(None), slice(2, nj - 1), slice(2, ni - 1))
+    assert float(np.abs(prec[psl] - prec_ref[psl]).max()) <= 1e-3 * float(np.abs(prec_ref[psl]).max()) + 1e-30
 
 
 def test_base_state_set_again(cress):
