@@ -103,6 +103,14 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
   return d;
 }
 
+// The same for a K-major tile without swizzle: core matrices of 8 rows x 16
+// bytes (128 contiguous bytes), `lbo` bytes apart along K and `sbo` bytes
+// apart from one 8-row group to the next.
+__device__ __forceinline__ uint64_t core_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(sbo >> 4) << 32 |
+         (uint64_t)1u << 46;
+}
+
 // Instruction descriptor, kind::f16: FP32 accumulator (bits 4..5 = 1),
 // A and B BF16 (bits 7..9, 10..12 = 1), both K-major, N >> 3 in bits
 // 17..22, M >> 4 in bits 24..28.
