@@ -30,9 +30,9 @@
 //
 // Why this shape, and what it measured (us per substep; marching k with a
 // ring of xy tiles before, tile 0 / tile 13 -> this kernel):
-//   64 x 64 x 40    85 -> 14    (16 tiles on 148 SMs, 64 levels in a row)
-//   203 x 131 x 54  125 -> 31
-//   512 x 512 x 64  321 / 289 -> 197: 4.1 TB/s of its 48 bytes per cell, 0.63 of
+//   64 x 64 x 40    85 -> 10    (16 tiles on 148 SMs, 64 levels in a row)
+//   203 x 131 x 54  125 -> 28
+//   512 x 512 x 64  321 / 289 -> 196: 4.1 TB/s of its 48 bytes per cell, 0.63 of
 //                   the measured copy bandwidth, 54.3 bytes per cell of DRAM traffic
 // Marching k, all levels of a column wait for one another and a grid of few
 // tiles leaves SMs idle; a substep also spent about 270 warp instructions per 32
@@ -72,6 +72,31 @@ __device__ __forceinline__ int wrap_row(const HeviRowArgs& a, bool vrow, int r) 
     if (vrow ? r == a.g.nj : r == a.g.nj - 1) return vrow ? 3 : 2;
   }
   return r;
+}
+
+// Programmatic dependent launch: the next substep's blocks are scheduled once
+// every block of this one is in its last row, as they leave their SMs, and set up
+// (barriers, tables) while the rest finish; grid_dependency_wait then waits
+// for all of it, with its stores visible.  Plain launches / triggered at
+// the block's start / in the last row, us per substep: 64 x 64 x 40 14.3 / 11.0 /
+// 10.4, 203 x 131 x 54 31.2 / 29.3 / 28.0, 512 x 512 x 64 196.8 / 202.8 / 196.0 (blocks that wait
+// on a free SM while others work cost more than they save).
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+int launch_dependent(dim3 grid, int threads, size_t bytes, cudaStream_t st, void (*kernel)(P...), const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...) == cudaSuccess ? 0 : CRESS_E_CUDA;
 }
 
 // What only lanes at the domain's x edges store besides their pair, as one
@@ -149,8 +174,9 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
   if (lane0 == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
-    issue(j0 - 1);
   }
+  // Up to here and through the tables below nothing a running kernel writes
+  // is read.
   {
     auto fill = [&](int o, const void* src, int n16) {
       for (int n = threadIdx.x; n < n16; n += blockDim.x)
@@ -164,6 +190,8 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     for (int n = nC * 32 + threadIdx.x; n < kHrMaxWarps * 32; n += blockDim.x)
       reinterpret_cast<uint4*>(smem + Y::oE)[n] = reinterpret_cast<uint4*>(smem + Y::oW)[n] = make_uint4(0, 0, 0, 0);
   }
+  grid_dependency_wait();
+  if (lane0 == 0) issue(j0 - 1);
   __syncthreads();
 
   const int ilast = min(i0 + kHrCols - 1, ni - 2);
@@ -192,7 +220,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
   for (int l = 0; l < L; ++l) {
     const int k = min(k0 + l, nk), ic = min(i, g.px - 2);
     const size_t at = (size_t)(k - 1) * g.plane + (size_t)wrap_row(a, true, j0 - 1) * g.px + ic;
-    vc[l] = F2{__ldg(reinterpret_cast<const unsigned long long*>(a.v + at))};
+    vc[l] = ld2(a.v + at);   // not a read-only load: it must stay below the dependency wait
     tc[l] = vsp[l] = pk[l] = zero;
     if constexpr (!Y::park) held[2 * l] = held[2 * l + 1] = zero;
     else {
@@ -322,6 +350,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
       issue(r + 1);
     }
     if (r <= j0) continue;
+    if (r == j1 + 1) grid_launch_dependents();   // the strip's last solve
     if (nlev < L) {   // levels above nk-2: nothing they hold may enter the sums
 #pragma unroll
       for (int l = 1; l < L; ++l)
@@ -492,8 +521,7 @@ int launch(const HeviRowMaps& m, const HeviRowArgs& a, cudaStream_t st) {
   if (cudaFuncSetAttribute(k_hevi_row<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
     return CRESS_E_CUDA;
   const dim3 grid((unsigned)a.tiles_x, (unsigned)((g.nj - 3 + a.rows - 1) / a.rows));
-  k_hevi_row<L><<<grid, 32 * nC, bytes, st>>>(m, a);
-  return cudaGetLastError() == cudaSuccess ? 0 : CRESS_E_CUDA;
+  return launch_dependent(grid, 32 * nC, bytes, st, k_hevi_row<L>, m, a);
 }
 
 }  // namespace
@@ -591,8 +619,7 @@ static int launch_batch(const HeviRowJob* jobs_d, int njobs, int nblocks, int nC
   const size_t bytes = HrLayout<L>::bytes(nC);
   if (cudaFuncSetAttribute(k_hevi_row_batch<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
     return CRESS_E_CUDA;
-  k_hevi_row_batch<L><<<nblocks, 32 * nC, bytes, st>>>(jobs_d, njobs);
-  return cudaGetLastError() == cudaSuccess ? 0 : CRESS_E_CUDA;
+  return launch_dependent(dim3(nblocks), 32 * nC, bytes, st, k_hevi_row_batch<L>, jobs_d, njobs);
 }
 
 int launch_hevi_row_batch(const HeviRowJob* jobs_d, int njobs, int nblocks, int nk, cudaStream_t st) {
