@@ -177,8 +177,9 @@ __device__ __forceinline__ void fall_sweep(float* fld, const FallSpeed& us, cons
 // What bounds it: memory, one read of the field and of its speed and one
 // write where the field changes, and the latency of a column's march, which
 // the batches of loads hide.  One sub-step per sweep, level by level, with eight
-// speed fields stored and read: 634 us at 512 x 512 x 64; this: 449.
-__global__ void __launch_bounds__(128) k_micro_fall(const MicroArgs a) {
+// speed fields stored and read: 634 us at 512 x 512 x 64; this: 449, and 405 with
+// the registers held to 72 for seven blocks per SM (eight blocks: the same).
+__global__ void __launch_bounds__(128, 7) k_micro_fall(const MicroArgs a) {
   const Grid g = a.g;
   const int nk = g.nk;
   const int i = col_lo(g) + blockIdx.x * blockDim.x + threadIdx.x;

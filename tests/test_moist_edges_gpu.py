@@ -28,7 +28,7 @@ def test_moist_scalars_edges(cress, oracle_lib, monkeypatch, nx, ny, nz, tubopt,
 
 @pytest.mark.parametrize("nz,dz,dtb,npstp", [
     (6, 300.0, 2.0, 1), (6, 300.0, 10.0, 2), (6, 300.0, 20.0, 3), (12, 900.0, 90.0, 4), (6, 300.0, 40.0, 5),
-    (17, 700.0, 120.0, 6), (20, 600.0, 120.0, 7), (6, 300.0, 90.0, 10)])
+    (17, 700.0, 120.0, 6), (20, 600.0, 120.0, 7), (6, 300.0, 70.0, 9)])
 def test_sedimentation_sweeps(cress, oracle_lib, nz, dz, dtb, npstp):
     # one to four sub-steps per sweep and more than one sweep, in columns shorter
     # and longer than a batch of loads; criteria of test_micro_gpu
