@@ -134,10 +134,12 @@ struct HrLayout {
   static constexpr int row = 256;
   static constexpr int sU = 0, sV = row * L, sP = 2 * row * L, sUF = 3 * row * L, sVF = 4 * row * L,
                        sWF = 5 * row * L, sPF = 6 * row * L, sW = 7 * row * L, stage = row * (8 * L + 1);
-  // row r-1's Bs and wr wait in shared memory where they fit beside the
-  // stages: with them in registers the row loop spills
-  static constexpr bool park = L <= 4;
-  static constexpr int parked = park ? 2 * row * L : 0;
+  // row r-1's wr and Bs wait in shared memory where they fit beside the
+  // stages (Bs with up to four levels per chunk): with them in registers the
+  // row loop spills (five levels with wr in registers too: 86.4 us per
+  // substep at 512 x 128 x 80, with it here 80.9)
+  static constexpr bool park = L <= 4;   // Bs too
+  static constexpr int parked = (park ? 2 : 1) * row * L;
   __host__ __device__ static size_t bytes(int nC) { return oS + (size_t)nC * (stage + parked); }
 };
 
@@ -214,7 +216,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
   const F2 zero{0}, dxiv{a.dxiv2}, dyiv{a.dyiv2}, dziv{a.dziv2};
   F2 tc[L], vc[L], vsp[L];                     // row r-1: damped pressure, new v; row r: v
   F2 pk[L];                                    // row r-1: p'
-  F2 held[Y::park ? 1 : 2 * L];                // row r-1: explicit p' tendency but the v part, w right-hand side
+  F2 held[Y::park ? 1 : L];                    // row r-1: explicit p' tendency but the v part (w right-hand side: parked)
   F2 wf0 = zero, t30 = zero, t3l = zero;       // row r-1: what the chunk's first and last level hand on
 #pragma unroll
   for (int l = 0; l < L; ++l) {
@@ -222,11 +224,10 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     const size_t at = (size_t)(k - 1) * g.plane + (size_t)wrap_row(a, true, j0 - 1) * g.px + ic;
     vc[l] = ld2(a.v + at);   // not a read-only load: it must stay below the dependency wait
     tc[l] = vsp[l] = pk[l] = zero;
-    if constexpr (!Y::park) held[2 * l] = held[2 * l + 1] = zero;
-    else {
-      uint64_t* h = reinterpret_cast<uint64_t*>(stage + Y::stage + 2 * Y::row * l + 8 * lane0);
-      h[0] = h[Y::row / 8] = 0;
-    }
+    uint64_t* h = reinterpret_cast<uint64_t*>(stage + Y::stage + Y::row * l + 8 * lane0);
+    h[0] = 0;
+    if constexpr (Y::park) h[Y::row / 8 * L] = 0;
+    else held[l] = zero;
   }
   bool fail = false;
   uint32_t par = 0;
@@ -247,12 +248,17 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     auto D = [&](int l, int n) { return *reinterpret_cast<const double2*>(dt + 16 * (2 * l + n)); };
     auto S = [&](int o, int l) { return F2{*reinterpret_cast<const uint64_t*>(sp + o + Y::row * l)}; };
     auto get = [&](int n) {
-      if constexpr (Y::park) return S(Y::stage, n);
-      else return held[n];
+      if (n & 1) return S(Y::stage, n >> 1);
+      if constexpr (Y::park) return S(Y::stage, L + (n >> 1));
+      else return held[n >> 1];
     };
     auto set = [&](int n, F2 x) {
-      if constexpr (Y::park) *reinterpret_cast<uint64_t*>(const_cast<unsigned char*>(sp) + Y::stage + Y::row * n) = x.b;
-      else held[n] = x;
+      auto put = [&](int m) {
+        *reinterpret_cast<uint64_t*>(const_cast<unsigned char*>(sp) + Y::stage + Y::row * m) = x.b;
+      };
+      if (n & 1) put(n >> 1);
+      else if constexpr (Y::park) put(L + (n >> 1));
+      else held[n >> 1] = x;
     };
     // level l's pair into a new field, and what an edge lane adds
     auto emit = [&](char* p, int l, F2 x, bool on) {
@@ -263,7 +269,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     };
     if (!fail) {   // a warp whose wait gave up stages nothing more and goes on with the barriers
       fail = !__all_sync(0xffffffffu, mbar_wait(bar, par, a.spin));
-      if (!fail) par ^= 1u;
+      if (L <= 4 && !fail) par ^= 1u;
     }
     // Level by level: row r's divergence and faces, then what row r-1 still
     // needed of them (its v part: row r-1 is complete from here on), then the
@@ -349,6 +355,10 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
       fence_proxy_async_smem();
       issue(r + 1);
     }
+    // Where the parity is turned decides what the compiler spills: here for
+    // five levels (73.5 us per substep at 512 x 128 x 80, 80.9 above), above for
+    // four (195.8 at 512 x 512 x 64, 201.0 here).
+    if (L > 4 && !fail) par ^= 1u;
     if (r <= j0) continue;
     if (r == j1 + 1) grid_launch_dependents();   // the strip's last solve
     if (nlev < L) {   // levels above nk-2: nothing they hold may enter the sums
