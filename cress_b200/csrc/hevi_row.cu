@@ -31,8 +31,8 @@
 // Why this shape, and what it measured (us per substep; marching k with a
 // ring of xy tiles before, tile 0 / tile 13 -> this kernel):
 //   64 x 64 x 40    85 -> 10    (16 tiles on 148 SMs, 64 levels in a row)
-//   203 x 131 x 54  125 -> 28
-//   512 x 512 x 64  321 / 289 -> 196: 4.1 TB/s of its 48 bytes per cell, 0.63 of
+//   203 x 131 x 54  125 -> 27
+//   512 x 512 x 64  321 / 289 -> 179: 4.5 TB/s of its 48 bytes per cell, 0.69 of
 //                   the measured copy bandwidth, 54.3 bytes per cell of DRAM traffic
 // Marching k, all levels of a column wait for one another and a grid of few
 // tiles leaves SMs idle; a substep also spent about 270 warp instructions per 32
@@ -40,7 +40,8 @@
 // of a row run at once, the strip length adapts to the grid, and it is about
 // 170 per 32 cells.  It is bound by the latency of its 16 warps per SM: 128 registers each
 // (which is why a row's p' tendency and w right-hand side wait in
-// shared memory, and why per-row addresses are formed again each row), two
+// shared memory, and why the row's addresses, the stage's place and the number of
+// own levels are formed again each row: 195 -> 179 us at 512 x 512 x 64), two
 // barriers per row.  Tried and slower: direct global loads instead of TMA (406 us at
 // 512 x 512 x 64: the row's loads are not in flight during the solve),
 // prefetching a second row into L2 by TMA (235 us), both rows' values in
@@ -154,15 +155,17 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
   const int lane0 = threadIdx.x & 31, c0 = threadIdx.x >> 5, nC = blockDim.x >> 5;
   const int k0 = 2 + c0 * L;
 
-  unsigned char* stage = smem + Y::oS + c0 * (Y::stage + Y::parked);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + Y::oB) + c0;
+  auto stage_of = [&](int c) { return smem + Y::oS + c * (Y::stage + Y::parked); };
+  auto bar_of = [&](int c) { return reinterpret_cast<uint64_t*>(smem + Y::oB) + c; };
   const int i0 = 2 + bx * kHrCols, i = i0 - 2 + 2 * lane0;
   const int j0 = 2 + by * a.rows, j1 = min(j0 + a.rows - 1, nj - 2);
 
   // Lane 0: stage row r (v one row further north) of the warp's levels.
-  auto issue = [&](int r) {
+  auto issue = [&](int r, int c) {
+    unsigned char* stage = stage_of(c);
+    uint64_t* bar = bar_of(c);
     mbar_arrive_expect_tx(bar, Y::stage);
-    const int x = i0 - 2, z = k0 - 1;   // x = 60 bx: a multiple of 4 floats
+    const int x = i0 - 2, z = 1 + c * L;   // x = 60 bx: a multiple of 4 floats
     const int rs = wrap_row(a, false, r);
     tma_load_3d(stage + Y::sU, &m.u, x, rs, z, bar);
     tma_load_3d(stage + Y::sV, &m.v, x, wrap_row(a, true, r + 1), z, bar);
@@ -174,7 +177,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     tma_load_3d(stage + Y::sPF, &m.pf, x, r, z, bar);
   };
   if (lane0 == 0) {
-    mbar_init(bar, 1);
+    mbar_init(bar_of(c0), 1);
     fence_mbar_init();
   }
   // Up to here and through the tables below nothing a running kernel writes
@@ -193,21 +196,16 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
       reinterpret_cast<uint4*>(smem + Y::oE)[n] = reinterpret_cast<uint4*>(smem + Y::oW)[n] = make_uint4(0, 0, 0, 0);
   }
   grid_dependency_wait();
-  if (lane0 == 0) issue(j0 - 1);
+  if (lane0 == 0) issue(j0 - 1, c0);
   __syncthreads();
 
   const int ilast = min(i0 + kHrCols - 1, ni - 2);
   const bool o0 = i >= i0 && i <= ilast, o1 = i + 1 >= i0 && i + 1 <= ilast;
   // the u face at ni-1 belongs to the tile that owns column ni-2
   const bool uf = ilast == ni - 2, u0 = o0 || (uf && i == ni - 1), u1 = o1 || (uf && i + 1 == ni - 1);
-  const int nlev = min(L, nk - 1 - k0);      // own levels k0 .. k0 + nlev - 1 <= nk-2
-  const bool top = k0 + nlev == nk - 1;
   const uint32_t px4 = 4u * (uint32_t)g.px, plane4 = 4u * (uint32_t)g.plane;
   const size_t at0 = 4 * ((size_t)(k0 - 1) * g.plane + (size_t)(j0 - 2) * g.px + i);   // (i, j0-2, k0)
-  char* pu = reinterpret_cast<char*>(a.un) + at0;   // row r of the new u and v, row r-1 of the new w and p'
-  char* pv = reinterpret_cast<char*>(a.vn) + at0;
-  char* pw = reinterpret_cast<char*>(a.wn) + at0 - px4;
-  char* pp = reinterpret_cast<char*>(a.pn) + at0 - px4;
+  size_t at_r = at0;   // row r of the new u and v; row r-1 of the new w and p' is px4 below
   auto lo2 = [](ulonglong2 q) { return F2{q.x}; };
   auto hi2 = [](ulonglong2 q) { return F2{q.y}; };
 
@@ -224,7 +222,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     const size_t at = (size_t)(k - 1) * g.plane + (size_t)wrap_row(a, true, j0 - 1) * g.px + ic;
     vc[l] = ld2(a.v + at);   // not a read-only load: it must stay below the dependency wait
     tc[l] = vsp[l] = pk[l] = zero;
-    uint64_t* h = reinterpret_cast<uint64_t*>(stage + Y::stage + Y::row * l + 8 * lane0);
+    uint64_t* h = reinterpret_cast<uint64_t*>(stage_of(c0) + Y::stage + Y::row * l + 8 * lane0);
     h[0] = 0;
     if constexpr (Y::park) h[Y::row / 8 * L] = 0;
     else held[l] = zero;
@@ -235,12 +233,19 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
   // row j0-1 gives the damped pressure only, row j1+1 that and the v face
   // north of the strip
   for (int r = j0 - 1; r <= j1 + 1; ++r) {
-    pu += px4; pv += px4; pw += px4; pp += px4;
+    at_r += px4;
     // opaque to the compiler, so that what is derived from them is formed
     // where it is used instead of being held in registers across the loop
     int lane = lane0, c = c0;
     uint32_t pl4 = plane4;
-    asm volatile("" : "+r"(lane), "+r"(c), "+r"(pl4));
+    size_t at = at_r;
+    asm volatile("" : "+r"(lane), "+r"(c), "+r"(pl4), "+l"(at));
+    char* const pu = reinterpret_cast<char*>(a.un) + at;
+    char* const pv = reinterpret_cast<char*>(a.vn) + at;
+    char* const pw = reinterpret_cast<char*>(a.wn) + at - px4;
+    char* const pp = reinterpret_cast<char*>(a.pn) + at - px4;
+    const int nlev = min(L, nk - 3 - c * L);      // own levels k0 .. k0 + nlev - 1 <= nk-2
+    const bool top = c * L + nlev == nk - 3;
     const unsigned char* sp = smem + Y::oS + c * (Y::stage + Y::parked) + 8 * lane;
     const unsigned char* ct = smem + Y::oT + c * (16 * kHrVec * L);
     const unsigned char* dt = smem + Y::oD + c * (32 * L);
@@ -268,7 +273,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
       if (e) put_edge(p + (uint64_t)pl4 * l, x, e);
     };
     if (!fail) {   // a warp whose wait gave up stages nothing more and goes on with the barriers
-      fail = !__all_sync(0xffffffffu, mbar_wait(bar, par, a.spin));
+      fail = !__all_sync(0xffffffffu, mbar_wait(bar_of(c), par, a.spin));
       if (L <= 4 && !fail) par ^= 1u;
     }
     // Level by level: row r's divergence and faces, then what row r-1 still
@@ -353,11 +358,11 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     __syncwarp();   // every lane has read the stage
     if (lane == 0 && !fail && r <= j1) {
       fence_proxy_async_smem();
-      issue(r + 1);
+      issue(r + 1, c);
     }
     // Where the parity is turned decides what the compiler spills: here for
-    // five levels (73.5 us per substep at 512 x 128 x 80, 80.9 above), above for
-    // four (195.8 at 512 x 512 x 64, 201.0 here).
+    // five levels (75 us per substep at 512 x 128 x 80, 81 above), above for
+    // four (178.8 at 512 x 512 x 64, 191.5 here).
     if (L > 4 && !fail) par ^= 1u;
     if (r <= j0) continue;
     if (r == j1 + 1) grid_launch_dependents();   // the strip's last solve
@@ -429,7 +434,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
 
   if (fail && lane0 == 0) {   // the copy in flight lands before the block leaves
     atomicExch(a.err, 1);
-    mbar_wait(bar, par);
+    mbar_wait(bar_of(c0), par);
   }
 }
 
