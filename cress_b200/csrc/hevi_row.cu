@@ -191,8 +191,10 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
     fill(Y::oD, a.tab.dbl, 2 * nC * L);
     fill(Y::oN, a.tab.dbl + 2 * nC * L, nC);
     fill(Y::oM, a.tab.dbl + (2 * L + 1) * nC, kHrMaxWarps * kHrMaxWarps);
-    // hand-overs of chunks beyond nC: the folds run in steps of four
-    for (int n = nC * 32 + threadIdx.x; n < kHrMaxWarps * 32; n += blockDim.x)
+    // hand-overs of chunks beyond nC: the folds run in steps of four, and of the
+    // top chunk, which hands nothing on (its levels above nk-2 may hold
+    // NaN)
+    for (int n = (nC - 1) * 32 + threadIdx.x; n < kHrMaxWarps * 32; n += blockDim.x)
       reinterpret_cast<uint4*>(smem + Y::oE)[n] = reinterpret_cast<uint4*>(smem + Y::oW)[n] = make_uint4(0, 0, 0, 0);
   }
   grid_dependency_wait();
@@ -313,6 +315,9 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
             const double cw = (double)(hi2(q6)).x(), dz = (double)dziv.x();
             fa[0] = __dmul_rn(ab.x, __fma_rn(cw, __fma_rn(-dz, (double)t30.x(), (double)wf0.x()) - (double)Gm.x(), (double)wp.x()));
             fb[0] = __dmul_rn(ab.x, __fma_rn(cw, __fma_rn(-dz, (double)t30.y(), (double)wf0.y()) - (double)Gm.y(), (double)wp.y()));
+            // w of level 2 is zero whatever its forcing, which is not the
+            // operator's to read, holds (a factor of zero would pass NaN on)
+            if (c == 0) fa[0] = fb[0] = 0.0;
           } else {        // stepwi.f90:325, gaussel.f90:189-240
             const F2 rw = fma2(hi2(q6), Gpp - Gm, wp);
             fa[l] = __fma_rn(ab.y, fa[l - 1], __dmul_rn(ab.x, (double)rw.x()));
@@ -322,11 +327,10 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
           if (l == L - 1) {   // what this chunk hands to the one above
             const double dz = (double)dziv.x();
             const double2 e = *reinterpret_cast<const double2*>(smem + Y::oN + 16 * c);   // bn, an
-            double xa = fa[l], xb = fb[l];
-            if (nlev < L) xa = xb = 0.0;
-            *reinterpret_cast<double2*>(smem + Y::oE + 16 * (c * 32 + lane)) =
-                make_double2(__fma_rn(e.x, xa, __dmul_rn(e.y, __fma_rn((double)t3l.x(), dz, (double)Gpp.x()))),
-                             __fma_rn(e.x, xb, __dmul_rn(e.y, __fma_rn((double)t3l.y(), dz, (double)Gpp.y()))));
+            if (!top)
+              *reinterpret_cast<double2*>(smem + Y::oE + 16 * (c * 32 + lane)) =
+                  make_double2(__fma_rn(e.x, fa[l], __dmul_rn(e.y, __fma_rn((double)t3l.x(), dz, (double)Gpp.x()))),
+                               __fma_rn(e.x, fb[l], __dmul_rn(e.y, __fma_rn((double)t3l.y(), dz, (double)Gpp.y()))));
           }
           vsp[l] = vs;
         }

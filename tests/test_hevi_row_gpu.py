@@ -7,6 +7,8 @@ the small step's tolerance (test_small_gpu.py)."""
 import numpy as np
 import pytest
 
+import helpers as H
+
 from test_ensemble_gpu import NAMES, member
 from test_small_gpu import check, run_pair
 
@@ -57,3 +59,46 @@ def test_ensemble_of_different_heights_matches_members(cress, oracle_lib):
             s.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("nx,ny,nz", [
+    (61, 9, 26),     # 13 chunks of 2, the last one full
+    (61, 9, 33),     # 11 full chunks of 3
+    (61, 9, 40),     # 14 chunks of 3, one level in the last: it holds nk-1 and nk as well
+    (61, 9, 41),     # two levels in the last: nk-1
+    (61, 9, 49),     # 13 chunks of 4, one level in the last
+    (61, 9, 64),     # 16 full chunks of 4
+    (61, 9, 72),     # 15 chunks of 5, two levels in the last
+    (61, 9, 80),     # 16 full chunks of 5: the tallest column and the most shared memory
+])
+def test_levels_the_operator_does_not_read_may_hold_anything(cress, oracle_lib, nx, ny, nz):
+    """NaN in every level that s_hevi does not read: the forcings below level 2
+    and above nk-2, that of w at level 2 too, and u, v, p', w below the first and
+    above the last level they are used at.  The oracle's interior does not
+    change by a bit, and the kernel's is the same as without them."""
+    ni, nj, nk = H.dims(nx, ny, nz)
+    dz = 18000.0 / nz
+    base = H.base3d(ni, nj, nk, dz, 1)
+    st, frc = H.small_state(ni, nj, nk, nz, base)
+    nst, nfrc = [a.copy() for a in st], [a.copy() for a in frc]
+    for n, a in enumerate(nst):       # index k-1; w is used at nk-1, the others up to nk-2
+        a[0] = np.nan
+        a[nk - 1 if n == 2 else nk - 2:] = np.nan
+    for a in nfrc:
+        a[0] = a[nk - 2:] = np.nan
+    nfrc[2][1] = np.nan
+    cfg = dict(ni=ni, nj=nj, nk=nk, dx=1000.0, dy=1000.0, dz=dz, sthopt=1, divopt=2, buyopt=1, weicoe=0.6)
+    inner = (slice(1, nk - 2), slice(1, nj), slice(1, ni))
+    want = [oracle_lib.small_steps(cfg, base, f, [a.copy() for a in s], 3, 0.5, prec=32, fp64_solve=1)
+            for s, f in ((st, frc), (nst, nfrc))]
+    out = []
+    for s_, f in ((st, frc), (nst, nfrc)):
+        s = cress.Solver(ni, nj, nk, 1000.0, 1000.0, dz, sthopt=1)
+        s.set_base3d(base)
+        out.append(s.smalldrv(3, 0.5, *s_, *f))
+        s.close()
+    for name, a, b, c, d in zip(("u", "v", "w", "pp"), *want, *out):
+        assert np.array_equal(a[inner], b[inner]), name
+        assert np.isfinite(d[inner]).all(), name
+        assert np.array_equal(c[inner], d[inner]), name
+    check(ni, nj, nk, want[0], out[0], 3)
