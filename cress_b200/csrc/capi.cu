@@ -293,14 +293,32 @@ int Ctx::wait_async(int keep) {
   return CRESS_OK;
 }
 
+// The scalars of one small step of length dts.
+HeviArgs Ctx::small_scalars(float dts) const {
+  HeviArgs a{};
+  a.g = g;
+  a.col = col_d;
+  a.err = err_d;
+  a.dts = dts;
+  a.dxiv = 1.f / cfg.dx; a.dyiv = 1.f / cfg.dy; a.dziv = 1.f / cfg.dz;
+  a.divch = kDivndc / dts * cfg.dx * cfg.dy;     // pgrad.f90:253
+  a.divcv = kDivndc / dts * cfg.dz * cfg.dz;     // pgrad.f90:254
+  a.weicoe = cfg.weicoe;
+  a.dtdzw = dts * a.dziv * cfg.weicoe;           // pgradiv.f90:135
+  a.dtw = dts * cfg.weicoe;                      // buoywsi.f90:153
+  a.g05 = .5f * kG;
+  a.g05n = -.5f * kG;
+  a.divopt = cfg.divopt; a.buyopt = cfg.buyopt; a.sthopt = cfg.sthopt; a.bbc = cfg.bbc;
+  a.spin = spin_limit;
+  return a;
+}
+
 // Elimination factors of the w system for one dts (w_system_factors,
-// wsystem.h: s_stepwi's coefficients and s_gaussel's factors), uploaded
-// once per distinct dts.
-int Ctx::thomas_for(float dts, const HeviArgs& a, const ThomasSet** out) {
-  uint32_t key;
-  std::memcpy(&key, &dts, 4);
-  auto it = thomas.find(key);
-  if (it != thomas.end()) { *out = &it->second; return CRESS_OK; }
+// wsystem.h: s_stepwi's coefficients and s_gaussel's factors) and the level
+// tables formed with them, as one block; off: the parts' offsets in it (rr,
+// aa, cp, the HeviLevel rows, the row kernel's two tables), which depend on
+// the grid alone.
+std::vector<unsigned char> Ctx::thomas_block(float dts, size_t (&off)[6]) const {
   const int nk = g.nk;
   std::vector<float> rr(nk + 2), work(4 * (size_t)(nk + 2));
   std::vector<double> cp(nk + 2), aa(nk + 2);
@@ -311,8 +329,7 @@ int Ctx::thomas_for(float dts, const HeviArgs& a, const ThomasSet** out) {
   std::vector<float> rlev;
   std::vector<double> rdbl;
   if (hevi_row_supported(g))
-    hevi_row_table(col_h.data(), nk, rr.data(), aa.data(), cp.data(), a, &rlev, &rdbl);
-  // one block, one copy: a new step length is set up inside a step's call
+    hevi_row_table(col_h.data(), nk, rr.data(), aa.data(), cp.data(), small_scalars(dts), &rlev, &rdbl);
   std::vector<unsigned char> buf;
   auto add = [&](const void* p, size_t n) {
     const size_t at = (buf.size() + 255) / 256 * 256;
@@ -320,27 +337,39 @@ int Ctx::thomas_for(float dts, const HeviArgs& a, const ThomasSet** out) {
     if (n) std::memcpy(buf.data() + at, p, n);
     return at;
   };
-  const size_t o_rr = add(rr.data(), sizeof(float) * rr.size()), o_aa = add(aa.data(), sizeof(double) * aa.size()),
-               o_cp = add(cp.data(), sizeof(double) * cp.size()),
-               o_l3 = add(rows.data(), sizeof(HeviLevel) * rows.size()),
-               o_rl = add(rlev.data(), sizeof(float) * rlev.size()),
-               o_rd = add(rdbl.data(), sizeof(double) * rdbl.size());
-  unsigned char* d = nullptr;
+  off[0] = add(rr.data(), sizeof(float) * rr.size());
+  off[1] = add(aa.data(), sizeof(double) * aa.size());
+  off[2] = add(cp.data(), sizeof(double) * cp.size());
+  off[3] = add(rows.data(), sizeof(HeviLevel) * rows.size());
+  off[4] = add(rlev.data(), sizeof(float) * rlev.size());
+  off[5] = add(rdbl.data(), sizeof(double) * rdbl.size());
+  return buf;
+}
+
+// The set of one dts, uploaded once per distinct dts.
+int Ctx::thomas_for(float dts, const ThomasSet** out) {
+  uint32_t key;
+  std::memcpy(&key, &dts, 4);
+  auto it = thomas.find(key);
+  if (it != thomas.end()) { *out = &it->second; return CRESS_OK; }
+  size_t off[6];
+  const std::vector<unsigned char> buf = thomas_block(dts, off);
+  ThomasSet t;
   int rc;
-  if ((rc = cuda_check(cudaMalloc(&d, buf.size()), "cudaMalloc (tridiagonal factors)"))) return rc;
-  owned.push_back(d);
+  if ((rc = cuda_check(cudaMalloc(&t.block, buf.size()), "cudaMalloc (tridiagonal factors)"))) return rc;
+  owned.push_back(t.block);
   // the host buffer is freed on return: make the copy complete
-  if ((rc = cuda_check(cudaMemcpyAsync(d, buf.data(), buf.size(), cudaMemcpyHostToDevice, stream), "copy factors")) ||
+  if ((rc = cuda_check(cudaMemcpyAsync(t.block, buf.data(), buf.size(), cudaMemcpyHostToDevice, stream),
+                       "copy factors")) ||
       (rc = cuda_check(cudaStreamSynchronize(stream), "sync after factor upload")))
     return rc;
-  ThomasSet t;
-  t.rr = reinterpret_cast<float*>(d + o_rr);
-  t.aa = reinterpret_cast<double*>(d + o_aa);
-  t.cp = reinterpret_cast<double*>(d + o_cp);
-  t.lvl3 = reinterpret_cast<HeviLevel*>(d + o_l3);
-  if (!rlev.empty()) {
-    t.row_lev = reinterpret_cast<float4*>(d + o_rl);
-    t.row_dbl = reinterpret_cast<double2*>(d + o_rd);
+  t.rr = reinterpret_cast<float*>(t.block + off[0]);
+  t.aa = reinterpret_cast<double*>(t.block + off[1]);
+  t.cp = reinterpret_cast<double*>(t.block + off[2]);
+  t.lvl3 = reinterpret_cast<HeviLevel*>(t.block + off[3]);
+  if (hevi_row_supported(g)) {
+    t.row_lev = reinterpret_cast<float4*>(t.block + off[4]);
+    t.row_dbl = reinterpret_cast<double2*>(t.block + off[5]);
   }
   auto res = thomas.emplace(key, t);
   *out = &res.first->second;
@@ -394,16 +423,21 @@ int Ctx::tmap(const float* buf, int rows, CUtensorMap* out, int levels) {
 // (forcing.cuh: columns, reciprocals, derived quotients), formed on the
 // host with the same IEEE operations the device would use and kept per
 // distinct dtb2 (the half first step and the regular one).
+std::vector<float> Ctx::level_rows(float dtb2) const {
+  const int nc = g.nk + 1;
+  auto B = [&](int f, int kk) { return col_h[(size_t)f * nc + kk]; };
+  std::vector<float> t((size_t)nc * kLevelStride, 0.f);
+  for (int kk = 0; kk < nc; ++kk)
+    for (int f = 0; f < D_NFIELDS; ++f) t[(size_t)kk * kLevelStride + f] = level_value(f, kk, B, dtb2);
+  return t;
+}
+
 int Ctx::level_table(float dtb2, const float** out) {
   uint32_t key;
   std::memcpy(&key, &dtb2, 4);
   auto it = level_tables.find(key);
   if (it != level_tables.end()) { *out = it->second; return CRESS_OK; }
-  const int nk = g.nk, nc = nk + 1;
-  auto B = [&](int f, int kk) { return col_h[(size_t)f * nc + kk]; };
-  std::vector<float> t((size_t)nc * kLevelStride, 0.f);
-  for (int kk = 0; kk < nc; ++kk)
-    for (int f = 0; f < D_NFIELDS; ++f) t[(size_t)kk * kLevelStride + f] = level_value(f, kk, B, dtb2);
+  const std::vector<float> t = level_rows(dtb2);
   float* d = nullptr;
   int rc;
   if ((rc = cuda_check(cudaMalloc(&d, sizeof(float) * t.size()), "cudaMalloc level table"))) return rc;
@@ -414,6 +448,42 @@ int Ctx::level_table(float dtb2, const float** out) {
     return rc;
   level_tables.emplace(key, d);
   *out = d;
+  return CRESS_OK;
+}
+
+// After a change of the base columns (col_h, whose copy to col_d is queued):
+// every table formed from them is formed again in place, for each step length
+// kept, and what was captured goes, since captured steps hold values of the
+// old base state (an ensemble sees the new generation and drops its own).
+int Ctx::base_changed() {
+  ++generation;
+  cudaStreamSynchronize(stream);
+  free_graphs();
+  int rc;
+  // one table at a time, complete before its host form is freed
+  auto put = [&](void* d, const void* h, size_t n) {
+    const int r = cuda_check(cudaMemcpyAsync(d, h, n, cudaMemcpyHostToDevice, stream), "copy base tables");
+    return r ? r : cuda_check(cudaStreamSynchronize(stream), "sync base tables");
+  };
+  auto length = [](uint32_t key) {
+    float v;
+    std::memcpy(&v, &key, 4);
+    return v;
+  };
+  for (auto& kv : thomas) {
+    size_t off[6];
+    const std::vector<unsigned char> b = thomas_block(length(kv.first), off);
+    if ((rc = put(kv.second.block, b.data(), b.size()))) return rc;
+  }
+  for (auto& kv : level_tables) {
+    const std::vector<float> t = level_rows(length(kv.first));
+    if ((rc = put(kv.second, t.data(), sizeof(float) * t.size()))) return rc;
+  }
+  for (auto& kv : micro_tables) {
+    std::vector<MicroLevel> t(g.nk + 1);
+    micro_levels(col_h.data(), g.nk, length(kv.first), t.data());
+    if ((rc = put(kv.second, t.data(), sizeof(MicroLevel) * t.size()))) return rc;
+  }
   return CRESS_OK;
 }
 
@@ -446,23 +516,7 @@ int Ctx::row_ends_future() {
 }
 
 // The microphysics' level table of one step length (micro.cuh), kept per
-// distinct one like the large step's; a new base state rewrites the tables
-// in place (captured steps read them).
-int Ctx::refresh_micro_tables() {
-  std::vector<MicroLevel> t(g.nk + 1);
-  for (auto& kv : micro_tables) {
-    float dtb;
-    std::memcpy(&dtb, &kv.first, 4);
-    micro_levels(col_h.data(), g.nk, dtb, t.data());
-    int rc;
-    if ((rc = cuda_check(cudaMemcpyAsync(kv.second, t.data(), sizeof(MicroLevel) * t.size(), cudaMemcpyHostToDevice,
-                                         stream), "copy microphysics table")) ||
-        (rc = cuda_check(cudaStreamSynchronize(stream), "sync microphysics table")))
-      return rc;
-  }
-  return CRESS_OK;
-}
-
+// distinct one like the large step's.
 int Ctx::micro_table(float dtb, const MicroLevel** out) {
   uint32_t key;
   std::memcpy(&key, &dtb, 4);
@@ -495,27 +549,13 @@ int Ctx::small_steps(int nsstp, float dts, std::vector<HeviJob>* jobs, std::vect
   const bool heve = cfg.impopt == 0;
   const ThomasSet* th = nullptr;
   int rc;
-  HeviArgs a{};
-  a.g = g;
-  a.col = col_d;
+  HeviArgs a = small_scalars(dts);
   if (level_tables.empty()) {   // any level table serves: the small step reads only its columns
     const float* t = nullptr;
     if ((rc = level_table(0.f, &t))) return rc;
   }
   a.lvl = level_tables.begin()->second;
-  a.err = err_d;
-  a.dts = dts;
-  a.dxiv = 1.f / cfg.dx; a.dyiv = 1.f / cfg.dy; a.dziv = 1.f / cfg.dz;
-  a.divch = kDivndc / dts * cfg.dx * cfg.dy;     // pgrad.f90:253
-  a.divcv = kDivndc / dts * cfg.dz * cfg.dz;     // pgrad.f90:254
-  a.weicoe = cfg.weicoe;
-  a.dtdzw = dts * a.dziv * cfg.weicoe;           // pgradiv.f90:135
-  a.dtw = dts * cfg.weicoe;                      // buoywsi.f90:153
-  a.g05 = .5f * kG;
-  a.g05n = -.5f * kG;
-  a.divopt = cfg.divopt; a.buyopt = cfg.buyopt; a.sthopt = cfg.sthopt; a.bbc = cfg.bbc;
-  a.spin = spin_limit;
-  if (!heve && (rc = thomas_for(dts, a, &th))) return rc;
+  if (!heve && (rc = thomas_for(dts, &th))) return rc;
   if (th) { a.thom_rr = th->rr; a.thom_aa = th->aa; a.thom_cp = th->cp; a.lvl3 = th->lvl3; }
   const bool row = row_kernel() && !jobs;
   if (rjobs && !row) return set_error(CRESS_E_UNSUPPORTED, "the row kernel does not run on this grid");
@@ -1079,6 +1119,7 @@ struct Ensemble {
   };
   std::map<std::string, Rec> grec;
   std::map<std::string, int> gseen;
+  std::vector<unsigned> generations;  // the members' when the graphs were captured
   void free_graphs() {
     for (auto& kv : grec) {
       if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
@@ -1326,6 +1367,14 @@ int Ensemble::step(long long ctime, float dtb, int nsstp, float dts) {
   bool sampling = false;
   for (Ctx* c : members) sampling |= c->sampler != nullptr;
   if (!graphs || sampling) return eager();
+  // a member's base state changed: what was captured holds the old one
+  std::vector<unsigned> gens;
+  for (Ctx* c : members) gens.push_back(c->generation);
+  if (gens != generations) {
+    cudaStreamSynchronize(stream);
+    free_graphs();
+    generations = gens;
+  }
   std::string key;
   for (Ctx* c : members) {
     const std::vector<float*> ps = c->pointer_state();
@@ -1552,7 +1601,8 @@ int cress_set_spin_limit(cress_ctx* ctx, int probes) {
   Ctx* c = reinterpret_cast<Ctx*>(ctx);
   if (!c) return set_error(CRESS_E_ARG, "null context");
   c->spin_limit = probes < 0 ? kSpinLimit : (uint32_t)probes;
-  c->free_graphs();   // captured steps carry the old limit
+  ++c->generation;    // captured steps carry the old limit
+  c->free_graphs();
   return CRESS_OK;
 }
 
@@ -1581,11 +1631,8 @@ int cress_set_base3d(cress_ctx* ctx, const float* const* b3) {
                                       cudaMemcpyHostToDevice, c->stream),
                       "copy base columns");
   if (rc) return rc;
-  rc = cuda_check(cudaStreamSynchronize(c->stream), "sync base columns");
-  if (rc) return rc;
-  c->thomas.clear();
   c->base_set = true;
-  return c->refresh_micro_tables();
+  return c->base_changed();
 }
 
 int cress_put_field(cress_ctx* ctx, int field, int level, const float* host) {
@@ -1707,10 +1754,8 @@ int cress_set_base_large(cress_ctx* ctx, const float* ubr, const float* vbr, con
                                       cudaMemcpyHostToDevice, c->stream),
                       "copy large-step columns");
   if (rc) return rc;
-  rc = cuda_check(cudaStreamSynchronize(c->stream), "sync large-step columns");
-  if (rc) return rc;
   c->large_set = true;
-  return CRESS_OK;
+  return c->base_changed();
 }
 
 int cress_set_base_moist(cress_ctx* ctx, const float* pbr, const float* qvbr) {
@@ -1735,9 +1780,8 @@ int cress_set_base_moist(cress_ctx* ctx, const float* pbr, const float* qvbr) {
   int rc = cuda_check(cudaMemcpyAsync(c->col_d, c->col_h.data(), sizeof(float) * c->col_h.size(),
                                       cudaMemcpyHostToDevice, c->stream), "copy moist columns");
   if (rc) return rc;
-  if ((rc = cuda_check(cudaStreamSynchronize(c->stream), "sync moist columns"))) return rc;
   c->moist_set = true;
-  return c->refresh_micro_tables();
+  return c->base_changed();
 }
 
 int cress_cloudphy(cress_ctx* ctx, float dtb, float thresq) {

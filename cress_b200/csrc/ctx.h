@@ -20,6 +20,7 @@ int cuda_check(cudaError_t e, const char* what);
 
 // Elimination factors of the w system for one dts (device arrays indexed by k).
 struct ThomasSet {
+  unsigned char* block = nullptr;   // holds all of them
   float* rr = nullptr;
   double* aa = nullptr;
   double* cp = nullptr;
@@ -83,12 +84,17 @@ struct Ctx {
   // grown as needed
   void* rec_d = nullptr;
   long long rec_bytes = 0;
-  int thomas_for(float dts, const HeviArgs& a, const ThomasSet** out);   // a: the step's scalars
+  HeviArgs small_scalars(float dts) const;
+  std::vector<unsigned char> thomas_block(float dts, size_t (&off)[6]) const;
+  int thomas_for(float dts, const ThomasSet** out);
   std::map<uint32_t, float*> level_tables;   // level table per 2*dtb (bits)
+  std::vector<float> level_rows(float dtb2) const;
   int level_table(float dtb2, const float** out);
   std::map<uint32_t, MicroLevel*> micro_tables;   // microphysics level table per step (bits)
   int micro_table(float dtb, const MicroLevel** out);
-  int refresh_micro_tables();
+  // counts changes of what captured steps hold by value (base state, wait limit)
+  unsigned generation = 0;
+  int base_changed();
   // whether the HE-VI substeps run the row-marching kernel
   bool row_kernel() const;
   int small_steps(int nsstp, float dts);
