@@ -451,6 +451,19 @@ int Ctx::level_table(float dtb2, const float** out) {
   return CRESS_OK;
 }
 
+// Make cols, which have passed their checks, the base columns; *set: whether
+// they were given before.  Nothing is done where they are the ones in use
+// (and nothing `other` changed with them).
+int Ctx::use_columns(const std::vector<float>& cols, bool* set, bool other) {
+  if (*set && !other && std::memcmp(cols.data(), col_h.data(), sizeof(float) * cols.size()) == 0) return CRESS_OK;
+  col_h = cols;
+  const int rc = cuda_check(cudaMemcpyAsync(col_d, col_h.data(), sizeof(float) * col_h.size(), cudaMemcpyHostToDevice,
+                                            stream), "copy base columns");
+  if (rc) return rc;
+  *set = true;
+  return base_changed();
+}
+
 // After a change of the base columns (col_h, whose copy to col_d is queued):
 // every table formed from them is formed again in place, for each step length
 // kept, and what was captured goes, since captured steps hold values of the
@@ -1623,16 +1636,13 @@ int cress_set_base3d(cress_ctx* ctx, const float* const* b3) {
   const int ni = c->cfg.ni, nj = c->cfg.nj, nk = c->cfg.nk;
   // The columns are taken at the domain centre; every point the small step
   // reads (i in 1..ni, j in 1..nj) must carry the same value.
-  const NonUniform bad = base_columns(b3, ni, nj, nk, c->col_h.data());
+  // They are taken over together, once all have passed.
+  std::vector<float> cols = c->col_h;
+  const NonUniform bad = base_columns(b3, ni, nj, nk, cols.data());
   if (bad.n >= 0)
     return set_error(CRESS_E_NONUNIFORM, "base array %d varies horizontally at (%d,%d,%d): %g vs %g", bad.n,
                      bad.i, bad.j, bad.k, (double)bad.x, (double)bad.v);
-  int rc = cuda_check(cudaMemcpyAsync(c->col_d, c->col_h.data(), sizeof(float) * c->col_h.size(),
-                                      cudaMemcpyHostToDevice, c->stream),
-                      "copy base columns");
-  if (rc) return rc;
-  c->base_set = true;
-  return c->base_changed();
+  return c->use_columns(cols, &c->base_set);
 }
 
 int cress_put_field(cress_ctx* ctx, int field, int level, const float* host) {
@@ -1739,23 +1749,20 @@ int cress_set_base_large(cress_ctx* ctx, const float* ubr, const float* vbr, con
   const float* src[3] = {ubr, vbr, rbct};
   const int dst[3] = {C_UBR, C_VBR, C_RBCT};
   const int ic = ni / 2, jc = nj / 2;
+  std::vector<float> cols = c->col_h;
   for (int n = 0; n < 3; ++n)
     for (int k = 1; k <= nk; ++k) {
       const float v = at(src[n], ic, jc, k);
-      c->col_h[(size_t)dst[n] * (nk + 1) + k] = v;
+      cols[(size_t)dst[n] * (nk + 1) + k] = v;
       for (int j = 1; j <= nj - 1; ++j)
         for (int i = 1; i <= ni - 1; ++i)
           if (at(src[n], i, j, k) != v)
             return set_error(CRESS_E_NONUNIFORM, "large-step base array %d varies horizontally at (%d,%d,%d)",
                              n, i, j, k);
     }
+  const bool other = c->ksp0 != ksp0;
   c->ksp0 = ksp0;
-  int rc = cuda_check(cudaMemcpyAsync(c->col_d, c->col_h.data(), sizeof(float) * c->col_h.size(),
-                                      cudaMemcpyHostToDevice, c->stream),
-                      "copy large-step columns");
-  if (rc) return rc;
-  c->large_set = true;
-  return c->base_changed();
+  return c->use_columns(cols, &c->large_set, other);
 }
 
 int cress_set_base_moist(cress_ctx* ctx, const float* pbr, const float* qvbr) {
@@ -1768,20 +1775,17 @@ int cress_set_base_moist(cress_ctx* ctx, const float* pbr, const float* qvbr) {
   };
   const float* src[2] = {pbr, qvbr};
   const int dst[2] = {C_PBR, C_QVBR};
+  std::vector<float> cols = c->col_h;
   for (int n = 0; n < 2; ++n)
     for (int k = 1; k <= nk; ++k) {
       const float v = at(src[n], ni / 2, nj / 2, k);
-      c->col_h[(size_t)dst[n] * (nk + 1) + k] = v;
+      cols[(size_t)dst[n] * (nk + 1) + k] = v;
       for (int j = 1; j <= nj - 1; ++j)
         for (int i = 1; i <= ni - 1; ++i)
           if (at(src[n], i, j, k) != v)
             return set_error(CRESS_E_NONUNIFORM, "moist base array %d varies horizontally at (%d,%d,%d)", n, i, j, k);
     }
-  int rc = cuda_check(cudaMemcpyAsync(c->col_d, c->col_h.data(), sizeof(float) * c->col_h.size(),
-                                      cudaMemcpyHostToDevice, c->stream), "copy moist columns");
-  if (rc) return rc;
-  c->moist_set = true;
-  return c->base_changed();
+  return c->use_columns(cols, &c->moist_set);
 }
 
 int cress_cloudphy(cress_ctx* ctx, float dtb, float thresq) {

@@ -94,6 +94,7 @@ struct Ctx {
   int micro_table(float dtb, const MicroLevel** out);
   // counts changes of what captured steps hold by value (base state, wait limit)
   unsigned generation = 0;
+  int use_columns(const std::vector<float>& cols, bool* set, bool other = false);
   int base_changed();
   // whether the HE-VI substeps run the row-marching kernel
   bool row_kernel() const;

@@ -132,3 +132,32 @@ def test_ensemble_follows(cress, oracle_lib):
         steps(f, 9, 9)
         same(levels(f, cress), g)
         f.close()
+
+
+@pytest.mark.parametrize("what", ["3d", "large", "moist"])
+def test_refused_base_changes_nothing(cress, oracle_lib, what):
+    """A base state with one value out of line in its last array is refused,
+    and a host that goes on gets the one in use: also for step lengths it
+    uses for the first time, whose tables are formed after the refusal."""
+    case = case_of(*SIZE, 8)
+    damp, _ = damping(oracle_lib, case, what)
+    bad = other(case["base"], what)
+    last = {"3d": "rcsq", "large": "vbr", "moist": "qvbr"}[what]
+    bad[last] = bad[last].copy()
+    at = (SIZE[2] - 2, 9, 11)
+    bad[last][at] += np.float32(.01) * abs(bad[last][at]) + np.float32(1e-3)
+    out = []
+    for refuse in (False, True):
+        s = solver(cress, case, case["base"], damp)
+        put(s, cress, case)
+        steps(s, 0, 1)
+        if refuse:
+            with pytest.raises(cress.CressError) as e:
+                set_base(s, case, bad, damp, what)
+            assert e.value.code == 4                 # CRESS_E_NONUNIFORM
+        steps(s, 1, 2)
+        out.append(levels(s, cress))
+        s.cloudphy(7.0)
+        out[-1].append([s.get_field(n, cress.FUTURE) for n in NAMES])
+        s.close()
+    same(*out)
