@@ -12,7 +12,7 @@
 // column blocks (128 output rows x 64 K, BF16) and W4 through a 2-stage TMA
 // ring; warp 9 (one lane) issues the MMAs (N = 128 per block into one half
 // of the 256 accumulator columns).  Two blocks share an SM.  Per tile: x_full (features
-// written), then per layer acc_full (accumulator ready) and h_full (next
+// written; one barrier for even, one for odd tiles), then per layer acc_full (accumulator ready) and h_full (next
 // activations written; after layer 4: accumulator read).  Every mbarrier wait is
 // bounded; on expiry the kernel records CRESS_E_TIMEOUT, stops all roles, drains its
 // copies and MMAs (bounded) and frees tensor memory.
@@ -160,18 +160,23 @@ __device__ __forceinline__ void fused_epilogue(const MicroArgs& a, const FusedAr
   auto features = [&](long long t, int par) {
     fused_features(a, p, t * kFusedTile + row, row, X, envs + par * kFusedTile);
     fence_proxy_async_smem();
-    mbar_arrive(x_full);
+    mbar_arrive(x_full + par);
   };
-  int pha = 0, par = 0;   // par: parity of the tile's number in this block
+  int pha = 0, par = 0, phx = 0;   // par: parity of the tile's number in this block; phx: its x_full's phase
   bool env = false, pending = false;
   float ys[kMlpOut];
   long long t = blockIdx.x;
   if (half == 0 && t < ntiles) features(t, 0);
-  for (; t < ntiles; t += gridDim.x, par ^= 1) {
+  for (; t < ntiles; t += gridDim.x, phx ^= par, par ^= 1) {
     if (__any_sync(full, *vfail != 0)) break;
     bool ok = true, env_t = false;
-    if (half == 1) {   // the features' writes, by the phase their arrival completes
-      ok = __all_sync(full, mbar_wait_sleep(x_full, par));
+    // The features' writes, by the phase their arrival completes.  The tiles
+    // alternate between two barriers: with one, warps 0-3 could complete the next
+    // tile's phase before these warps looked at this one's, and its parity would
+    // never come again.  The next phase of the same barrier is two tiles on, and
+    // waits for these warps' arrival on h_full in between.
+    if (half == 1) {
+      ok = __all_sync(full, mbar_wait_sleep(x_full + par, phx));
       env_t = envs[par * kFusedTile + row] != 0;
     }
     for (int l = 0; l < 3 && ok; ++l) {
@@ -241,7 +246,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
   unsigned char* X = WS + 2 * kWStage;            // features of one tile
   float* bias = reinterpret_cast<float*>(X + kXBytes);   // b1, b2, b3 (256 each), b4 (64)
   __shared__ unsigned char envs[2 * kFusedTile];  // inside the envelope, two tiles
-  __shared__ __align__(8) uint64_t x_full, h_full, acc_full, w_full[2], w_empty[2], mma_done;
+  __shared__ __align__(8) uint64_t x_full[2], h_full, acc_full, w_full[2], w_empty[2], mma_done;
   __shared__ uint32_t tmem_slot;
   __shared__ int fail;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -254,7 +259,8 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
     bias[n] = __ldg(p.params + off + (n - l * kMlpH));
   }
   if (threadIdx.x == 0) {
-    mbar_init(&x_full, 128);
+    mbar_init(&x_full[0], 128);
+    mbar_init(&x_full[1], 128);
     mbar_init(&h_full, 256);
     mbar_init(&acc_full, 1);
     mbar_init(&mma_done, 1);
@@ -298,11 +304,10 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
       const uint32_t id128 = idesc_bf16_f32(128, 128), id64 = idesc_bf16_f32(128, 64);
       const uint32_t hs = smem_u32(H), ws = smem_u32(WS);
       const uint64_t xdesc = core_desc(smem_u32(X), 128, 256);
-      int cnt = 0, phx = 0, phh = 0;
+      int cnt = 0, par = 0, phx = 0, phh = 0;   // par, phx: as in fused_epilogue
       bool ok = true;
-      for (long long t = blockIdx.x; ok && t < ntiles; t += gridDim.x) {
-        if (*vfail || !mbar_wait_sleep(&x_full, phx)) { ok = false; break; }
-        phx ^= 1;
+      for (long long t = blockIdx.x; ok && t < ntiles; t += gridDim.x, phx ^= par, par ^= 1) {
+        if (*vfail || !mbar_wait_sleep(&x_full[par], phx)) { ok = false; break; }
         for (int l = 0; l < 4 && ok; ++l) {
           if (l > 0 || t != blockIdx.x) {   // also layer 4's accumulator was read
             if (*vfail || !mbar_wait_sleep(&h_full, phh)) { ok = false; break; }
@@ -331,7 +336,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
       mbar_wait(&mma_done, 0);
     }
   } else {
-    fused_epilogue(a, p, H, X, envs, bias, tmem, &x_full, &h_full, &acc_full, vfail, ntiles);
+    fused_epilogue(a, p, H, X, envs, bias, tmem, x_full, &h_full, &acc_full, vfail, ntiles);
   }
   tc_fence_before();
   __syncthreads();

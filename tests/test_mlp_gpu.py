@@ -101,9 +101,9 @@ def test_training_reduces_loss(cress):
     assert last < 0.2 * first, (first, last)
 
 
-def _moist_solver(cress, oracle_lib, seed):
+def _moist_solver(cress, oracle_lib, seed, size=(40, 32, 24)):
     from cress_b200 import cases
-    case = cases.supercell_case(40, 32, 24, 1000.0, ztop=8000.0, seed=seed, cloud=True,
+    case = cases.supercell_case(*size, 1000.0, ztop=8000.0, seed=seed, cloud=True,
                                 rad=(6000.0, 6000.0, 1400.0))
     ni, nj, nk = case["dims"]
     zph = case["zph"]
@@ -173,9 +173,20 @@ def test_fused_inference_matches_chunked(cress, oracle_lib):
     """The fused persistent kernel (features, four tensor-core GEMMs with the
     activations in shared memory, application) gives the same large steps
     as the chunked path through separate GEMM launches."""
+    _fused_against_chunked(cress, oracle_lib, (40, 32, 24))
+
+
+def test_fused_inference_over_many_tiles(cress, oracle_lib):
+    """The same where a block runs five or six tiles one after the other, each
+    one's features and application beside its neighbours' layers, and the last
+    tile is not full (above, no block has more than one tile)."""
+    _fused_against_chunked(cress, oracle_lib, (71, 63, 46))
+
+
+def _fused_against_chunked(cress, oracle_lib, size):
     m = cress.Mlp(seed=8)
     m.reserve(200000)
-    s, dims = _moist_solver(cress, oracle_lib, 4)
+    s, dims = _moist_solver(cress, oracle_lib, 4, size)
     s.set_tuple_sampling(m, stride=1, keep_zero=0.2, seed=2)
     s.large_step(0, 2.5, 10, 0.5)
     s.large_step(5000, 5.0, 10, 1.0)
@@ -185,7 +196,7 @@ def test_fused_inference_matches_chunked(cress, oracle_lib):
     m.train(200, batch=4096, lr=1e-3, seed=1)
     out = []
     for chunk in (16384, 0):
-        s, dims = _moist_solver(cress, oracle_lib, 4)
+        s, dims = _moist_solver(cress, oracle_lib, 4, size)
         s.set_learned_micro(m, chunk=chunk, resid_tol=0.5)
         s.large_step(0, 2.5, 10, 0.5)
         s.large_step(5000, 5.0, 10, 1.0)
