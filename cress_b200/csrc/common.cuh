@@ -13,6 +13,19 @@
 
 namespace cress {
 
+// SMs of the current device, asked for once per device and thread.
+inline int sm_count() {
+  thread_local int known[16] = {};
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 16 && known[dev]) return known[dev];
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) {
+    cudaGetLastError();   // not the next launch's error
+    return 148;           // a B200's
+  }
+  if (dev >= 0 && dev < 16) known[dev] = n;
+  return n;
+}
+
 struct Grid {
   int ni, nj, nk;   // reference dims (ni = nx+3, nj = ny+3, nk = nz+3)
   int px, py;       // x pitch (floats) and y extent of one plane

@@ -2,7 +2,7 @@
 // periodic halo planes): internal interface.
 #pragma once
 #include <map>
-#include <utility>
+#include <tuple>
 #include <cuda_runtime.h>
 #include "common.cuh"
 #include "hevi.cuh"
@@ -215,18 +215,20 @@ inline int level_chunk(int n, long long tiles, long long resident) {
 }
 
 // Blocks of a kernel the GPU holds at once (threads and bytes of shared
-// memory per block), asked for once per thread.
+// memory per block), asked for once per device and thread.
 template <class K>
 inline long long resident_blocks(K kern, int threads, size_t bytes) {
-  thread_local std::map<std::pair<const void*, size_t>, long long> known;
-  long long& n = known[{reinterpret_cast<const void*>(kern), bytes}];
-  if (!n) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, bytes) != cudaSuccess || per_sm < 1)
-      per_sm = 1;
-    n = 148LL * per_sm;
+  thread_local std::map<std::tuple<int, const void*, int, size_t>, long long> known;
+  int dev = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  const auto key = std::make_tuple(dev, reinterpret_cast<const void*>(kern), threads, bytes);
+  const auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, bytes) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();   // not the launch's error; the next call asks again
+    return sm_count();
   }
-  return n;
+  return known[key] = (long long)sm_count() * per_sm;
 }
 
 }  // namespace cress

@@ -556,7 +556,7 @@ int hevi_row_tiles_x(const Grid& g) { return (g.ni - 3 + kHrCols - 1) / kHrCols;
 // recomputes and its start, and the blocks run in waves of one per SM; the
 // shortest total wins.
 int hevi_row_rows(const Grid* const* g, int n) {
-  const int nsm = 148;
+  const int nsm = sm_count();
   int best = 1, ny_max = 1;
   for (int m = 0; m < n; ++m) ny_max = std::max(ny_max, g[m]->nj - 3);
   double cost = 1e30;

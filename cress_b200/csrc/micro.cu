@@ -478,9 +478,7 @@ int launch_cloudphy_fused(const MicroArgs& a, const float* w, Mlp* m, const Lear
     return rc;
   if (cudaFuncSetAttribute(k_mlp_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem) != cudaSuccess)
     return CRESS_E_CUDA;
-  int dev = 0, nsm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int nsm = sm_count();
   FusedArgs p{};
   p.w = w;
   p.norm = m->norm_d;

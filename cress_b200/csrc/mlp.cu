@@ -20,6 +20,7 @@
 #include <vector>
 #include "../../include/cress_b200.h"
 #include "mlp.cuh"
+#include "common.cuh"
 #include "mlp_impl.cuh"
 
 namespace cress {
@@ -287,7 +288,7 @@ int Mlp::forward(int B) {
 // loss and gradient of a batch of 8192 took 1.17 ms before and 0.48 ms with it.
 static int wgrad_split(int n, int B) {
   const int tiles = kMlpH / 128 * ((n + 255) / 256);
-  const int parts = B / 256 < 148 / tiles ? B / 256 : 148 / tiles;
+  const int wave = sm_count() / tiles, parts = B / 256 < wave ? B / 256 : wave;
   return parts > 1 ? parts : 1;
 }
 
