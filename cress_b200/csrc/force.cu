@@ -154,10 +154,10 @@ __device__ __forceinline__ void force_point(const ForceArgs& a, const float* tab
   // 2nd-order sums Sx, Sy (coefficients cx, cy) and 4th-order sums Px, Py (dx,
   // dy); open x: the 2nd-order form in the boundary columns
   auto hsum = [&](F2 f, F2 Sx, F2 Sy, F2 Px, F2 Py, float cx, float cy, float px, float py) {
-    F2 r = fma2(f2(fourd3 * cx), Sx, f);
-    r = fma2(f2(fourd3 * cy), Sy, r);
-    r = fma2(f2(px), Px, r);
+    F2 r = fma2(f2(px), Px, f);   // the smaller terms first: they round at their own size
     r = fma2(f2(py), Py, r);
+    r = fma2(f2(fourd3 * cx), Sx, r);
+    r = fma2(f2(fourd3 * cy), Sy, r);
     if (edge) r = sel2(edge, fma2(f2(cy), Sy, fma2(f2(cx), Sx, f)), r);
     return r;
   };

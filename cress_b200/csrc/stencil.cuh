@@ -17,9 +17,12 @@ namespace cress {
 // the own column, and may be evaluated at every dz in -2..2 (a shared-memory
 // ring that holds those levels, whatever they contain at the ends of the
 // column).  The reference's nested second differences are one weighted sum
-// per direction, -(H(2) + H(-2)) + 4 (H(1) + H(-1)) - 6 H(0); it differs from
-// them by FP32 rounding, about 1e-6 of the field times the coefficient
-// (1e-3).  The reference clamps the vertical second difference at kmin and
+// per direction, 4 (d(1) + d(-1)) - (d(2) + d(-2)) of the differences d from
+// the point's own value, which are exact or round with the difference, not with the
+// field: a base state's wind cancels in them, as it does in the reference, whose
+// smoothed quantity is less the base state.  (Weighting the values themselves
+// rounds with the whole wind: the forcing of u then differs from 64 bits by up to
+// 6.3e-6 where this and the reference's form differ by 1e-7.)  The reference clamps the vertical second difference at kmin and
 // kmax (tmp3(kmin-1) = tmp3(kmin), tmp3(kmax+1) = tmp3(kmax)); here that is a
 // selection, so every offset is a compile-time constant.
 // edge: the points (bit 0 first, bit 1 second) in an open-x boundary column,
@@ -29,9 +32,9 @@ template <class FH, class FA>
 __device__ __forceinline__ F2 smooth_sum(F2 frc, int smtopt, float smhc, float smvcoe, int k, int kmin, int kmax,
                                          const FH& H, const FA& A, int edge = 0) {
   const F2 c = H(0, 0);
-  const F2 n1 = (H(1, 0) + H(-1, 0)) + (H(0, 1) + H(0, -1));
-  const F2 n2 = (H(2, 0) + H(-2, 0)) + (H(0, 2) + H(0, -2));
-  const F2 h4 = fma2(f2(-12.f), c, fma2(f2(4.f), n1, F2{0} - n2));
+  const F2 n1 = ((H(1, 0) - c) + (H(-1, 0) - c)) + ((H(0, 1) - c) + (H(0, -1) - c));
+  const F2 n2 = ((c - H(2, 0)) + (c - H(-2, 0))) + ((c - H(0, 2)) + (c - H(0, -2)));
+  const F2 h4 = fma2(f2(4.f), n1, n2);
   const F2 a0 = A(0), am = A(-1), ap = A(1);
   const F2 t30 = (ap + am) - 2.f * a0;
   F2 v = t30;
@@ -42,7 +45,7 @@ __device__ __forceinline__ F2 smooth_sum(F2 frc, int smtopt, float smhc, float s
   }
   const F2 r = fma2(f2(smvcoe), v, fma2(f2(smhc), h4, frc));
   if (!edge) return r;
-  return sel2(edge, fma2(f2(smvcoe), t30, fma2(f2(smhc), fma2(f2(-4.f), c, n1), frc)), r);
+  return sel2(edge, fma2(f2(smvcoe), t30, fma2(f2(smhc), n1, frc)), r);
 }
 
 // The same term by term in the reference's parenthesisation (the moist scalars,
