@@ -501,9 +501,9 @@ int Ctx::base_changed() {
 }
 
 // Tiles 0 and 13 run the row-marching kernel where its chunks cover the
-// column (tile 13 is offered up to kHevi3MaxNk levels): it is the faster one at
-// every size measured, 14 us against 85 us per substep at 64x64x40 and 0.197 ms
-// against 0.289 ms (0.321 ms with tile 0's k_hevi2) at 512x512x64.
+// column: it is the fastest at every size measured, 10 us against 85 us per
+// substep at 64x64x40 and 0.175 ms against 0.321 ms (tile 0's k_hevi2) at
+// 512x512x64.  Tile 13 is offered up to kHevi3MaxNk levels, as it is declared.
 bool Ctx::row_kernel() const {
   return cfg.impopt == 1 && (cfg.tile == 0 || (cfg.tile == 13 && g.nk <= kHevi3MaxNk)) && hevi_row_supported(g);
 }
@@ -571,6 +571,8 @@ int Ctx::small_steps(int nsstp, float dts, std::vector<HeviJob>* jobs, std::vect
   if (!heve && (rc = thomas_for(dts, &th))) return rc;
   if (th) { a.thom_rr = th->rr; a.thom_aa = th->aa; a.thom_cp = th->cp; a.lvl3 = th->lvl3; }
   const bool row = row_kernel() && !jobs;
+  if (!heve && !jobs && cfg.tile == 13 && !row)
+    return set_error(CRESS_E_UNSUPPORTED, "HE-VI tile 13 needs 8 <= nk <= %d", kHevi3MaxNk);
   if (rjobs && !row) return set_error(CRESS_E_UNSUPPORTED, "the row kernel does not run on this grid");
   HeviRowArgs ra{};
   HeviRowMaps rm;
@@ -1068,10 +1070,16 @@ int Ctx::autotune(int nsstp, float dts, int reps, int* best, float* ms) {
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
     return set_error(CRESS_E_CUDA, "cudaEventCreate failed");
   float best_ms = 0.f;
+  float ms0 = 0.f;
+  bool row0 = false;   // tile 0 was timed and runs the row kernel
   int best_tile = -1, rc = CRESS_OK;
   for (int t = 0; t < CRESS_NTILES; ++t) {
     cfg.tile = t;
     if (ms) ms[t] = -1.f;
+    if (t == 13 && row0 && row_kernel()) {   // the same kernel: one timing for both, and tile 0 on a tie
+      if (ms) ms[t] = ms0;
+      continue;
+    }
     rc = small_steps(nsstp, dts);   // warm-up; a shape the grid cannot use is skipped
     if (rc == CRESS_E_UNSUPPORTED) { rc = CRESS_OK; continue; }
     if (rc) break;
@@ -1085,6 +1093,7 @@ int Ctx::autotune(int nsstp, float dts, int reps, int* best, float* ms) {
     cudaEventElapsedTime(&t_ms, e0, e1);
     t_ms /= (float)(reps * nsstp);
     if (ms) ms[t] = t_ms;
+    if (t == 0) { ms0 = t_ms; row0 = row_kernel(); }
     if (best_tile < 0 || t_ms < best_ms) { best_ms = t_ms; best_tile = t; }
   }
   cudaEventDestroy(e0);
@@ -1121,7 +1130,7 @@ struct Ensemble {
   cudaEvent_t staged = nullptr;       // the last copy out of jobs_h has completed
   long long launches = 0;
   bool graphs = true;
-  int tile = 0;                       // the batched acoustic kernel: tile 0's or tile 13's
+  int tile = 0;                       // 0 or 13: the members' tile
   struct Rec {
     cudaGraphExec_t exec = nullptr;
     HeviJob* jobs_d = nullptr;        // this graph's job table and its pinned source
@@ -1285,8 +1294,7 @@ int Ensemble::jobs_for(int nsstp, float dts, HeviJob* jh, int* nblocks, int* nk_
   return CRESS_OK;
 }
 
-// Tile 13 holds each column's eliminated right-hand sides on chip, so every
-// member needs nk <= kHevi3MaxNk.
+// Tile 13 is declared for 8 <= nk <= kHevi3MaxNk (there its kernel is tile 0's).
 int Ensemble::set_tile(int t) {
   if (t != 0 && t != 13) return set_error(CRESS_E_ARG, "ensemble tile %d (0 or 13)", t);
   if (t == 13)
@@ -1316,6 +1324,7 @@ int Ensemble::autotune(int nsstp, float dts, int reps, int* best, float* ms) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int rc = CRESS_OK, best_t = -1;
   float best_ms = 0.f;
+  bool row0 = false;   // tile 0 was timed and runs the row kernel
   if (cudaMalloc(&jd, sizeof(HeviJob) * need) != cudaSuccess ||
       cudaMallocHost(&jh, sizeof(HeviJob) * need) != cudaSuccess || cudaEventCreate(&e0) != cudaSuccess ||
       cudaEventCreate(&e1) != cudaSuccess)
@@ -1324,6 +1333,10 @@ int Ensemble::autotune(int nsstp, float dts, int reps, int* best, float* ms) {
   for (int q = 0; q < 2 && !rc; ++q) {
     if (ms) ms[q] = -1.f;
     if (set_tile(cand[q]) != CRESS_OK) continue;   // tile 13 needs nk <= kHevi3MaxNk
+    if (q == 1 && row0 && rows()) {   // the same kernel: one timing for both, and tile 0 on a tie
+      if (ms) ms[1] = best_ms;
+      continue;
+    }
     int nblocks = 0, nk_max = 0;
     if ((rc = jobs_for(nsstp, dts, jh, &nblocks, &nk_max))) break;
     if ((rc = cuda_check(cudaMemcpyAsync(jd, jh, sizeof(HeviJob) * need, cudaMemcpyHostToDevice, stream),
@@ -1343,6 +1356,7 @@ int Ensemble::autotune(int nsstp, float dts, int reps, int* best, float* ms) {
     cudaEventElapsedTime(&t_ms, e0, e1);
     t_ms /= (float)(reps * nsstp);
     if (ms) ms[q] = t_ms;
+    if (q == 0) row0 = rows();
     if (best_t < 0 || t_ms < best_ms) { best_ms = t_ms; best_t = cand[q]; }
   }
   cudaStreamSynchronize(stream);

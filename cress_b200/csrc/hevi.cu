@@ -386,7 +386,6 @@ int launch_hevi_substep(const HeviArgs& a, const HeviMaps& maps, int tile, cudaS
     case 0: return launch_hevi2(a, maps, 0, st);
     case 11: return launch_hevi2(a, maps, 1, st);
     case 12: return launch_hevi3(a, maps, st);
-    case 13: return CRESS_E_UNSUPPORTED;   // the row kernel (hevi_row.cu): nk <= kHevi3MaxNk
     case 1: return launch_t<2, 5, float>(a, maps, st);
     case 2: return launch_t<8, 4, float>(a, maps, st);
     case 3: return launch_t<4, 5, double>(a, maps, st);

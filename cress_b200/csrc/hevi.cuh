@@ -59,9 +59,9 @@ struct alignas(16) HeviLevel {
 };
 static_assert(sizeof(HeviLevel) == 144, "HeviLevel is nine 16-byte vectors");
 
-// Largest nk of tiles 12 and 13.  Tile 12: the eliminated right-hand sides of
-// levels 3..nk-2 of two columns in FP64 fill 4 (nk - 4) <= 256 tensor-memory
-// columns per thread.
+// Largest nk of tile 12: the eliminated right-hand sides of levels 3..nk-2 of
+// two columns in FP64 fill 4 (nk - 4) <= 256 tensor-memory columns per thread.
+// Tile 13 is declared for the same heights (cress_cfg.tile).
 constexpr int kHevi3MaxNk = 68;
 
 struct HeviArgs {
@@ -94,7 +94,8 @@ struct HeviArgs {
 int hevi_tile_rows(int tile);
 // The on-chip kernel (tile 12); needs a.lvl3 and nk <= kHevi3MaxNk.
 int launch_hevi3(const HeviArgs& a, const HeviMaps& maps, cudaStream_t st);
-// Launch one substep; `maps` must describe the buffers in `a` with the
+// Launch one substep of tiles 0-12 (tile 13 and, up to 83 levels nk, tile 0 go to
+// hevi_row.cu); `maps` must describe the buffers in `a` with the
 // box rows of HeviRows<hevi_tile_rows(tile)>.
 int launch_hevi_substep(const HeviArgs& a, const HeviMaps& maps, int tile, cudaStream_t st);
 // One member's substep in an ensemble launch (tile 0's or tile 13's kernel

@@ -309,7 +309,8 @@ int cress_diagnostics(cress_ctx* ctx, int level, double* out);
  * the current state, which it leaves untouched (only the future level is
  * written), and keeps the fastest as the context's tile.  best_tile and
  * ms_per_substep[CRESS_NTILES] (milliseconds per substep, -1 for shapes
- * this grid cannot use) may be null. */
+ * this grid cannot use) may be null.  Where tiles 0 and 13 are one kernel it is
+ * timed once and both get that time. */
 int cress_autotune(cress_ctx* ctx, int nsstp, float dts, int reps, int* best_tile, float* ms_per_substep);
 
 /* Ensembles.  An ensemble groups contexts of independent domains (any
@@ -327,12 +328,12 @@ int cress_autotune(cress_ctx* ctx, int nsstp, float dts, int reps, int* best_til
  * height in separate launches) when every member's grid allows it, else
  * tile 0's 32x8 kernel.  The ensemble's tile is 13 (every member with
  * 8 <= nk <= 68) when every member was created with tile 13, else 0, and the
- * members are set
- * to the ensemble's tile.  cress_ensemble_set_tile switches it (0 or 13);
+ * members are set to the ensemble's tile.  cress_ensemble_set_tile switches it (0 or 13);
  * cress_ensemble_autotune times both over `reps` loops of nsstp batched
  * substeps of length dts on the members' present state (only the future
  * levels are written) and keeps the faster (best_tile, ms_per_substep[2]
- * for tiles 0 and 13, -1 where unusable; both may be null).  Members stay
+ * for tiles 0 and 13, -1 where unusable; both may be null; where they are one
+ * kernel it is timed once).  Members stay
  * valid contexts (sync calls, cress_large_step); destroy the ensemble
  * before its members. */
 typedef struct cress_ensemble cress_ensemble;

@@ -40,10 +40,39 @@ def test_levels_beyond_the_chunks_run_the_ring_kernel(cress, oracle_lib):
     check(ni, nj, nk, ref, out, 2)
 
 
-def test_ensemble_of_different_heights_matches_members(cress, oracle_lib):
+def test_tile_13_is_tile_0_up_to_its_height(cress, oracle_lib):
+    """Tiles 0 and 13 are one kernel up to nk = 68, which the autotuner times
+    once; above, tile 13 stays refused."""
+    for nz in (65, 66):
+        ni, nj, nk = H.dims(24, 12, nz)
+        base = H.base3d(ni, nj, nk, 200.0, 1)
+        st, frc = H.small_state(ni, nj, nk, 2, base)
+        out = []
+        for tile in (0, 13):
+            s = cress.Solver(ni, nj, nk, 1000.0, 1000.0, 200.0, sthopt=1, tile=tile)
+            s.set_base3d(base)
+            if tile == 13 and nk > 68:
+                with pytest.raises(cress.CressError) as e:
+                    s.smalldrv(2, 0.5, *st, *frc)
+                assert e.value.code == 2             # CRESS_E_UNSUPPORTED
+            else:
+                out.append(s.smalldrv(2, 0.5, *st, *frc))
+                best, ms = s.autotune(2, 0.5, reps=2)
+                assert ms[0] > 0 and best != 13
+                assert ms[13] == (ms[0] if nk <= 68 else -1)
+            s.close()
+        for a in out[1:]:
+            for x, y in zip(out[0], a):
+                assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("sizes", [
+    [(40, 33, 22, 1), (64, 20, 36, 2), (29, 45, 22, 3)],
+    [(190, 41, 22, 1), (131, 70, 22, 2), (64, 20, 22, 3)],   # members with tiles inside the edges, strips of two rows
+])
+def test_ensemble_of_different_heights_matches_members(cress, oracle_lib, sizes):
     """Members with different chunk lengths go out in separate launches; each
     equals the member stepped alone, bit for bit."""
-    sizes = [(40, 33, 22, 1), (64, 20, 36, 2), (29, 45, 22, 3)]
     out = []
     for together in (False, True):
         sols = [member(cress, oracle_lib, *sz) for sz in sizes]
