@@ -4,7 +4,7 @@ Every ring wait in the kernels is bounded; when one gives up, the kernel
 records it in the context's device error word, stops issuing copies, waits
 (with the full limit) for the copies already in flight and returns, and the
 host reports CRESS_E_TIMEOUT.  The test hook cress_set_spin_limit(0) makes
-the level loop's first wait give up at once, so every block takes that
+the kernel's first wait give up at once, so every block takes that
 path; nothing is left waiting and no copy outlives its block.  The same
 context must then run normally again and match the oracle.
 """
@@ -18,8 +18,9 @@ pytestmark = pytest.mark.gpu
 STAG = {"u": "u", "v": "v", "w": "s", "pp": "s"}
 
 
-def test_wait_gives_up_reports_timeout_and_context_recovers(cress, oracle_lib):
-    nx, ny, nz, nsstp, dts = 40, 24, 20, 2, 0.5
+@pytest.mark.parametrize("nz", [20, 82])   # the row march, and the level loop of taller columns
+def test_wait_gives_up_reports_timeout_and_context_recovers(cress, oracle_lib, nz):
+    nx, ny, nsstp, dts = 40, 24, 2, 0.5
     ni, nj, nk = H.dims(nx, ny, nz)
     base = H.base3d(ni, nj, nk, 250.0, 1)
     st, frc = H.small_state(ni, nj, nk, 3, base)

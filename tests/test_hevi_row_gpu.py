@@ -35,6 +35,19 @@ def test_options(cress, oracle_lib, divopt, sthopt):
     check(ni, nj, nk, ref, out, 4)
 
 
+@pytest.mark.parametrize("nx,ny,nz", [
+    (250, 118, 20),   # chunks of 2, strips of 5 rows, the last of 3
+    (130, 259, 37),   # chunks of 3, strips of 6 rows, the last of 1
+    (190, 203, 54),   # chunks of 4, strips of 6 rows, the last of 5
+    (190, 151, 80),   # 16 full chunks of 5, strips of 5 rows, the last of 1
+])
+def test_strips_of_several_rows(cress, oracle_lib, nx, ny, nz):
+    # what a solved row leaves for the next: parked values, the exchange
+    # buffers used again, the copies' parity over many rows; tiles without edge
+    ni, nj, nk, ref, out = run_pair(cress, oracle_lib, nx, ny, nz, 3, sthopt=1, seed=nx + nz, tile=0)
+    check(ni, nj, nk, ref, out, 3)
+
+
 def test_levels_beyond_the_chunks_run_the_ring_kernel(cress, oracle_lib):
     ni, nj, nk, ref, out = run_pair(cress, oracle_lib, 40, 12, 82, 2, sthopt=1, seed=8, tile=0, dz=150.0)
     check(ni, nj, nk, ref, out, 2)
