@@ -549,6 +549,8 @@ class Mlp:
         return y
 
     def loss_grad(self, x, t):
+        """Mean-square loss and its gradient for one batch (to FP32 rounding:
+        the sums' parts are added in no fixed order)."""
         x = np.ascontiguousarray(x, np.float32)
         t = np.ascontiguousarray(t, np.float32)
         loss = np.zeros(1, np.float32)

@@ -32,7 +32,7 @@
 // ring of xy tiles before, tile 0 / tile 13 -> this kernel):
 //   64 x 64 x 40    85 -> 10    (16 tiles on 148 SMs, 64 levels in a row)
 //   203 x 131 x 54  125 -> 27
-//   512 x 512 x 64  321 / 289 -> 179: 4.5 TB/s of its 48 bytes per cell, 0.69 of
+//   512 x 512 x 64  321 / 289 -> 175: 4.6 TB/s of its 48 bytes per cell, 0.70 of
 //                   the measured copy bandwidth, 54.3 bytes per cell of DRAM traffic
 // Marching k, all levels of a column wait for one another and a grid of few
 // tiles leaves SMs idle; a substep also spent about 270 warp instructions per 32
@@ -41,7 +41,7 @@
 // 170 per 32 cells.  It is bound by the latency of its 16 warps per SM: 128 registers each
 // (which is why a row's p' tendency and w right-hand side wait in
 // shared memory, and why the row's addresses, the stage's place and the number of
-// own levels are formed again each row: 195 -> 179 us at 512 x 512 x 64), two
+// own levels are formed again each row: 195 -> 175 us at 512 x 512 x 64), two
 // barriers per row.  Tried and slower: direct global loads instead of TMA (406 us at
 // 512 x 512 x 64: the row's loads are not in flight during the solve),
 // prefetching a second row into L2 by TMA (235 us), both rows' values in

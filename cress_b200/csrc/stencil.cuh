@@ -22,9 +22,10 @@ namespace cress {
 // field: a base state's wind cancels in them, as it does in the reference, whose
 // smoothed quantity is less the base state.  (Weighting the values themselves
 // rounds with the whole wind: the forcing of u then differs from 64 bits by up to
-// 6.3e-6 where this and the reference's form differ by 1e-7.)  The reference clamps the vertical second difference at kmin and
-// kmax (tmp3(kmin-1) = tmp3(kmin), tmp3(kmax+1) = tmp3(kmax)); here that is a
-// selection, so every offset is a compile-time constant.
+// 6.2e-6 where this and the reference's form differ by 1e-7.)  The reference
+// clamps the vertical second difference at kmin and kmax (tmp3(kmin-1) =
+// tmp3(kmin), tmp3(kmax+1) = tmp3(kmax)); here that is a selection, so every offset
+// is a compile-time constant.
 // edge: the points (bit 0 first, bit 1 second) in an open-x boundary column,
 // where only the 2nd-order part applies (smoo4uvw.f90:286-330 and the other
 // smoo4*: the 4th-order loops run over i = 2+iwest .. with iwest = 1).

@@ -422,7 +422,10 @@ int cress_mlp_set_norm(cress_mlp* m, const float* host);
 /* Network function: x [n][16] standardized inputs -> y [n][9]. */
 int cress_mlp_forward(cress_mlp* m, int n, const float* x, float* y);
 /* Mean-square loss and its gradient w.r.t. every parameter for one batch
- * (x [n][16], t [n][9] standardized; n a multiple of 128). */
+ * (x [n][16], t [n][9] standardized; n a multiple of 128).  Loss and
+ * gradients, the weights' too, are FP32 sums whose parts meet in no fixed
+ * order: two calls on the same inputs agree to rounding, not bit for bit, and
+ * so do two training runs. */
 int cress_mlp_loss_grad(cress_mlp* m, int n, const float* x, const float* t, float* loss, float* grad);
 /* Tuple store (transformed, unstandardized features and targets). */
 int cress_mlp_reserve(cress_mlp* m, long long cap);
