@@ -35,8 +35,8 @@ HEVI_BYTES_PER_CELL = 48  # u,v,w,p' read + write and 4 forcings read, float32
 # DRAM bytes per cell of one HE-VI launch measured by ncu on a 384x384x64
 # domain (dram__bytes_read.sum + dram__bytes_write.sum over 384*384*63
 # cells); the traffic grows with the cells.  Tiles 0 and 13 run the
-# row-marching kernel: 374.6 + 129.3 MB.
-HEVI_TRAFFIC_PER_CELL = {t: (374.62e6 + 129.25e6) / (384 * 384 * 63) for t in (0, 13)}
+# row-marching kernel: 374.1 + 128.3 MB.
+HEVI_TRAFFIC_PER_CELL = {t: (374.11e6 + 128.30e6) / (384 * 384 * 63) for t in (0, 13)}
 HEVI_KERNEL = {0: "k_hevi_row", 11: "k_hevi2", 12: "k_hevi3", 13: "k_hevi_row"}
 METRIC = "cell-updates/s on 1 B200: plain vs learned-microphysics form at stated error"
 MOIST = ["qv", "qc", "qr", "qi", "qs", "qg", "ni", "ns", "ng"]

@@ -28,7 +28,7 @@
 //
 // What bounds it: instruction issue.  Every advection term is a sum of (wind
 // sum) x (difference) with the per-level constants factored out of it, the
-// smoothing one weighted sum per direction (stencil.cuh): 926 -> 870 us for
+// smoothing one sum of differences per direction (stencil.cuh): 926 -> 870 us for
 // both kernels at 512 x 512 x 64 with the eddy mixing.  The launch bounds
 // name the blocks per SM that the rings leave room for (two with the eddy
 // viscosity staged, three without), so that the registers are used up: left

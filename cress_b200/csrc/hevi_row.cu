@@ -38,7 +38,7 @@
 // tiles leaves SMs idle; a substep also spent about 270 warp instructions per 32
 // cells, half of them on ring, address and halo bookkeeping.  Here the levels
 // of a row run at once, the strip length adapts to the grid, and it is about
-// 170 per 32 cells.  It is bound by the latency of its 16 warps per SM: 128 registers each
+// 155 per 32 cells.  It is bound by the latency of its 16 warps per SM: 128 registers each
 // (which is why a row's p' tendency and w right-hand side wait in
 // shared memory, and why the row's addresses, the stage's place and the number of
 // own levels are formed again each row: 195 -> 175 us at 512 x 512 x 64), two
