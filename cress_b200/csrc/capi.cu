@@ -1161,6 +1161,8 @@ struct Ensemble {
     if (done) cudaEventDestroy(done);
     if (jobs_d) cudaFree(jobs_d);
     if (jobs_h) cudaFreeHost(jobs_h);
+    for (cudaEvent_t x : side_ev) cudaEventDestroy(x);
+    for (cudaStream_t x : side) cudaStreamDestroy(x);
     if (stream) cudaStreamDestroy(stream);
   }
   int large_step(long long ctime, float dtb, int nsstp, float dts, HeviJob* jd, HeviJob* jh, bool eager);
@@ -1168,24 +1170,53 @@ struct Ensemble {
   int set_tile(int t);
   // Whether the batched substeps run the row kernel (every member's grid
   // must allow it; else tile 0's k_hevi2_batch).  Then a substep is one
-  // launch per group of members with equal chunk lengths and counts
-  // (members of equal nk share one).
+  // launch per group of members with equal chunk lengths, four at most,
+  // and the groups, which have nothing to wait for from one another, run beside
+  // each other on the streams of `side`.  Twelve 64x64 members of twelve
+  // heights, us per substep: one launch per height, one after the other, 153; on
+  // eight streams 111; one per chunk length, each on its stream, 64.
   bool rows() const {
     for (const Ctx* c : members)
       if (!c->row_kernel()) return false;
     return true;
   }
-  struct Group { int first, n, nblocks, nk; };
+  struct Group { int first, n, nblocks, nk; };   // nk: the tallest
   std::vector<Group> groups;   // of the jobs last formed
-  int batch(const HeviJob* jobs, int st, int nblocks, int nk_max) {   // substep st of the job table
+  std::vector<cudaStream_t> side;
+  std::vector<cudaEvent_t> side_ev;
+  // The nsstp substeps of a job table on the device, `loops` times over:
+  // ordered after the work on `stream`, and later work there after them.
+  int substeps(const HeviJob* jobs, int nsstp, int nblocks, int nk_max, int loops = 1) {
     const cress_cfg& c0 = members[0]->cfg;
-    const int n = (int)members.size();
-    if (groups.empty())
-      return launch_hevi_batch(jobs + (size_t)st * n, n, nblocks, nk_max, c0.divopt, c0.sthopt != 0, c0.buyopt == 1, stream);
-    const HeviRowJob* rj = reinterpret_cast<const HeviRowJob*>(jobs) + (size_t)st * n;
-    for (const Group& q : groups) {
-      const int rc = launch_hevi_row_batch(rj + q.first, q.n, q.nblocks, q.nk, stream);
-      if (rc) return rc;
+    const int n = (int)members.size(), ns = (int)groups.size();   // streams used
+    int rc;
+    for (int q = (int)side.size(); q < ns - 1; ++q) {
+      cudaStream_t x = nullptr;
+      cudaEvent_t y = nullptr;
+      if ((rc = cuda_check(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking), "ensemble stream"))) return rc;
+      side.push_back(x);
+      if ((rc = cuda_check(cudaEventCreateWithFlags(&y, cudaEventDisableTiming), "ensemble event"))) return rc;
+      side_ev.push_back(y);
+    }
+    if (ns > 1) cudaEventRecord(fork, stream);
+    for (int q = 0; q < ns - 1; ++q) cudaStreamWaitEvent(side[q], fork, 0);
+    for (int st = 0; st < loops * nsstp; ++st) {
+      const size_t at = (size_t)(st % nsstp) * n;
+      if (groups.empty()) {
+        if ((rc = launch_hevi_batch(jobs + at, n, nblocks, nk_max, c0.divopt, c0.sthopt != 0, c0.buyopt == 1, stream)))
+          return rc;
+        ++launches;
+      }
+      for (size_t q = 0; q < groups.size(); ++q) {
+        const HeviRowJob* rj = reinterpret_cast<const HeviRowJob*>(jobs) + at + groups[q].first;
+        if ((rc = launch_hevi_row_batch(rj, groups[q].n, groups[q].nblocks, groups[q].nk, q ? side[q - 1] : stream)))
+          return rc;
+        ++launches;
+      }
+    }
+    for (int q = 0; q < ns - 1; ++q) {
+      cudaEventRecord(side_ev[q], side[q]);
+      cudaStreamWaitEvent(stream, side_ev[q], 0);
     }
     return CRESS_OK;
   }
@@ -1218,11 +1249,8 @@ int Ensemble::large_step(long long ctime, float dtb, int nsstp, float dts, HeviJ
                        "copy ensemble jobs")))
     return rc;
   if (eager) cudaEventRecord(staged, stream);
-  for (int st = 0; st < nsstp; ++st) {
-    if ((rc = batch(jd, st, nblocks, nk_max)))
-      return set_error(rc, "ensemble small-step launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-    ++launches;
-  }
+  if ((rc = substeps(jd, nsstp, nblocks, nk_max)))
+    return set_error(rc, "ensemble small-step launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   cudaEventRecord(done, stream);
   for (int m = 0; m < n; ++m) {
     Ctx* c = members[m];
@@ -1250,17 +1278,15 @@ int Ensemble::jobs_for(int nsstp, float dts, HeviJob* jh, int* nblocks, int* nk_
     // the jobs of a substep in group order, in the table's memory
     static_assert(sizeof(HeviRowJob) <= sizeof(HeviJob), "the job tables hold either kind");
     HeviRowJob* rj = reinterpret_cast<HeviRowJob*>(jh);
-    std::map<std::pair<int, int>, std::vector<int>> by;   // (chunk length, chunks) -> members
-    for (int m = 0; m < n; ++m) {
-      const int nk = members[m]->g.nk, L = hevi_row_chunk(nk);
-      by[{L, (nk - 3 + L - 1) / L}].push_back(m);
-    }
+    std::map<int, std::vector<int>> by;   // chunk length -> members
+    for (int m = 0; m < n; ++m) by[hevi_row_chunk(members[m]->g.nk)].push_back(m);
+    std::vector<const Grid*> gs;   // the groups share the GPU, and so one number of rows
+    for (const Ctx* c : members) gs.push_back(&c->g);
+    const int rows_ = hevi_row_rows(gs.data(), n);
     int at = 0;
     for (auto& kv : by) {
-      std::vector<const Grid*> gs;
-      for (int m : kv.second) gs.push_back(&members[m]->g);
-      const int rows_ = hevi_row_rows(gs.data(), (int)gs.size());
-      Group q{at, (int)gs.size(), 0, gs[0]->nk};
+      Group q{at, (int)kv.second.size(), 0, 0};
+      for (int m : kv.second) q.nk = std::max(q.nk, members[m]->g.nk);
       for (int m : kv.second) {
         std::vector<HeviRowJob> per;
         if ((rc = members[m]->small_steps(nsstp, dts, nullptr, &per))) return rc;
@@ -1342,11 +1368,12 @@ int Ensemble::autotune(int nsstp, float dts, int reps, int* best, float* ms) {
     if ((rc = cuda_check(cudaMemcpyAsync(jd, jh, sizeof(HeviJob) * need, cudaMemcpyHostToDevice, stream),
                          "copy ensemble jobs")))
       break;
-    for (int st = 0; st < nsstp && !rc; ++st) rc = batch(jd, st, nblocks, nk_max);   // warm-up
+    const long long l0 = launches;
+    rc = substeps(jd, nsstp, nblocks, nk_max);   // warm-up
     cudaEventRecord(e0, stream);
-    for (int r = 0; r < reps && !rc; ++r)
-      for (int st = 0; st < nsstp && !rc; ++st) rc = batch(jd, st, nblocks, nk_max);
+    if (!rc) rc = substeps(jd, nsstp, nblocks, nk_max, reps);
     cudaEventRecord(e1, stream);
+    launches = l0;
     if (rc == CRESS_E_UNSUPPORTED) { rc = CRESS_OK; continue; }
     if (rc || (rc = cuda_check(cudaEventSynchronize(e1), "ensemble autotune sync"))) break;
     for (Ctx* c : members)

@@ -145,14 +145,17 @@ struct HrLayout {
 };
 
 // EDGE: the tile holds columns whose values have images in x (the others
-// carry no code for them).
-template <int L, bool EDGE>
+// carry no code for them).  BATCH: the block has the warps of the launch's
+// tallest grid; those beyond this one's chunks leave, and the barriers count
+// the others.
+template <int L, bool EDGE, bool BATCH>
 __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviRowArgs& a, unsigned char* smem, int bx,
                                                int by) {
   using Y = HrLayout<L>;
   const Grid& g = a.g;
   const int nk = g.nk, ni = g.ni, nj = g.nj;
-  const int lane0 = threadIdx.x & 31, c0 = threadIdx.x >> 5, nC = blockDim.x >> 5;
+  const int lane0 = threadIdx.x & 31, c0 = threadIdx.x >> 5;
+  const int nC = BATCH ? (nk - 4 + L) / L : blockDim.x >> 5;   // levels 2..nk-2
   const int k0 = 2 + c0 * L;
 
   auto stage_of = [&](int c) { return smem + Y::oS + c * (Y::stage + Y::parked); };
@@ -198,8 +201,13 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
       reinterpret_cast<uint4*>(smem + Y::oE)[n] = reinterpret_cast<uint4*>(smem + Y::oW)[n] = make_uint4(0, 0, 0, 0);
   }
   grid_dependency_wait();
-  if (lane0 == 0) issue(j0 - 1, c0);
+  if (lane0 == 0 && (!BATCH || c0 < nC)) issue(j0 - 1, c0);
   __syncthreads();
+  if (BATCH && c0 >= nC) return;
+  auto block_sync = [&]() {
+    if constexpr (BATCH) asm volatile("bar.sync 1, %0;" ::"r"(32 * nC) : "memory");
+    else __syncthreads();
+  };
 
   const int ilast = min(i0 + kHrCols - 1, ni - 2);
   const bool o0 = i >= i0 && i <= ilast, o1 = i + 1 >= i0 && i + 1 <= ilast;
@@ -375,7 +383,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
       for (int l = 1; l < L; ++l)
         if (l >= nlev) fa[l] = fb[l] = 0.0;
     }
-    __syncthreads();
+    block_sync();
     double xa = 0.0, xb = 0.0;
     for (int n = 0; n < c; n += 4) {   // the entry value from the chunks below
 #pragma unroll
@@ -396,7 +404,7 @@ __device__ __forceinline__ void hevi_row_strip(const HeviRowMaps& m, const HeviR
       yb = __fma_rn(-cp.x, yb, fb[l]);
     }
     *reinterpret_cast<double2*>(smem + Y::oW + 16 * (c * 32 + lane)) = make_double2(ya, yb);
-    __syncthreads();
+    block_sync();
     ya = yb = 0.0;
     for (int n = (c + 1) & ~3; n < nC; n += 4) {   // w of the level above, from the chunks above
 #pragma unroll
@@ -446,8 +454,8 @@ template <int L>
 __global__ void __launch_bounds__(32 * kHrMaxWarps, 1)
 k_hevi_row(const __grid_constant__ HeviRowMaps m, const __grid_constant__ HeviRowArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  if (blockIdx.x == 0 || blockIdx.x + 1 == a.tiles_x) hevi_row_strip<L, true>(m, a, smem, blockIdx.x, blockIdx.y);
-  else hevi_row_strip<L, false>(m, a, smem, blockIdx.x, blockIdx.y);
+  if (blockIdx.x == 0 || blockIdx.x + 1 == a.tiles_x) hevi_row_strip<L, true, false>(m, a, smem, blockIdx.x, blockIdx.y);
+  else hevi_row_strip<L, false, false>(m, a, smem, blockIdx.x, blockIdx.y);
 }
 
 // Every member of an ensemble in one launch: block b belongs to the member
@@ -479,8 +487,8 @@ __global__ void __launch_bounds__(32 * kHrMaxWarps, 1) k_hevi_row_batch(const He
   __syncthreads();
   const HeviRowArgs& a = *reinterpret_cast<const HeviRowArgs*>(words);
   const int t = b - job.first_block, bx = t % a.tiles_x;
-  if (bx == 0 || bx + 1 == a.tiles_x) hevi_row_strip<L, true>(job.maps, a, smem, bx, t / a.tiles_x);
-  else hevi_row_strip<L, false>(job.maps, a, smem, bx, t / a.tiles_x);
+  if (bx == 0 || bx + 1 == a.tiles_x) hevi_row_strip<L, true, true>(job.maps, a, smem, bx, t / a.tiles_x);
+  else hevi_row_strip<L, false, true>(job.maps, a, smem, bx, t / a.tiles_x);
 }
 
 // The boundary levels and the y ghosts the row kernel leaves out, once after

@@ -69,9 +69,9 @@ bool hevi_row_supported(const Grid& g);
 // x ghosts; the boundary levels and the y ghosts are left to
 // launch_hevi_row_ends.
 int launch_hevi_row(const HeviRowMaps& m, const HeviRowArgs& a, cudaStream_t st);
-// The same for njobs members with equal chunk lengths and chunk counts (jobs
-// in device memory, nblocks blocks in all).
-int launch_hevi_row_batch(const HeviRowJob* jobs_d, int njobs, int nblocks, int nk, cudaStream_t st);
+// The same for njobs members with equal chunk lengths (jobs in device memory,
+// nblocks blocks in all), the tallest of nk_max levels.
+int launch_hevi_row_batch(const HeviRowJob* jobs_d, int njobs, int nblocks, int nk_max, cudaStream_t st);
 // The boundary levels and y ghosts, once after the last substep of a loop
 // (a.u, a.v, a.p: the level the loop started from).
 int launch_hevi_row_ends(const HeviRowArgs& a, cudaStream_t st);

@@ -324,9 +324,9 @@ int cress_autotune(cress_ctx* ctx, int nsstp, float dts, int reps, int* best_til
  * were seen before replays one CUDA graph of the whole ensemble step
  * (cress_ensemble_set_graphs(e, 0) turns that off).  Members need impopt=1
  * and the same divopt, sthopt (zero or not) and buyopt.  The shared
- * acoustic launch runs the row-marching kernel (members of different
- * height in separate launches) when every member's grid allows it, else
- * tile 0's 32x8 kernel.  The ensemble's tile is 13 (every member with
+ * acoustic launch runs the row-marching kernel (up to four launches beside each
+ * other, for members of up to 32, 48, 64 and 80 levels) when every member's grid
+ * allows it, else tile 0's 32x8 kernel.  The ensemble's tile is 13 (every member with
  * 8 <= nk <= 68) when every member was created with tile 13, else 0, and the
  * members are set to the ensemble's tile.  cress_ensemble_set_tile switches it (0 or 13);
  * cress_ensemble_autotune times both over `reps` loops of nsstp batched

@@ -79,18 +79,21 @@ def test_tile_13_is_tile_0_up_to_its_height(cress, oracle_lib):
                 assert np.array_equal(x, y)
 
 
+@pytest.mark.parametrize("graphs", [False, True])
 @pytest.mark.parametrize("sizes", [
     [(40, 33, 22, 1), (64, 20, 36, 2), (29, 45, 22, 3)],
     [(190, 41, 22, 1), (131, 70, 22, 2), (64, 20, 22, 3)],   # members with tiles inside the edges, strips of two rows
+    # one launch for heights of equal chunk length (22 and 30: 11 and 15 warps), four in all
+    [(40, 33, 22, 1), (64, 20, 30, 2), (29, 45, 40, 3), (24, 18, 54, 4), (31, 25, 60, 5), (24, 20, 69, 6)],
 ])
-def test_ensemble_of_different_heights_matches_members(cress, oracle_lib, sizes):
-    """Members with different chunk lengths go out in separate launches; each
-    equals the member stepped alone, bit for bit."""
+def test_ensemble_of_different_heights_matches_members(cress, oracle_lib, sizes, graphs):
+    """Members of different heights share a launch where their chunks are
+    equally long; each equals the member stepped alone, bit for bit."""
     out = []
     for together in (False, True):
         sols = [member(cress, oracle_lib, *sz) for sz in sizes]
-        ens = cress.Ensemble(sols, graphs=False) if together else None
-        for step in range(2):
+        ens = cress.Ensemble(sols, graphs=graphs) if together else None
+        for step in range(9 if graphs else 2):
             h = 0.5 if step == 0 else 1.0
             for s in [ens] if together else sols:
                 s.large_step(step * 5000, 5.0 * h, 10, h)
