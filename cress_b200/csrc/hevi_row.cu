@@ -48,6 +48,7 @@
 // registers (265 us: spills).
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <cmath>
 #include "common.cuh"
 #include "f2.cuh"
 #include "hevi_row.cuh"
@@ -560,18 +561,35 @@ bool hevi_row_supported(const Grid& g) {
 
 int hevi_row_tiles_x(const Grid& g) { return (g.ni - 3 + kHrCols - 1) / kHrCols; }
 
+// Blocks of a column of nk levels an SM holds: 4096 registers (128 per
+// thread) and a stage of shared memory per warp.  Two from 8 chunks down (nk = 19),
+// five at the fewest; one for tall columns.
+static int blocks_per_sm(int nk) {
+  const int L = hevi_row_chunk(nk), nC = chunks(nk, L);
+  const size_t bytes = L == 2 ? HrLayout<2>::bytes(nC) : L == 3 ? HrLayout<3>::bytes(nC)
+                     : L == 4 ? HrLayout<4>::bytes(nC) : HrLayout<5>::bytes(nC);
+  const int by_smem = (int)(228 * 1024 / (bytes + 1024 + sizeof(HeviRowArgs)));
+  return std::max(1, std::min(kHrMaxWarps / nC, by_smem));
+}
+
 // Rows per strip: a block costs its rows plus about 1.3 for the row it
-// recomputes and its start, and the blocks run in waves of one per SM; the
-// shortest total wins.
+// recomputes and its start, and the blocks run in waves of what the SMs hold; the
+// shortest total wins.  (Waves of one per SM whatever the height: 512 x 512 x 5
+// 65 us per substep, this 25; the level march before it 42.)
 int hevi_row_rows(const Grid* const* g, int n) {
   const int nsm = sm_count();
+  std::vector<int> per(n);
   int best = 1, ny_max = 1;
-  for (int m = 0; m < n; ++m) ny_max = std::max(ny_max, g[m]->nj - 3);
+  for (int m = 0; m < n; ++m) {
+    ny_max = std::max(ny_max, g[m]->nj - 3);
+    per[m] = blocks_per_sm(g[m]->nk);
+  }
   double cost = 1e30;
   for (int r = 1; r <= ny_max; ++r) {
-    long long t = 0;
-    for (int m = 0; m < n; ++m) t += (long long)hevi_row_tiles_x(*g[m]) * ((g[m]->nj - 3 + r - 1) / r);
-    const double c = (double)((t + nsm - 1) / nsm) * (r + 1.3);
+    double t = 0.0;   // SMs' worth of blocks
+    for (int m = 0; m < n; ++m)
+      t += (double)hevi_row_tiles_x(*g[m]) * ((g[m]->nj - 3 + r - 1) / r) / per[m];
+    const double c = std::ceil(t / nsm - 1e-9) * (r + 1.3);
     if (c < cost - 1e-9) { cost = c; best = r; }
   }
   return best;

@@ -52,6 +52,7 @@ def run(cress, oracle_lib, case, init, rx, ry, impopt, tubopt, advopt, dx, dtbig
 
 @pytest.mark.parametrize("kind,nz,rx,ry,impopt,tubopt,advopt", [
     ("dry", 24, 11, 13, 1, 0, 3),
+    ("dry", 7, 11, 13, 1, 0, 2),      # several blocks per SM
     ("dry", 37, 11, 13, 1, 1, 2),
     ("dry", 30, 11, 13, 0, 1, 2),
     ("dry", 78, 7, 13, 1, 0, 2),
