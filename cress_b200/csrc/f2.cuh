@@ -81,4 +81,38 @@ __device__ __forceinline__ F2 pair_at(const float* p, int dx) {
   return mid2(ld2(p + dx - 1), ld2(p + dx + 1));
 }
 
+// The same pair kept as two floats and, through the intrinsics, open to the fusing
+// of a multiply with an add: for k_scalars, whose separate terms (the reference's
+// parenthesisation) the compiler schedules better in it.  512 x 512 x 64, without and with
+// the eddy mixing: 1193 and 1403 us, in F2 1257 and 1496.
+struct V2 {
+  float2 v;
+  __device__ __forceinline__ float x() const { return v.x; }
+  __device__ __forceinline__ float y() const { return v.y; }
+};
+
+__device__ __forceinline__ V2 v2(float a, float b) { return V2{make_float2(a, b)}; }
+__device__ __forceinline__ V2 v2(float a) { return v2(a, a); }
+__device__ __forceinline__ V2 operator+(V2 a, V2 b) { return V2{__fadd2_rn(a.v, b.v)}; }
+__device__ __forceinline__ V2 operator*(V2 a, V2 b) { return V2{__fmul2_rn(a.v, b.v)}; }
+__device__ __forceinline__ V2 operator-(V2 a, V2 b) {
+  const F2 d = f2(a.x(), a.y()) - f2(b.x(), b.y());
+  V2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.v.x), "=f"(r.v.y) : "l"(d.b));
+  return r;
+}
+__device__ __forceinline__ V2 operator*(float s, V2 b) { return v2(s) * b; }
+__device__ __forceinline__ V2 operator*(V2 a, float s) { return a * v2(s); }
+__device__ __forceinline__ V2 operator-(V2 a, float s) { return a - v2(s); }
+__device__ __forceinline__ V2 fmax2(V2 a, float s) { return v2(fmaxf(a.x(), s), fmaxf(a.y(), s)); }
+__device__ __forceinline__ V2 sel2(int mask, V2 a, V2 b) {
+  return v2((mask & 1) ? a.x() : b.x(), (mask & 2) ? a.y() : b.y());
+}
+__device__ __forceinline__ V2 ldv2(const float* p) { return V2{*reinterpret_cast<const float2*>(p)}; }
+__device__ __forceinline__ void st2(float* p, V2 a) { *reinterpret_cast<float2*>(p) = a.v; }
+__device__ __forceinline__ V2 vpair_at(const float* p, int dx) {
+  if ((dx & 1) == 0) return ldv2(p + dx);
+  return v2(ldv2(p + dx - 1).y(), ldv2(p + dx + 1).x());
+}
+
 }  // namespace cress

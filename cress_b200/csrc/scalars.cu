@@ -64,7 +64,10 @@ struct ScLayout {
 // packed FP32x2 arithmetic (f2.cuh), so each operation serves two points.
 constexpr int kScPairs = kHeviTX / 2;
 
-template <int S, bool TURB>
+// CUT: the column is cut into chunks of levels (blockIdx.z).  A whole column has its
+// bounds known to the compiler: 512 x 512 x 64 1356 -> 1257 us (and 1193 with pairs kept
+// as two floats, V2 of f2.cuh).
+template <int S, bool TURB, bool CUT>
 __global__ void __launch_bounds__(kScPairs * kScalarTY * kScGroup)
 k_scalars(const __grid_constant__ MoistMaps m, const MoistScalarArgs a) {
   // level k+2 must have been issued (at k' = k+5-S) before level k waits for it
@@ -104,8 +107,8 @@ k_scalars(const __grid_constant__ MoistMaps m, const MoistScalarArgs a) {
 
   // this block's levels kA..kB of 2..nk-2 (blockIdx.z), and the levels it
   // stages, two more at either end; level lv lives in slot (lv-lv0) % S
-  const int kA = 2 + blockIdx.z * a.kchunk, kB = min(kA + a.kchunk - 1, nk - 2);
-  const int lv0 = max(kA - 2, 1), lmax = min(nk - 1, kB + 2);
+  const int kA = CUT ? 2 + blockIdx.z * a.kchunk : 2, kB = CUT ? min(kA + a.kchunk - 1, nk - 2) : nk - 2;
+  const int lv0 = CUT ? max(kA - 2, 1) : 1, lmax = CUT ? min(nk - 1, kB + 2) : nk - 1;
   int issued = 0;   // highest level thread 0 has issued
   auto issue = [&](int lv) {
     issued = lv;
@@ -172,65 +175,65 @@ k_scalars(const __grid_constant__ MoistMaps m, const MoistScalarArgs a) {
       const float* V = st0 + L::oV + oV;
       // rstuvwc.f90:172-210 fluxes at the faces the stencil touches
       const float r8u = C(C_RST8U, k), r8v = C(C_RST8V, k);
-      const F2 fu_m1 = r8u * pair_at(U, -1), fu_0 = r8u * ld2(U);
-      const F2 fu_p1 = r8u * pair_at(U, 1), fu_p2 = r8u * ld2(U + 2);
-      const F2 fv_m1 = r8v * ld2(V - BX), fv_0 = r8v * ld2(V);
-      const F2 fv_p1 = r8v * ld2(V + BX), fv_p2 = r8v * ld2(V + 2 * BX);
-      auto WC = [&](F2 w, int kk) { return a.sthopt ? w * C(C_IJCB8W, kk) : w; };
-      const F2 fw_0 = C(C_RST8W, k) * WC(ld2(st0 + L::oW + oU), k);
-      const F2 fw_1 = C(C_RST8W, k + 1) * WC(ld2(st(1) + L::oW + oU), k + 1);
+      const V2 fu_m1 = r8u * vpair_at(U, -1), fu_0 = r8u * ldv2(U);
+      const V2 fu_p1 = r8u * vpair_at(U, 1), fu_p2 = r8u * ldv2(U + 2);
+      const V2 fv_m1 = r8v * ldv2(V - BX), fv_0 = r8v * ldv2(V);
+      const V2 fv_p1 = r8v * ldv2(V + BX), fv_p2 = r8v * ldv2(V + 2 * BX);
+      auto WC = [&](V2 w, int kk) { return a.sthopt ? w * C(C_IJCB8W, kk) : w; };
+      const V2 fw_0 = C(C_RST8W, k) * WC(ldv2(st0 + L::oW + oU), k);
+      const V2 fw_1 = C(C_RST8W, k + 1) * WC(ldv2(st(1) + L::oW + oU), k + 1);
       const float rbct5 = .5f * (C(C_RBCT, k) + C(C_RBCT, k + 1));
       const float rst = C(C_RST, k);
       const float dtdrst = C(D_DTDRST, k);                                  // steps.f90:528
 
       // advs.f90:205-370
-      const F2 s0 = ld2(S0);
-      const F2 t1a = fu_0 * (s0 - pair_at(S0, -1)) * dxv05n;
-      const F2 t1b = fu_p1 * (pair_at(S0, 1) - s0) * dxv05n;
-      const F2 t2a = fv_0 * (s0 - ld2(S0 - BX)) * dyv05n;
-      const F2 t2b = fv_p1 * (ld2(S0 + BX) - s0) * dyv05n;
-      F2 f = (t1a + t1b) + (t2a + t2b);
-      const F2 w1a = (fu_m1 + fu_0) * (s0 - ld2(S0 - 2)) * dxv24;
-      const F2 w1b = (fu_p1 + fu_p2) * (ld2(S0 + 2) - s0) * dxv24;
-      const F2 w2a = (fv_m1 + fv_0) * (s0 - ld2(S0 - 2 * BX)) * dyv24;
-      const F2 w2b = (fv_p1 + fv_p2) * (ld2(S0 + 2 * BX) - s0) * dyv24;
-      const F2 f2nd = f;
+      const V2 s0 = ldv2(S0);
+      const V2 t1a = fu_0 * (s0 - vpair_at(S0, -1)) * dxv05n;
+      const V2 t1b = fu_p1 * (vpair_at(S0, 1) - s0) * dxv05n;
+      const V2 t2a = fv_0 * (s0 - ldv2(S0 - BX)) * dyv05n;
+      const V2 t2b = fv_p1 * (ldv2(S0 + BX) - s0) * dyv05n;
+      V2 f = (t1a + t1b) + (t2a + t2b);
+      const V2 w1a = (fu_m1 + fu_0) * (s0 - ldv2(S0 - 2)) * dxv24;
+      const V2 w1b = (fu_p1 + fu_p2) * (ldv2(S0 + 2) - s0) * dxv24;
+      const V2 w2a = (fv_m1 + fv_0) * (s0 - ldv2(S0 - 2 * BX)) * dyv24;
+      const V2 w2b = (fv_p1 + fv_p2) * (ldv2(S0 + 2 * BX) - s0) * dyv24;
+      const V2 f2nd = f;
       f = fourd3 * f + ((w1a + w1b) + (w2a + w2b));
       if (edge) f = sel2(edge, f2nd, f);   // open x: 2nd order in the boundary columns (advs.f90:312-350)
-      const F2 t3a = fw_0 * (s0 - ld2(st(-1) + L::oS + oS)) * dzv05n;
-      const F2 t3b = fw_1 * (ld2(st(1) + L::oS + oS) - s0) * dzv05n;
-      F2 vadv = t3a + t3b;
+      const V2 t3a = fw_0 * (s0 - ldv2(st(-1) + L::oS + oS)) * dzv05n;
+      const V2 t3b = fw_1 * (ldv2(st(1) + L::oS + oS) - s0) * dzv05n;
+      V2 vadv = t3a + t3b;
       if (a.advopt == 3 && k >= 3 && k <= nk - 3) {   // advs.f90:372-416: 4th order in z
         const float dzv24 = oned24 * a.dziv;
-        const F2 fw_m1 = C(C_RST8W, k - 1) * WC(ld2(st(-1) + L::oW + oU), k - 1);
-        const F2 fw_2 = C(C_RST8W, k + 2) * WC(ld2(st(2) + L::oW + oU), k + 2);
-        const F2 t3w_m = (fw_m1 + fw_0) * (s0 - ld2(st(-2) + L::oS + oS)) * dzv24;
-        const F2 t3w_p = (fw_1 + fw_2) * (ld2(st(2) + L::oS + oS) - s0) * dzv24;
+        const V2 fw_m1 = C(C_RST8W, k - 1) * WC(ldv2(st(-1) + L::oW + oU), k - 1);
+        const V2 fw_2 = C(C_RST8W, k + 2) * WC(ldv2(st(2) + L::oW + oU), k + 2);
+        const V2 t3w_m = (fw_m1 + fw_0) * (s0 - ldv2(st(-2) + L::oS + oS)) * dzv24;
+        const V2 t3w_p = (fw_1 + fw_2) * (ldv2(st(2) + L::oS + oS) - s0) * dzv24;
         vadv = fourd3 * vadv + (t3w_m + t3w_p);
       }
       f = f + vadv;
 
       // the species at t-dt at an offset (horizontal ones on level k only)
       auto SPo = [&](int dx, int dy, int dz) {
-        return dz == 0 ? pair_at(SP0 + dy * BX, dx) : ld2(st(dz) + L::oSP + oS);
+        return dz == 0 ? vpair_at(SP0 + dy * BX, dx) : ldv2(st(dz) + L::oSP + oS);
       };
       if (smooth) {
         auto A = [&](int dx, int dy, int dz) {
           const int kk = k + dz;
-          const F2 v = SPo(dx, dy, dz);
+          const V2 v = SPo(dx, dy, dz);
           return isqv ? C(C_RBR, kk) * (v - C(C_QVBR, kk)) : C(C_RBR, kk) * v;
         };
         f = smooth_tile(f, a.smtopt, a.smhcoe, a.smvcoe, k, 2, nk - 2, A, edge);
       }
       if constexpr (TURB) {
         auto R = [&](int dx, int dy, int dz) {
-          return dz == 0 ? pair_at(st0 + L::oR + oR + dy * BX, dx) : ld2(st(dz) + L::oR + oR);
+          return dz == 0 ? vpair_at(st0 + L::oR + oR + dy * BX, dx) : ldv2(st(dz) + L::oR + oR);
         };
         f = turb_scalar_at(f, C, k, a.cpriv, a.kdiv, a.dxiv, a.dyiv, a.dziv, R, SPo);
       }
-      const F2 spv = ld2(SP0);
+      const V2 spv = ldv2(SP0);
       if (vsp && k >= a.ksp0 - 1) f = f - rbct5 * rst * (isqv ? spv - C(C_QVBR, k) : spv);
-      F2 sf = spv + f * dtdrst;
+      V2 sf = spv + f * dtdrst;
       if (n < 6) sf = fmax2(sf, 0.f);
       // the pair's first index is even, so the pair store is 8-byte aligned
       auto put = [&](long long at) {
@@ -267,8 +270,9 @@ int launch_sc(const MoistScalarArgs& a, const MoistMaps& maps, cudaStream_t st) 
   const Grid& g = a.g;
   const size_t bytes = L::bytes(g.nk);
   if (bytes > 227 * 1024) return CRESS_E_UNSUPPORTED;
-  if (cudaFuncSetAttribute(k_scalars<S, TURB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
-      cudaSuccess)
+  auto cut = k_scalars<S, TURB, true>, whole = k_scalars<S, TURB, false>;
+  if (cudaFuncSetAttribute(cut, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+      cudaFuncSetAttribute(whole, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
     return CRESS_E_CUDA;
   const int nx = g.ni - 3, ny = g.nj - 3;
   dim3 block(kScPairs, kScalarTY, kScGroup);
@@ -276,9 +280,10 @@ int launch_sc(const MoistScalarArgs& a, const MoistMaps& maps, cudaStream_t st) 
   const int n = g.nk - 3;   // levels 2..nk-2
   MoistScalarArgs b = a;
   b.kchunk = level_chunk(n, (long long)grid.x * grid.y,
-                         resident_blocks(k_scalars<S, TURB>, kScPairs * kScalarTY * kScGroup, bytes));
+                         resident_blocks(cut, kScPairs * kScalarTY * kScGroup, bytes));
   grid.z = (n + b.kchunk - 1) / b.kchunk;
-  k_scalars<S, TURB><<<grid, block, bytes, st>>>(maps, b);
+  auto kern = grid.z > 1 ? cut : whole;
+  kern<<<grid, block, bytes, st>>>(maps, b);
   return cudaGetLastError() == cudaSuccess ? 0 : CRESS_E_CUDA;
 }
 

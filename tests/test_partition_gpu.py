@@ -56,6 +56,7 @@ def run(cress, oracle_lib, case, init, rx, ry, impopt, tubopt, advopt, dx, dtbig
     ("dry", 37, 11, 13, 1, 1, 2),
     ("dry", 30, 11, 13, 0, 1, 2),
     ("dry", 78, 7, 13, 1, 0, 2),
+    ("moist", 48, 11, 13, 1, 0, 2),
     ("moist", 54, 11, 13, 1, 2, 2),
     ("moist", 26, 23, 15, 1, 1, 3),
 ])
