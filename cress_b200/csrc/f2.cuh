@@ -83,8 +83,9 @@ __device__ __forceinline__ F2 pair_at(const float* p, int dx) {
 
 // The same pair kept as two floats and, through the intrinsics, open to the fusing
 // of a multiply with an add: for k_scalars, whose separate terms (the reference's
-// parenthesisation) the compiler schedules better in it.  512 x 512 x 64, without and with
-// the eddy mixing: 1193 and 1403 us, in F2 1257 and 1496.
+// parenthesisation) the compiler schedules better in it, and k_hevi2.  512 x 512 x 64
+// scalars, without and with the eddy mixing: 1193 and 1403 us, in F2 1257 and 1496; a
+// substep of tile 11 at 256 x 256 x 60: 162 us, in F2 168.
 struct V2 {
   float2 v;
   __device__ __forceinline__ float x() const { return v.x; }

@@ -164,7 +164,7 @@ __device__ __forceinline__ void hevi2_tile(const HeviMaps& m, const HeviArgs& a,
   const int fyA = 2 * ty, fyB = fyA + 1;       // own rows in the forcing boxes (from j0)
   const float dts = a.dts, dxiv = a.dxiv, dyiv = a.dyiv, dziv = a.dziv;
   const float weic1m = 1.f - a.weicoe;
-  F2 t3v_prev = f2(0.f), fpdvj_prev = f2(0.f), wb8s_prev = f2(0.f);   // rows A, B
+  V2 t3v_prev = v2(0.f), fpdvj_prev = v2(0.f), wb8s_prev = v2(0.f);   // rows A, B
   double fA_prev = 0.0, fB_prev = 0.0;
   bool fail = false;
   // 32-bit element indices (the launcher checks that every field fits)
@@ -211,23 +211,23 @@ __device__ __forceinline__ void hevi2_tile(const HeviMaps& m, const HeviArgs& a,
       else th = pp;
       return jcbk * th;
     };
-    // rows A and B of the thread packed into the two lanes of F2 (f2.cuh):
+    // rows A and B of the thread packed into the two lanes of V2 (f2.cuh):
     // every operation below is one packed instruction for both rows
-    auto col2 = [&](const float* base, int oy) { return f2(base[oy * BX + ox], base[(oy + 1) * BX + ox]); };
-    F2 wc0 = col2(W0, oyA), wc1 = col2(W1, oyA);
+    auto col2 = [&](const float* base, int oy) { return v2(base[oy * BX + ox], base[(oy + 1) * BX + ox]); };
+    V2 wc0 = col2(W0, oyA), wc1 = col2(W1, oyA);
     if constexpr (STH) { wc0 = wc0 * ij8wk; wc1 = wc1 * ij8wk1; }
-    const F2 div = (rst8wk * wc0 - rst8wk1 * wc1) * dziv +
+    const V2 div = (rst8wk * wc0 - rst8wk1 * wc1) * dziv +
                    ((rst8u * col2(U, oyA) - rst8u * col2(U + 1, oyA)) * dxiv +
                     (rst8v * col2(V, oyA) - rst8v * col2(V + BX, oyA)) * dyiv);      // diver3d.f90:318
-    const F2 pp = col2(P, oyA);
-    F2 th;                                                                         // pgrad.f90:341,363
+    const V2 pp = col2(P, oyA);
+    V2 th;                                                                         // pgrad.f90:341,363
     if constexpr (DIV == 2) th = pp + a.divch * div * ijcbk;
     else if constexpr (DIV == 1) th = pp + a.divcv * jcbk * div;
     else th = pp;
-    const F2 tc = jcbk * th;
+    const V2 tc = jcbk * th;
     t3h[oyA * BX + ox] = tc.x();
     t3h[oyB * BX + ox] = tc.y();
-    const F2 t3v = (DIV >= 1) ? pp + a.divcv * jcbk * div : pp;                    // pgrad.f90:300
+    const V2 t3v = (DIV >= 1) ? pp + a.divcv * jcbk * div : pp;                    // pgrad.f90:300
     if (has_halo) t3h[hy * BX + hx] = t3h_of(div3d_at(hx, hy), P[hy * BX + hx]);
     __syncthreads();
     // a stage is refilled only by a thread 0 that saw its previous copy land
@@ -238,16 +238,16 @@ __device__ __forceinline__ void hevi2_tile(const HeviMaps& m, const HeviArgs& a,
 
     // stepuv.f90:294,304 with pgrad.f90:379,389: west u faces, the east
     // face from the next lane (lane 31 forms its own)
-    const F2 un0 = col2(U, oyA) + dts * (col2(UF, fyA) + (col2(t3h - 1, oyA) - tc) * dxiv) * irst8u;
-    F2 un1 = f2(__shfl_down_sync(full, un0.x(), 1), __shfl_down_sync(full, un0.y(), 1));
+    const V2 un0 = col2(U, oyA) + dts * (col2(UF, fyA) + (col2(t3h - 1, oyA) - tc) * dxiv) * irst8u;
+    V2 un1 = v2(__shfl_down_sync(full, un0.x(), 1), __shfl_down_sync(full, un0.y(), 1));
     if (tx == TX - 1)
       un1 = col2(U + 1, oyA) + dts * (col2(UF + 1, fyA) + (tc - col2(t3h + 1, oyA)) * dxiv) * irst8u;
     // v faces south of rows A and B (the one between the rows serves both),
     // and north of row B
-    const F2 vs = col2(V, oyA) + dts * (col2(VF, fyA) + (f2(t3h[(oyA - 1) * BX + ox], tc.x()) - tc) * dyiv) * irst8v;
+    const V2 vs = col2(V, oyA) + dts * (col2(VF, fyA) + (v2(t3h[(oyA - 1) * BX + ox], tc.x()) - tc) * dyiv) * irst8v;
     const float vf2 = V[(oyB + 1) * BX + ox] +
                       dts * (VF[(fyB + 1) * BX + ox] + (tc.y() - t3h[(oyB + 1) * BX + ox]) * dyiv) * irst8v;
-    const F2 vn = f2(vs.y(), vf2);
+    const V2 vn = v2(vs.y(), vf2);
 
     const float jcb8u = CK(k, C_JCB8U), jcb8v = CK(k, C_JCB8V);
     const float rcsq = CK(k, C_RCSQ), rst = CK(k, C_RST), rbr = CK(k, C_RBR), ircsq = CK(k, C_IRCSQ);
@@ -275,20 +275,20 @@ __device__ __forceinline__ void hevi2_tile(const HeviMaps& m, const HeviArgs& a,
     if (ownA) store_uv(edgeA, ylastA, jA, idA, un0.x(), un1.x(), vs.x(), vn.x());
     if (ownB) store_uv(edgeB, ylastB, jB, idB, un0.y(), un1.y(), vs.y(), vn.y());
 
-    F2 phd = (jcb8u * un0 - jcb8u * un1) * dxiv + (jcb8v * vs - jcb8v * vn) * dyiv;    // diver2d.f90:288
+    V2 phd = (jcb8u * un0 - jcb8u * un1) * dxiv + (jcb8v * vs - jcb8v * vn) * dyiv;    // diver2d.f90:288
     phd = rcsq * phd;                                                                   // diverpih.f90:208
-    const F2 wk = col2(W0, oyA), wk1 = col2(W1, oyA);
-    const F2 pvd = rcsq * (wk - wk1) * dziv;                                            // diverpiv.f90:124
-    const F2 fp = col2(PF, fyA) + phd + weic1m * (a.g05 * (wk + wk1) * rst + pvd);      // advbspi.f90:158
+    const V2 wk = col2(W0, oyA), wk1 = col2(W1, oyA);
+    const V2 pvd = rcsq * (wk - wk1) * dziv;                                            // diverpiv.f90:124
+    const V2 fp = col2(PF, fyA) + phd + weic1m * (a.g05 * (wk + wk1) * rst + pvd);      // advbspi.f90:158
     if (ownA) a.p_new[idA] = fp.x();   // parked until the way down
     if (ownB) a.p_new[idB] = fp.y();
-    const F2 fpdvj = fp * ijcbk;                                                        // pgradiv.f90:149
-    const F2 wb8s = (pp * rst + fp * rbr * a.dtw) * ircsq * a.g05n;                     // buoywsi.f90:171
+    const V2 fpdvj = fp * ijcbk;                                                        // pgradiv.f90:149
+    const V2 wb8s = (pp * rst + fp * rbr * a.dtw) * ircsq * a.g05n;                     // buoywsi.f90:171
     if (k >= 3) {
-      const F2 wpg = (t3v_prev - t3v) * dziv;                                           // pgrad.f90:320
-      F2 fw = col2(WF, fyA) + wpg + (fpdvj_prev - fpdvj) * a.dtdzw;                     // pgradiv.f90:163
+      const V2 wpg = (t3v_prev - t3v) * dziv;                                           // pgrad.f90:320
+      V2 fw = col2(WF, fyA) + wpg + (fpdvj_prev - fpdvj) * a.dtdzw;                     // pgradiv.f90:163
       if constexpr (BUY) fw = fw + (wb8s_prev + wb8s);                                  // buoywsi.f90:205
-      const F2 wrhs = wk + dts * fw * irst8w;                                           // stepwi.f90:325
+      const V2 wrhs = wk + dts * fw * irst8w;                                           // stepwi.f90:325
       // gaussel.f90:189-240 in double with the 1-D factors, one recurrence per row
       const double rr = (double)TH_RR(k), aa = TH_AA(k);
       const double fA = (k == 3) ? (double)wrhs.x() * aa : ((double)wrhs.x() - rr * fA_prev) * aa;
